@@ -60,7 +60,7 @@ def listed():
         # long sequences under a band mask, forward and checkpointed backward
         _case("train", "sw_affine", 4, 8192, 8192, band=1024, name="sw_affine_banded_4x8192x8192"),
         # thousands of pairs of uneven lengths in one packed launch: the benchmark's batch
-        _plan_case("sw_affine", 4096, 32, 2048, 3, cols=8, name="sw_affine_plan_4096"),
+        _plan_case("sw_affine", 4096, 32, 2048, 3, cols=8, T=1.0, name="sw_affine_plan_4096"),
         # the end-to-end layer's loss: value and entropy, backward into the scores
         _case("entropy", "sw_affine", 256, 512, 512, name="sw_affine_entropy_256x512x512"),
         # a loss on the alignment map itself: forward, adjoint and a Hessian-vector product
