@@ -57,17 +57,21 @@ bool lin_eligible(float go, float ge, float T, const swb_options* opt) {
   return xo <= 0.0 && xe <= 0.0;
 }
 // Default columns per lane of the padded entry points, for the linear-domain
-// kernels: 8 on batches at least 256 columns wide (half the bands, each
-// step's fixed work spread over twice the cells: measured faster from
-// 64 x 1024^2 to 4 x 4096^2); 2 on batches at most 64 columns wide (one band
-// with every lane live: forward + adjoint of 1 x 64^2 in 84 us against 105 at
-// 4, 128 x 64^2 in 87 against 106); else 4.  The log domain always takes 4.
-int default_r(long long L2m, bool lin) {
+// kernels: 2 on batches at most 64 columns wide (one band with every lane
+// live), 8 on wide batches with enough bands of 256 columns to fill the GPU
+// (half the bands, each step's fixed work spread over twice the cells), else
+// 4, whose steps are shorter: what counts then is the chain of steps.  The
+// log domain always takes 4.  Forward + adjoint, affine, 4 against 8 columns,
+// us: 4 x 1024^2 (16 bands of 256) 778 / 861; 64 x 1024^2 (256) 875 / 992;
+// 256 x 512^2 (512) 534 / 548; 512 x 512^2 (1024) 834 / 715.
+constexpr long long kWideBands = 768;
+int default_r(long long B, long long L2m, bool lin) {
   if (!lin) return kDefaultR;
-  return L2m >= 256 ? 8 : (L2m <= 64 ? 2 : kDefaultR);
+  if (L2m <= 64) return 2;
+  return L2m >= 256 && B * ((L2m + 255) / 256) >= kWideBands ? 8 : kDefaultR;
 }
-int pick_r(const swb_options* opt, long long L2m, bool lin) {
-  return (opt && opt->cols_per_lane) ? opt->cols_per_lane : default_r(L2m, lin);
+int pick_r(const swb_options* opt, long long B, long long L2m, bool lin) {
+  return (opt && opt->cols_per_lane) ? opt->cols_per_lane : default_r(B, L2m, lin);
 }
 
 struct Layout {
@@ -94,6 +98,29 @@ Layout layout_sizes(long long B, size_t slots, size_t edge_floats, size_t bp_flo
   l.off_ckpt = o;       o = align_up(o + sizeof(float) * ck_floats);
   l.total = o;
   return l;
+}
+
+// Small padded batches of the local models in the linear domain: the outside
+// recursion runs as a sweep of its own, then every band's segments (sw_lin.cu).
+// With more bands than this the adjoint's own chains fill the GPU, and the
+// sweep would only add work.  Adjoint against sweep + segments, affine, 4
+// columns per lane, us: 1 x 1024 x 2048 (16 bands) 682 / 367; 4 x 1024^2 (32)
+// 548 / 304; 16 x 1024^2 (128) 552 / 453; 32 x 1024^2 (256) 557 / 571;
+// 64 x 1024^2 (512) 563 / 783.
+constexpr long long kSegSlots = 192;
+struct SegPlan {
+  int nseg = 0;
+  size_t off_state = 0, off_part = 0, total = 0;   // total 0: not used
+};
+template <int R>
+SegPlan seg_plan(const Layout& l, long long slots) {
+  SegPlan p;
+  if (!swb::split_code<R>() || slots > kSegSlots) return p;
+  p.nseg = (l.nchunks + swb::kSeg - 1) / swb::kSeg;
+  p.off_state = l.total;
+  p.off_part = p.off_state + align_up(sizeof(float) * (size_t)slots * p.nseg * swb::BDims<R>::BREC);
+  p.total = p.off_part + align_up(sizeof(float) * 4 * (size_t)slots * p.nseg);
+  return p;
 }
 
 int chunks_for(long long L1) { return (int)((L1 + 31 + swb::C_STEPS - 1) / swb::C_STEPS); }
@@ -132,6 +159,8 @@ struct DevInfo {
   int occ[2][5][2] = {};   // [kernel fwd/bwd][model_index][R == 4?]
   int locc[2][2][3] = {};  // linear-domain kernels: [fwd/bwd][NS == 3?][R: 2, 4, 8]
   int locc_sparse[2][3] = {};  // linear-domain adjoint, sparse checkpoints: [NS == 3?][R: 2, 4, 8]
+  int sweep[2][3] = {};        // outside sweep: [NS == 3?][R: 2, 4, 8]
+  int seg[2][2][3] = {};       // segments: [sparse?][NS == 3?][R: 2, 4, 8]
   bool ready = false;
 };
 DevInfo g_dev[64];
@@ -160,7 +189,20 @@ cudaError_t setup_lin(DevInfo& d) {
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
       &d.locc[1][NS == 3][ridx(R)], swb::lbwd_kernel<NS, R, kWarpsBwd>, 32 * kWarpsBwd,
       lbwd_smem<NS, R>());
-  if (e != cudaSuccess || R == 2) return e;   // the checkpointed op runs 4 or 8 columns per lane
+  if (e != cudaSuccess) return e;
+  if constexpr (swb::split_code<R>()) {
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.sweep[NS == 3][ridx(R)], swb::lbeta_kernel<NS, R>, 128,
+                                                         0)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(swb::lseg_kernel<NS, R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)lbwd_smem<NS, R>())) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(swb::lseg_kernel<NS, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)lbwd_smem<NS, R>())) != cudaSuccess ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.seg[0][NS == 3][ridx(R)], swb::lseg_kernel<NS, R, false>,
+                                                         32, lbwd_smem<NS, R>())) != cudaSuccess ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.seg[1][NS == 3][ridx(R)], swb::lseg_kernel<NS, R, true>,
+                                                         32, lbwd_smem<NS, R>())) != cudaSuccess)
+    return e;
+  }
   e = cudaFuncSetAttribute(swb::lbwd_kernel<NS, R, kWarpsBwd, true>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lbwd_smem<NS, R>());
   if (e != cudaSuccess) return e;
@@ -245,6 +287,23 @@ int static_scratch(void** out) {
   return SWB_OK;
 }
 
+// The outside sweep and the segments of a padded batch.
+template <int NS, int R>
+int launch_segments(Args a, const DevInfo& d, const SegPlan& p, char* w, bool sparse, int max_ctas, cudaStream_t st) {
+  a.bck = reinterpret_cast<float*>(w + p.off_state);
+  a.spart = reinterpret_cast<float*>(w + p.off_part);
+  a.nseg = p.nseg;
+  const long long slots = (long long)a.B * a.nb, n = slots * p.nseg;
+  const int os = d.sweep[NS == 3][ridx(R)], og = d.seg[sparse][NS == 3][ridx(R)];
+  long long gs = std::min<long long>((slots + 3) / 4, (long long)d.sms * std::max(os, 1));
+  long long gg = std::min<long long>(n, (long long)d.sms * std::max(og, 1));
+  if (max_ctas > 0) { gs = std::min<long long>(gs, max_ctas); gg = std::min<long long>(gg, max_ctas); }
+  swb::lbeta_kernel<NS, R><<<(int)std::max(1LL, gs), 128, 0, st>>>(a);
+  if (sparse) swb::lseg_kernel<NS, R, true><<<(int)std::max(1LL, gg), 32, lbwd_smem<NS, R>(), st>>>(a);
+  else swb::lseg_kernel<NS, R, false><<<(int)std::max(1LL, gg), 32, lbwd_smem<NS, R>(), st>>>(a);
+  return cudaPeekAtLastError() == cudaSuccess ? SWB_OK : SWB_ERR_CUDA;
+}
+
 // Common launch: per-call resets, then the forward and adjoint kernels.
 template <int NS, int R, int G = 0>
 int launch(Args a, const Layout& l, long long ntasks, size_t map_elems, bool clear_map, void* ws,
@@ -305,6 +364,11 @@ int launch(Args a, const Layout& l, long long ntasks, size_t map_elems, bool cle
   if (grid_b < 1) grid_b = 1;
   if (lin) {
     if constexpr (G == 0) {
+      SegPlan seg;
+      if (a.layout == 0 && !value_only && !a.fault_inject) {
+        seg = seg_plan<R>(l, ntasks);
+        if (ws_bytes < seg.total) seg = SegPlan{};
+      }
       swb::lfwd_kernel<NS, R><<<grid_f, 32 * kWarpsFwd, 0, st>>>(a);
       if (cudaPeekAtLastError() != cudaSuccess) return SWB_ERR_CUDA;
       if (opt && opt->split_event &&
@@ -313,6 +377,10 @@ int launch(Args a, const Layout& l, long long ntasks, size_t map_elems, bool cle
       if (value_only) {
         swb::lvalue_kernel<NS, R><<<(a.B + 3) / 4, 128, 0, st>>>(a);
         return cudaPeekAtLastError() == cudaSuccess ? SWB_OK : SWB_ERR_CUDA;
+      }
+      if constexpr (swb::split_code<R>()) {
+        if (seg.total)
+          return launch_segments<NS, R>(a, *d, seg, w, false, opt ? opt->max_ctas : 0, st);
       }
       swb::lbwd_kernel<NS, R, kWarpsBwd><<<grid_b, 32 * kWarpsBwd, lbwd_smem<NS, R>(), st>>>(a);
       return cudaPeekAtLastError() == cudaSuccess ? SWB_OK : SWB_ERR_CUDA;
@@ -351,14 +419,15 @@ int launch_padded_r(const float* scores, const int* lengths, int B, int L1m, int
   a.go = go; a.ge = ge; a.T = T;
   a.nb = l.nb; a.nchunks = l.nchunks;
   a.value = value; a.g_open = g_open; a.g_ext = g_ext; a.g_T = g_T;
-  return launch<NS, R, G>(a, l, (long long)B * l.nb, map_elems, true, ws, ws_bytes, stream, opt);
+  // with full lengths the adjoint writes every cell of the map
+  return launch<NS, R, G>(a, l, (long long)B * l.nb, map_elems, lengths != nullptr, ws, ws_bytes, stream, opt);
 }
 
 template <int NS, int G = 0>
 int launch_padded(const float* scores, const int* lengths, int B, int L1m, int L2m, float go,
                   float ge, float T, float* value, float* map, float* g_open, float* g_ext,
                   float* g_T, void* ws, size_t ws_bytes, void* stream, const swb_options* opt) {
-  const int r = pick_r(opt, L2m, lin_eligible<NS, G>(go, ge, T, opt));
+  const int r = pick_r(opt, B, L2m, lin_eligible<NS, G>(go, ge, T, opt));
   if (r == 2)
     return launch_padded_r<NS, 2, G>(scores, lengths, B, L1m, L2m, go, ge, T, value, map, g_open,
                                      g_ext, g_T, ws, ws_bytes, stream, opt);
@@ -407,7 +476,7 @@ int launch_value(const float* scores, const int* lengths, int B, int L1m, int L2
     return launch<NS, R, G>(a, l, (long long)B * l.nb, 0, false, ws, ws_bytes, stream, nullptr, true);
   };
   if constexpr (G == 0) {
-    const int r = default_r(L2m, lin_eligible<NS, G>(go, ge, T, nullptr));
+    const int r = default_r(B, L2m, lin_eligible<NS, G>(go, ge, T, nullptr));
     if (r == 8) return run(std::integral_constant<int, 8>{});
     if (r == 2) return run(std::integral_constant<int, 2>{});
   }
@@ -804,12 +873,16 @@ int ck_adjoint_r(const float* scores, const int* lengths, int B, int L1m, int L2
   swb::adjoint_reset_kernel<<<(B + 255) / 256, 256, 0, st>>>(a.counters, a.pair_done, B);
   if (cudaMemsetAsync(w + l.off_bpush, 0xff, l.off_ckpt - l.off_bpush, st) != cudaSuccess)
     return SWB_ERR_CUDA;
-  if (map_elems > 0 && cudaMemsetAsync(map, 0, map_elems * sizeof(float), st) != cudaSuccess)
+  if (lengths && map_elems > 0 && cudaMemsetAsync(map, 0, map_elems * sizeof(float), st) != cudaSuccess)
     return SWB_ERR_CUDA;
   const long long ntasks = (long long)B * l.nb;
   const int ob = kc > 1 ? d->locc_sparse[NS == 3][ridx(R)] : d->locc[1][NS == 3][ridx(R)];
   const long long cap = (long long)d->sms * (ob > 0 ? ob : 1);
   const int grid = (int)std::max(1LL, std::min((ntasks + kWarpsBwd - 1) / kWarpsBwd, cap));
+  if constexpr (swb::split_code<R>()) {
+    const SegPlan seg = seg_plan<R>(l, ntasks);
+    if (seg.total && ws_bytes >= seg.total) return launch_segments<NS, R>(a, *d, seg, w, kc > 1, 0, st);
+  }
   if (kc > 1)
     swb::lbwd_kernel<NS, R, kWarpsBwd, true><<<grid, 32 * kWarpsBwd, lbwd_smem<NS, R>(), st>>>(a);
   else
@@ -822,7 +895,7 @@ int ck_adjoint_r(const float* scores, const int* lengths, int B, int L1m, int L2
 template <int NS>
 int ck_forward(const float* scores, const int* lengths, int B, int L1m, int L2m, float go, float ge,
                float T, int kc, float* value, void* ws, size_t ws_bytes, void* stream_v) {
-  const int r = default_r(L2m, true);
+  const int r = default_r(B, L2m, true);
   if (r == 8)
     return ck_forward_r<NS, 8>(scores, lengths, B, L1m, L2m, go, ge, T, kc, value, ws, ws_bytes, stream_v);
   if (r == 2)
@@ -834,7 +907,7 @@ template <int NS>
 int ck_adjoint(const float* scores, const int* lengths, int B, int L1m, int L2m, float go, float ge,
                float T, int kc, float* value, float* map, float* g_open, float* g_ext, float* g_T,
                void* ws, size_t ws_bytes, void* stream_v) {
-  const int r = default_r(L2m, true);
+  const int r = default_r(B, L2m, true);
   if (r == 8)
     return ck_adjoint_r<NS, 8>(scores, lengths, B, L1m, L2m, go, ge, T, kc, value, map, g_open, g_ext,
                                g_T, ws, ws_bytes, stream_v);
@@ -845,11 +918,17 @@ int ck_adjoint(const float* scores, const int* lengths, int B, int L1m, int L2m,
                              g_T, ws, ws_bytes, stream_v);
 }
 
+// A layout's bytes with the segments' states and partials, where they are used.
+template <int R> size_t with_segments(const Layout& l, long long B) {
+  return std::max(l.total, seg_plan<R>(l, B * l.nb).total);
+}
+
 template <int NS>
 size_t ck_workspace(long long B, long long L1m, long long L2m, int kc) {
-  const int r = default_r(L2m, true);
-  return r == 8 ? ck_layout<NS, 8>(B, L1m, L2m, kc).total
-                : (r == 2 ? ck_layout<NS, 2>(B, L1m, L2m, kc).total : ck_layout<NS, 4>(B, L1m, L2m, kc).total);
+  const int r = default_r(B, L2m, true);
+  return r == 8   ? with_segments<8>(ck_layout<NS, 8>(B, L1m, L2m, kc), B)
+         : r == 2 ? with_segments<2>(ck_layout<NS, 2>(B, L1m, L2m, kc), B)
+                  : with_segments<4>(ck_layout<NS, 4>(B, L1m, L2m, kc), B);
 }
 
 }  // namespace
@@ -858,8 +937,8 @@ extern "C" {
 
 int swb_cols_per_lane(int family, int L2max, float gap_open, float gap_ext, float temp) {
   // family: 1 linear, 3 affine (local); 2, 4, 5 global and Saigo-Vert
-  if (family == 1) return default_r(L2max, lin_eligible<1, 0>(gap_open, 0.f, temp, nullptr));
-  if (family == 3) return default_r(L2max, lin_eligible<3, 0>(gap_open, gap_ext, temp, nullptr));
+  if (family == 1) return default_r(1, L2max, lin_eligible<1, 0>(gap_open, 0.f, temp, nullptr));
+  if (family == 3) return default_r(1, L2max, lin_eligible<3, 0>(gap_open, gap_ext, temp, nullptr));
   return (family >= 1 && family <= 5) ? kDefaultR : SWB_ERR_ARG;
 }
 
@@ -1052,8 +1131,9 @@ int swb_nw_param_jacobian(const float* scores, const int* lengths, int B, int L1
 
 size_t swb_sw_affine_workspace_bytes(int B, int L1max, int L2max) {
   if (B <= 0) return 0;
-  return std::max({layout_for<3, 2>(B, L1max, L2max).total, layout_for<3, 4>(B, L1max, L2max).total,
-                   layout_for<3, 8>(B, L1max, L2max).total});
+  return std::max({with_segments<2>(layout_for<3, 2>(B, L1max, L2max), B),
+                   with_segments<4>(layout_for<3, 4>(B, L1max, L2max), B),
+                   with_segments<8>(layout_for<3, 8>(B, L1max, L2max), B)});
 }
 
 int swb_scan_scores(const float* x, int B, long long per_item, float limit, float sentinel,
@@ -1104,8 +1184,9 @@ int swb_sw_value(const float* scores, const int* lengths, int B, int L1max, int 
 
 size_t swb_sw_workspace_bytes(int B, int L1max, int L2max) {
   if (B <= 0) return 0;
-  return std::max({layout_for<1, 2>(B, L1max, L2max).total, layout_for<1, 4>(B, L1max, L2max).total,
-                   layout_for<1, 8>(B, L1max, L2max).total});
+  return std::max({with_segments<2>(layout_for<1, 2>(B, L1max, L2max), B),
+                   with_segments<4>(layout_for<1, 4>(B, L1max, L2max), B),
+                   with_segments<8>(layout_for<1, 8>(B, L1max, L2max), B)});
 }
 
 int swb_sw_affine_forward(const float* scores, const int* lengths, int B, int L1max, int L2max,
@@ -1121,7 +1202,7 @@ int swb_sw_affine_forward_static(const float* scores, const int* lengths, int B,
                                  float* value, float* map, float* grad_open, float* grad_ext,
                                  float* grad_temp, void* stream, const swb_options* opt) {
   // size check first: an oversize batch is rejected before any CUDA call
-  const int r = pick_r(opt, L2max, lin_eligible<3, 0>(gap_open, gap_ext, temp, opt));
+  const int r = pick_r(opt, B, L2max, lin_eligible<3, 0>(gap_open, gap_ext, temp, opt));
   if (B > 0 && L1max >= 0 && L2max >= 0 && valid_r_local(r)) {
     const size_t need = r == 2 ? layout_for<3, 2>(B, L1max, L2max).total
                                : (r == 4 ? layout_for<3, 4>(B, L1max, L2max).total

@@ -116,6 +116,10 @@ struct Args {
   float* edge;                // [B*nb][2*NS][Lmax1] sentinel-initialised
   float* bpush;               // [B*nb][NP][Lmax1+1] sentinel-initialised
   float* ckpt;                // [B*nb][nchunks][CKF][32]
+  // linear-domain kernels, small padded batches (outside sweep, then segments)
+  float* bck;                 // [B*nb][nseg] outside-recursion states
+  float* spart;               // [B*nb][nseg][4] gradient partials
+  int nseg;                   // segments per band
   unsigned long long spin_limit_ns;
   int fault_inject;           // 1: band>0 waits on a word nobody writes (tests only)
   float* never_written;       // target of fault_inject polls

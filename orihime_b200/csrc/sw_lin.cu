@@ -136,71 +136,128 @@ __device__ __forceinline__ void zero_chunk_rows(const Pair& pr, int kc, int col0
   }
 }
 
+// ---------------------------------------------------------------------------
+// packed columns
+// ---------------------------------------------------------------------------
+// A lane's R columns are kept as R / 2 float2 pairs (k, k + R/2), so that one
+// packed fp32 instruction (fma.rn.f32x2 and its kin, the same rounding per
+// component) works on two columns, and the diagonal inputs of pair k are
+// simply pair k - 1 of the row above: only pair 0 has to be put together.
+__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+// column c of a row of pairs
+template <int H> __device__ __forceinline__ float& col(float2 (&p)[H], int c) {
+  return c < H ? p[c < H ? c : 0].x : p[c >= H ? c - H : 0].y;
+}
+// Sum over the columns, a short tree.
+template <int H> __device__ __forceinline__ float sum2(const float2 (&p)[H]) {
+  float2 s[H];
+#pragma unroll
+  for (int k = 0; k < H; ++k) s[k] = p[k];
+#pragma unroll
+  for (int h = 1; h < H; h *= 2)
+#pragma unroll
+    for (int k = 0; k + h < H; k += 2 * h) s[k] = add2(s[k], s[k + h]);
+  return s[0].x + s[0].y;
+}
+// 2^d as bits for d + 127 given: 0 below the exponent range.
+__device__ __forceinline__ float p2b(int d127) { return __int_as_float(max(d127, 0) << 23); }
+
 // Checkpoint floats per lane (CKF, padded to float4), one checkpoint record
 // (LREC: CK4 groups of [lane][4]) and adjoint shared-memory floats per lane
 // per step (FW).  A band's checkpoint region holds ceil(nchunks / ck_every)
 // records, then one float per chunk: the chunk's largest normalised alpha
-// frame (the adjoint's quiet-chunk test).  An affine record keeps M and I of
-// the lane's row but not D: D is rebuilt from M, the left lane's values and
-// the frames with the forward's own operations (lck_unpack), bit for bit, so
-// a record is 24 floats per lane instead of 32 at 8 columns per lane.
+// frame (the adjoint's quiet-chunk test).  A record keeps M and I of the
+// lane's row (linear: A), D of its first column, the left lane's diagonal sum
+// and two frames; the rest of D, the column sums and the normalised frame are
+// rebuilt with the forward's own operations, bit for bit: 20 floats per lane
+// at 8 columns per lane (12 for the linear gap).
 template <int NS, int R> struct LDims {
-  static constexpr int NSTORE = NS == 3 ? 2 : 1;         // states stored per column
-  static constexpr int CKV = NSTORE * R + NS + 3;        // raw row, left values, e, n, nl
+  static constexpr int H = R / 2;
+  static constexpr int CKV = NS == 3 ? 2 * R + 4 : R + 3;
   static constexpr int CKF = (CKV + 3) / 4 * 4;
   static constexpr int CK4 = CKF / 4;
   static constexpr int LREC = CKF * 32;
   // affine: M, I, D (raw) and the scaled score per column; linear: A, the
-  // emission part E (A_diag + 1), and the scaled score; then e and n
+  // emission part E (A_diag + 1), and the scaled score; then the frame e
   static constexpr int NF = NS == 3 ? 4 : 3;
-  static constexpr int FW = NF * R + 2;
+  static constexpr int FW = NF * R + 1;
 };
 
 // Lane state of the forward wavefront.
 template <int NS, int R> struct LState {
-  float v[NS][R];   // raw values of the lane's latest row (frame e)
-  float cs[NS == 3 ? R : 1];   // affine: their column sums (M + I) + D (frame e)
-  float lv[NS];     // the left lane's latest row, last column (normalised frame nl)
-  float vs[NS];     // the lane's last column in its normalised frame n
-  int e, n, nl;
+  static constexpr int H = R / 2;
+  float2 v[NS == 3 ? 2 : 1][H];    // raw M and I (linear: A) of the lane's latest row (frame e)
+  float2 c[NS == 3 ? H : 1];       // affine: the row's column sums (M + I) + D (frame e)
+  float ds;                        // the left lane's column sum (linear: A) of that row, last column (frame e)
+  float od, oc;                    // out to the right lane: D of the column after the last, the last column's sum
+  int e, n, nd;                    // raw frame, normalised frame, the left lane's normalised frame of that row
 };
 
-// Affine: the column sums of the lane's row, the diagonal inputs of the next
-// row's M (formed once per row, not once per cell).
-template <int NS, int R>
-__device__ __forceinline__ void lstate_sums(LState<NS, R>& s) {
-  if constexpr (NS == 3) {
-#pragma unroll
-    for (int c = 0; c < R; ++c) s.cs[c] = (s.v[0][c] + s.v[1][c]) + s.v[2][c];
-  }
-}
+// Exponent bound of a non-negative sum: x <= 2^(sexp(x) - 126).
+__device__ __forceinline__ int sexp(float x) { return (int)(__float_as_uint(x) >> 23); }
 
 template <int NS, int R>
 __device__ __forceinline__ void lstate_zero(LState<NS, R>& s) {
+  constexpr int H = R / 2;
 #pragma unroll
-  for (int q = 0; q < NS; ++q) {
-    s.lv[q] = 0.f; s.vs[q] = 0.f;
-#pragma unroll
-    for (int c = 0; c < R; ++c) s.v[q][c] = 0.f;
+  for (int k = 0; k < H; ++k) {
+    s.v[0][k] = dup2(0.f);
+    if constexpr (NS == 3) { s.v[1][k] = dup2(0.f); s.c[k] = dup2(0.f); }
   }
-  lstate_sums(s);
-  s.e = 0; s.n = 0; s.nl = 0;
+  s.ds = 0.f; s.od = 0.f; s.oc = 0.f;
+  s.e = 0; s.n = 0; s.nd = 0;
+}
+
+// Columns past the pair (DM): 0 the band has none, 1 it may have some and they
+// are masked without a branch, 2 a warp-uniform branch on whether it has any.
+// The kernels at 8 columns per lane, which run with every scheduler full,
+// keep one copy of their steps (2, and no copy for chunks inside the pair):
+// with several the instruction cache misses cost more than the branches
+// (4096 ragged pairs, forward + adjoint: 7.0 ms against 5.0).  The narrower
+// ones run few warps, and there a branch costs its latency.
+template <int R> __host__ __device__ constexpr bool split_code() { return R < 8; }
+template <int DM> __device__ __forceinline__ bool masks(bool has_dead) {
+  return DM == 1 || (DM == 2 && has_dead);
+}
+
+// D of a row from its first column's D and the row's M: D runs along the
+// lane's columns, one fma per column on that chain; `od` is the next lane's
+// first D.  Columns past the pair get 0.
+template <int NS, int R, int DM>
+__device__ __forceinline__ void ldchain(const float2 (&m)[R / 2], float d0, float gO, float gE, int nlive, bool hd,
+                                        float2 (&d)[R / 2], float& od) {
+  constexpr int H = R / 2;
+  float2 t[H];
+#pragma unroll
+  for (int k = 0; k < H; ++k) t[k] = mul2(dup2(gO), m[k]);
+  col(d, 0) = d0;
+#pragma unroll
+  for (int c = 1; c < R; ++c) col(d, c) = fmaf(gE, col(d, c - 1), col(t, c - 1));
+  od = fmaf(gE, col(d, R - 1), col(t, R - 1));
+  if (masks<DM>(hd)) {
+#pragma unroll
+    for (int c = 0; c < R; ++c)
+      if (c >= nlive) col(d, c) = 0.f;
+  }
 }
 
 template <int NS, int R>
-__device__ __forceinline__ void lck_store(float* rec, int lane, const LState<NS, R>& s) {
+__device__ __forceinline__ void lck_store(float* rec, int lane, const LState<NS, R>& s, float d0) {
   using L = LDims<NS, R>;
-  constexpr int V = L::NSTORE * R;   // where the left values start
+  constexpr int H = R / 2;
   float x[L::CKF];
 #pragma unroll
-  for (int q = 0; q < L::NSTORE; ++q)
+  for (int q = 0; q < (NS == 3 ? 2 : 1); ++q)
 #pragma unroll
-    for (int c = 0; c < R; ++c) x[q * R + c] = s.v[q][c];
-#pragma unroll
-  for (int q = 0; q < NS; ++q) x[V + q] = s.lv[q];
-  x[V + NS] = __int_as_float(s.e);
-  x[V + NS + 1] = __int_as_float(s.n);
-  x[V + NS + 2] = __int_as_float(s.nl);
+    for (int k = 0; k < H; ++k) { x[q * R + 2 * k] = s.v[q][k].x; x[q * R + 2 * k + 1] = s.v[q][k].y; }
+  constexpr int V = NS == 3 ? 2 * R : R;
+  x[V] = s.ds;
+  x[V + 1] = __int_as_float(s.e);
+  x[V + 2] = __int_as_float(s.nd);
+  if constexpr (NS == 3) x[V + 3] = d0;
 #pragma unroll
   for (int f = L::CKV; f < L::CKF; ++f) x[f] = 0.f;
 #pragma unroll
@@ -208,137 +265,297 @@ __device__ __forceinline__ void lck_store(float* rec, int lane, const LState<NS,
     reinterpret_cast<float4*>(rec + g * 128)[lane] = make_float4(x[4 * g], x[4 * g + 1], x[4 * g + 2], x[4 * g + 3]);
 }
 
-template <int NS, int R>
-__device__ __forceinline__ void lck_load(const float* rec, int lane, float (&x)[LDims<NS, R>::CKF]) {
+// Restores the lane state of a record (`rec` + lane: global or staged in
+// shared memory), rebuilding D, the sums and the normalised frame with the
+// operations lcells used for that row; `d` is the row's D.
+template <int NS, int R, int DM>
+__device__ __forceinline__ void lck_restore(const float* rec, int lane, LState<NS, R>& s, float gO, float gE,
+                                            int nlive, bool hd, float2 (&d)[R / 2]) {
   using L = LDims<NS, R>;
+  constexpr int H = R / 2;
+  float x[L::CKF];
 #pragma unroll
   for (int g = 0; g < L::CK4; ++g) {
     const float4 y = reinterpret_cast<const float4*>(rec + g * 128)[lane];
     x[4 * g] = y.x; x[4 * g + 1] = y.y; x[4 * g + 2] = y.z; x[4 * g + 3] = y.w;
   }
-}
-
-// Restores the lane state of a record.  Affine: D is rebuilt as lcells
-// computed it for that row -- column 0 from the left lane's values (in its
-// frame nl, converted to the row's frame e), column c > 0 from column c - 1
-// of M and D, then zero past the pair -- with the same operations in the
-// same order, so the restored state equals the forward's bit for bit.
-template <int NS, int R>
-__device__ __forceinline__ void lck_unpack(const float (&x)[LDims<NS, R>::CKF], LState<NS, R>& s,
-                                           float gO, float gE, int nlive, bool has_dead) {
-  using L = LDims<NS, R>;
-  constexpr int V = L::NSTORE * R;
 #pragma unroll
-  for (int q = 0; q < L::NSTORE; ++q)
+  for (int q = 0; q < (NS == 3 ? 2 : 1); ++q)
 #pragma unroll
-    for (int c = 0; c < R; ++c) s.v[q][c] = x[q * R + c];
-#pragma unroll
-  for (int q = 0; q < NS; ++q) s.lv[q] = x[V + q];
-  s.e = __float_as_int(x[V + NS]);
-  s.n = __float_as_int(x[V + NS + 1]);
-  s.nl = __float_as_int(x[V + NS + 2]);
+    for (int k = 0; k < H; ++k) s.v[q][k] = make_float2(x[q * R + 2 * k], x[q * R + 2 * k + 1]);
+  constexpr int V = NS == 3 ? 2 * R : R;
+  s.ds = x[V];
+  s.e = __float_as_int(x[V + 1]);
+  s.nd = __float_as_int(x[V + 2]);
+  float rs;
   if constexpr (NS == 3) {
-    const float fL = p2i(s.nl - s.e);
-    const float gOl = gO * fL, gEl = gE * fL;
+    ldchain<NS, R, DM>(s.v[0], x[V + 3], gO, gE, nlive, hd, d, s.od);
 #pragma unroll
-    for (int c = 0; c < R; ++c)
-      s.v[2][c] = c == 0 ? fmaf(gEl, s.lv[2], gOl * s.lv[0]) : fmaf(gE, s.v[2][c - 1], gO * s.v[0][c - 1]);
-    if (has_dead) {
-#pragma unroll
-      for (int c = 0; c < R; ++c)
-        if (c >= nlive) s.v[2][c] = 0.f;
-    }
-  }
-  lstate_sums(s);
-  const float f = p2i(s.e - s.n);
-#pragma unroll
-  for (int q = 0; q < NS; ++q) s.vs[q] = s.v[q][R - 1] * f;
-}
-
-// One step of the forward wavefront for one lane: (xl, xn) is the left
-// lane's last column of this row (normalised frame xn), xs the scaled scores
-// (NEG where the cell does not exist).  Updates the state to this row;
-// returns the step's compute frame in `et` (the raw values' frame) and the
-// row's sum over its columns and states in `rs` (frame et).
-// Affine: M, I, D; linear: A (and, for the adjoint, the emission part em).
-template <int NS, int R>
-__device__ __forceinline__ void lcells(LState<NS, R>& s, const float (&xl)[NS], int xn,
-                                       const float (&xs)[R], bool live, float gO, float gE, int nlive,
-                                       bool has_dead, int& et, float (&em)[R], float& rs) {
-  // diagonal inputs of column 0: the left lane's previous row
-  const int nd = s.nl;
-  float dg[NS];
-#pragma unroll
-  for (int q = 0; q < NS; ++q) { dg[q] = s.lv[q]; s.lv[q] = xl[q]; }
-  s.nl = xn;
-  et = max(max(s.n, xn), nd);
-  // st: the fresh-start term 1 in frame et.  Before the lane's first row every
-  // input of the step is 0, so st = 0 keeps the whole row at 0 (E is finite:
-  // the scores of such rows are 0)
-  const float fU = p2i(s.e - et), fL = p2i(xn - et), fD = p2i(nd - et), st = live ? p2i(-et) : 0.f;
-  float E[R];
-#pragma unroll
-  for (int c = 0; c < R; ++c) E[c] = ex2(xs[c]);
-  if constexpr (NS == 3) {
-    const float gOu = gO * fU, gEu = gE * fU, gOl = gO * fL, gEl = gE * fL;
-    float pS = (dg[0] + dg[1]) + dg[2], fP = fD;   // diagonal (M + I) + D of column 0
-#pragma unroll
-    for (int c = 0; c < R; ++c) {
-      const float oM = s.v[0][c], oI = s.v[1][c];
-      const float m = E[c] * fmaf(fP, pS, st);
-      const float iv = fmaf(gOu, oM, gEu * oI);
-      // D runs along the lane's columns: one fma per column on that chain
-      const float dv = c == 0 ? fmaf(gEl, s.lv[2], gOl * s.lv[0])
-                              : fmaf(gE, s.v[2][c - 1], gO * s.v[0][c - 1]);
-      s.v[0][c] = m; s.v[1][c] = iv; s.v[2][c] = dv;
-      pS = s.cs[c]; fP = fU;   // the previous row's column sum: column c + 1's diagonal
-      em[c] = 0.f;
-    }
-    if (has_dead) {   // columns past the pair: D would run on from the last live column
-#pragma unroll
-      for (int c = 0; c < R; ++c)
-        if (c >= nlive) s.v[2][c] = 0.f;
-    }
+    for (int k = 0; k < H; ++k) s.c[k] = add2(add2(s.v[0][k], s.v[1][k]), d[k]);
+    s.oc = s.c[H - 1].y;
+    rs = sum2(s.c);
   } else {
-    const float gU = gO * fU, gL = gO * fL;
-    float pA = dg[0], fP = fD;
+    s.od = 0.f;
+    s.oc = s.v[0][H - 1].y;
+    rs = sum2(s.v[0]);
+  }
+  s.n = max(s.e - 126 + sexp(rs), 0);
+}
+
+// One step of the forward wavefront for one lane: (xd, xc) are the left
+// lane's outputs of this row in its raw frame xe (normalised frame xn), E the
+// emissions 2^(s k) (0 past the pair).  Updates the state to this row in the
+// frame et (its raw frame from then on) and returns the row's sum over its
+// columns and states in `rs`.
+// Affine: M, I and `d` = D; linear: A and `d` = the emission part.
+template <int NS, int R, int DM>
+__device__ __forceinline__ void lcells(LState<NS, R>& s, float xd, float xc, int xe, int xn,
+                                       const float2 (&E)[R / 2], float gO, float gE, int nlive, bool hd,
+                                       float2 (&d)[R / 2], float& rs) {
+  constexpr int H = R / 2;
+  // the row's frame is at least every input's normalised frame, so that every
+  // converted input is <= 1 (a raw value's frame exceeds its normalised frame
+  // by at most 126)
+  const int et = max(max(s.n, xn), s.nd);
+  s.nd = xn;
+  const int q = 127 - et;
+  const float fU = p2b(s.e + q), fL = p2b(xe + q);
+  const float2 fU2 = dup2(fU), st2 = dup2(p2b(q));   // st: the fresh-start term 1 in frame et
+  if constexpr (NS == 3) {
+    float2 m[H];
 #pragma unroll
-    for (int c = 0; c < R; ++c) {
-      const float oA = s.v[0][c];
-      const float m = E[c] * fmaf(fP, pA, st);
-      const float left = c == 0 ? gL * s.lv[0] : gO * s.v[0][c - 1];
-      const float a = fmaf(gU, oA, m + left);
-      em[c] = m;
-      s.v[0][c] = a;
-      pA = oA; fP = fU;
+    for (int k = 0; k < H; ++k) {
+      const float2 p = k == 0 ? make_float2(s.ds, s.c[H - 1].x) : s.c[k > 0 ? k - 1 : 0];
+      m[k] = mul2(E[k], fma2(fU2, p, st2));
     }
-    if (has_dead) {
+    const float2 gOu = dup2(gO * fU), gEu = dup2(gE * fU);
+#pragma unroll
+    for (int k = 0; k < H; ++k) s.v[1][k] = fma2(gOu, s.v[0][k], mul2(gEu, s.v[1][k]));
+    ldchain<NS, R, DM>(m, xd * fL, gO, gE, nlive, hd, d, s.od);
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+      s.v[0][k] = m[k];
+      s.c[k] = add2(add2(m[k], s.v[1][k]), d[k]);
+    }
+    s.ds = xc * fL;
+    s.oc = s.c[H - 1].y;
+    rs = sum2(s.c);
+  } else {
+    const float2 gU = dup2(gO * fU);
+    float2 x[H];
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+      const float2 p = k == 0 ? make_float2(s.ds, s.v[0][H - 1].x) : s.v[0][k > 0 ? k - 1 : 0];
+      d[k] = mul2(E[k], fma2(fU2, p, st2));
+    }
+#pragma unroll
+    for (int k = 0; k < H; ++k) x[k] = fma2(gU, s.v[0][k], d[k]);
+    s.ds = xc * fL;
+    col(s.v[0], 0) = fmaf(gO, s.ds, col(x, 0));
+#pragma unroll
+    for (int c = 1; c < R; ++c) col(s.v[0], c) = fmaf(gO, col(s.v[0], c - 1), col(x, c));
+    if (masks<DM>(hd)) {
 #pragma unroll
       for (int c = 0; c < R; ++c)
-        if (c >= nlive) { s.v[0][c] = 0.f; em[c] = 0.f; }
+        if (c >= nlive) { col(s.v[0], c) = 0.f; col(d, c) = 0.f; }
     }
+    s.oc = s.v[0][H - 1].y;
+    rs = sum2(s.v[0]);
   }
   // the row sum over columns and states bounds every value of the row (all
-  // are >= 0; it exceeds the largest by at most a factor 3R) and is the row's
-  // partition term
-  lstate_sums(s);
-  float cs[R];
+  // are >= 0) and is the row's partition term
+  s.e = et;
+  s.n = max(1 - q + sexp(rs), 0);
+}
+
+// Scaled scores and emissions of one step as pairs: clamped at XMAX, NEG
+// (E = 0) in columns past the pair.
+template <int R, int DM>
+__device__ __forceinline__ void lemit(const float (&sb)[R], float k, int nlive, bool hd, float2 (&xs)[R / 2],
+                                      float2 (&E)[R / 2]) {
+  constexpr int H = R / 2;
+  float x[R];
 #pragma unroll
-  for (int c = 0; c < R; ++c) {
-    if constexpr (NS == 3) cs[c] = s.cs[c];
-    else cs[c] = s.v[0][c];
+  for (int c = 0; c < R; c += 2) {
+    const float2 t = mul2(make_float2(sb[c], sb[c + 1]), dup2(k));
+    x[c] = fminf(t.x, XMAX);
+    x[c + 1] = fminf(t.y, XMAX);
+  }
+  if (masks<DM>(hd)) {
+#pragma unroll
+    for (int c = 0; c < R; ++c)
+      if (c >= nlive) x[c] = NEG;
   }
 #pragma unroll
-  for (int h = 1; h < R; h *= 2)   // pairwise: a short dependency chain
-#pragma unroll
-    for (int c = 0; c + h < R; c += 2 * h) cs[c] += cs[c + h];
-  rs = cs[0];
-  s.e = et;
-  s.n = max(et + fexp(rs), 0);
-  const float f = p2i(et - s.n);
-#pragma unroll
-  for (int q = 0; q < NS; ++q) s.vs[q] = s.v[q][R - 1] * f;
+  for (int j = 0; j < H; ++j) {
+    xs[j] = make_float2(x[j], x[j + H]);
+    E[j] = make_float2(ex2(x[j]), ex2(x[j + H]));
+  }
 }
+
+// A lane's walk down (or up) the rows of its columns: whole float4 (float2 at
+// 2 columns) pieces when rows are 16-byte aligned (vec; a piece may reach past
+// the pair but not past the row pitch), else one load per column.  A row
+// outside the pair leaves `o` as it was: those values are finite and unused.
+// `fetch` loads without any test, for chunks whose rows are inside for every
+// lane (`inside`): a lane past the pair then reads on into the next rows,
+// which must still belong to the pair, and its columns are not used.
+template <int R> struct Rows {
+  static constexpr int Q = R >= 4 ? 4 : 2;   // columns per piece
+  const float* base;   // row 1, the lane's first column
+  long long ld;
+  int L1, l1a, l1b;    // rows; rows of the first and second piece (0: past the pitch)
+  int nlive;
+  int last;            // the last row whose band width can be read whole
+  bool vec;
+  __device__ __forceinline__ void init(const Pair& pr, int jl, int col0) {
+    base = pr.s + jl;
+    ld = pr.ld;
+    L1 = pr.L1;
+    vec = pr.vec;
+    nlive = min(max(pr.L2 - jl, 0), R);
+    l1a = jl + Q <= pr.ld ? L1 : 0;
+    l1b = jl + 2 * Q <= pr.ld ? L1 : 0;
+    const int over = col0 + 32 * R - pr.ld;   // floats past the row's end
+    last = over > 0 ? L1 - (over + pr.ld - 1) / pr.ld : L1;
+  }
+  // chunk kc's rows are inside the pair for every lane, and reading the whole
+  // band's width of each stays within it
+  __device__ __forceinline__ bool inside(int kc) const { return kc >= 32 / C_STEPS && (kc + 1) * C_STEPS <= last; }
+  template <bool VEC> __device__ __forceinline__ void fetch(const float* p, float (&o)[R]) const {
+    if constexpr (VEC && R == 2) {
+      const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+      o[0] = v.x; o[1] = v.y;
+    } else if constexpr (VEC) {
+#pragma unroll
+      for (int h = 0; h < R / 4; ++h) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(p) + h);
+        o[4 * h] = v.x; o[4 * h + 1] = v.y; o[4 * h + 2] = v.z; o[4 * h + 3] = v.w;
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < R; ++c) o[c] = __ldg(p + c);
+    }
+  }
+  __device__ __forceinline__ const float* at(int i) const { return base + (long long)(i - 1) * ld; }
+  __device__ __forceinline__ void load(const float* p, int i, float (&o)[R]) const {
+    if (vec) {
+      if ((unsigned)(i - 1) < (unsigned)l1a) {
+        if constexpr (R == 2) {
+          const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+          o[0] = v.x; o[1] = v.y;
+        } else {
+          const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+          o[0] = v.x; o[1] = v.y; o[R > 2 ? 2 : 0] = v.z; o[R > 3 ? 3 : 0] = v.w;
+        }
+      }
+      if constexpr (R == 8) {
+        if ((unsigned)(i - 1) < (unsigned)l1b) {
+          const float4 v = __ldg(reinterpret_cast<const float4*>(p) + 1);
+          o[4] = v.x; o[5] = v.y; o[6] = v.z; o[7] = v.w;
+        }
+      }
+    } else if ((unsigned)(i - 1) < (unsigned)L1) {
+#pragma unroll
+      for (int c = 0; c < R; ++c)
+        if (c < nlive) o[c] = __ldg(p + c);
+    }
+  }
+};
+
+// Writes a row of the map for the lane's columns (a row inside the pair):
+// columns past the pair hold 0, and those inside the row pitch are written.
+template <int R>
+__device__ __forceinline__ void store_pairs(float* dst, int jl, const Pair& pr, float2 (&v)[R / 2]) {
+  constexpr int H = R / 2;
+  if (pr.vec) {
+    if constexpr (R == 2) {
+      if (jl + 2 <= pr.ld) *reinterpret_cast<float2*>(dst) = v[0];
+    } else if constexpr (R == 4) {
+      if (jl + 4 <= pr.ld) *reinterpret_cast<float4*>(dst) = make_float4(v[0].x, v[H > 1 ? 1 : 0].x, v[0].y, v[H > 1 ? 1 : 0].y);
+    } else {
+      if (jl + 4 <= pr.ld) reinterpret_cast<float4*>(dst)[0] = make_float4(v[0].x, v[H > 1 ? 1 : 0].x, v[H > 2 ? 2 : 0].x, v[H > 3 ? 3 : 0].x);
+      if (jl + 8 <= pr.ld) reinterpret_cast<float4*>(dst)[1] = make_float4(v[0].y, v[H > 1 ? 1 : 0].y, v[H > 2 ? 2 : 0].y, v[H > 3 ? 3 : 0].y);
+    }
+  } else {
+    if (jl + R <= pr.ld) {
+#pragma unroll
+      for (int c = 0; c < R; ++c) dst[c] = col(v, c);
+    } else {
+#pragma unroll
+      for (int c = 0; c < R; ++c)
+        if (jl + c < pr.ld) dst[c] = col(v, c);
+    }
+  }
+}
+
+// *p (0 where !ok), a strong load; no branch.
+__device__ __forceinline__ float ld_poll_if(const float* p, bool ok) {
+  float v;
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %2, 0;\n mov.b32 %0, 0;\n @p ld.relaxed.gpu.global.f32 %0, [%1];\n}"
+               : "=&f"(v) : "l"(p), "r"((int)ok));
+  return v;
+}
+
+// Edge records, one per row of a band: the last lane's outputs of the row.
+// Affine: one float4 (od, oc, raw frame, normalised frame); linear: one
+// float2 (oc, the two frames packed).  A band's records start at the next
+// 16-byte boundary of its edge slice (2 NS floats per row hold them with the
+// padding; slices start at even offsets).
+template <int NS> struct LEdge {
+  __device__ static __forceinline__ float* base(float* edge, size_t off) {
+    return edge + (NS == 3 ? (off + 3) / 4 * 4 : off);
+  }
+  __device__ static __forceinline__ void put(float* b, int i, float od, float oc, int e, int n, int rs_exp) {
+    if constexpr (NS == 3) {
+      reinterpret_cast<float4*>(b)[i - 1] = make_float4(od, oc, __int_as_float(e), __int_as_float(n));
+    } else {
+      reinterpret_cast<float2*>(b)[i - 1] = make_float2(oc, __uint_as_float(((unsigned)e << 8) | (unsigned)rs_exp));
+    }
+  }
+  // record i (0 where !ok), a strong load; no branch
+  __device__ static __forceinline__ float4 get(const float* b, int i, bool ok) {
+    float4 v;
+    if constexpr (NS == 3) {
+      asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %5, 0;\n mov.b32 %0, 0;\n mov.b32 %1, 0;\n mov.b32 %2, 0;\n"
+                   " mov.b32 %3, 0;\n @p ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];\n}"
+                   : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w) : "l"(b + 4 * (size_t)(i - 1)), "r"((int)ok));
+    } else {
+      v.z = 0.f; v.w = 0.f;
+      asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %3, 0;\n mov.b32 %0, 0;\n mov.b32 %1, 0;\n"
+                   " @p ld.relaxed.gpu.global.v2.f32 {%0, %1}, [%2];\n}"
+                   : "=&f"(v.x), "=&f"(v.y) : "l"(b + 2 * (size_t)(i - 1)), "r"((int)ok));
+    }
+    return v;
+  }
+  __device__ static __forceinline__ bool missing(const float4& v) {
+    if constexpr (NS == 3)
+      return is_sentinel(v.x) || is_sentinel(v.y) || is_sentinel(v.z) || is_sentinel(v.w);
+    else
+      return is_sentinel(v.x) || is_sentinel(v.y);
+  }
+  // (od, oc, e, n) of a resolved record
+  __device__ static __forceinline__ float4 open(const float4& v) {
+    if constexpr (NS == 3) return v;
+    const unsigned w = __float_as_uint(v.y);
+    const int e = (int)(w >> 8);
+    return make_float4(0.f, v.x, __int_as_float(e), __int_as_float(max(e - 126 + (int)(w & 0xffu), 0)));
+  }
+  // Bounded wait for record i; on expiry the status word and the pair's flag
+  // are set and the record reads as 0.
+  __device__ static __noinline__ float4 wait(const float* b, int i, uint64_t deadline, unsigned* status,
+                                             unsigned* flag) {
+    for (int tries = 0;; ++tries) {
+      const float4 v = get(b, i, true);
+      if (!missing(v)) return v;
+      if (gtimer() > deadline) {
+        mark_timeout(status, flag);
+        return make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      if (tries > 16) __nanosleep(SWB_POLL_SLEEP);
+    }
+  }
+};
 
 // Scaled scores of one step, clamped at XMAX; NEG in columns past the pair
 // (E = 0 there).  Rows outside the pair hold scores 0 (load_row).
@@ -383,25 +600,33 @@ __device__ __forceinline__ LParams lparams(const Args& a) {
 // forward band task
 // ---------------------------------------------------------------------------
 
-// Score prefetch distance of the forward (steps; C_STEPS % SWB_FPF == 0).  A
-// whole chunk: each row is requested a chunk before its step (measured on the
-// 4096-pair bench batch at 8 columns per lane: forward 2.27 ms at 4 steps,
-// 2.59 at 2, 3.05 at 1).
-#ifndef SWB_FPF
-#define SWB_FPF SWB_C_STEPS
-#endif
-constexpr int FPF = SWB_FPF;
-static_assert(C_STEPS % FPF == 0, "the forward's prefetch distance must divide the chunk");
+// Score prefetch distance of the tangent kernels' forward (steps).
+constexpr int FPF = C_STEPS;
+// Score prefetch distance of the sweeps (steps): each row is requested this
+// many steps ahead; the narrow kernels, whose steps are shorter, look further.
+template <int R> __host__ __device__ constexpr int fwd_ahead() { return R == 8 ? 4 : 8; }
+// Steps per block of the forward: the left band's records are passed a block
+// at a time (about 220 cycles a time in a lone warp).
+template <int R> __host__ __device__ constexpr int fwd_block() { return split_code<R>() ? 2 * C_STEPS : C_STEPS; }
 
-// Forward wavefront of one band: per-lane partition sums (Kahan, in the
-// lane's largest normalised frame), the left-to-right edge records
-// (last column normalised, then its frame) and, every C steps, a checkpoint
-// of the lane state plus the chunk's largest normalised frame.  The band's
-// partition partial is (frame, mantissa sum): Z_band = sum * 2^frame.
-template <int NS, int R>
+// Forward wavefront of one band: per-lane partition sums (plain within a
+// chunk, Kahan over chunks, in the lane's largest normalised frame), the
+// left-to-right edge records and, every C steps, a checkpoint of the lane
+// state plus the chunk's largest normalised frame.  The band's partition
+// partial is (frame, mantissa sum): Z_band = sum * 2^frame.
+//
+// The left band's records of a block (WB steps) pass through shared memory,
+// where lane 0 reads the one of each step.  They are requested two blocks
+// ahead and put there one block ahead, two buffers in turn, so a block whose
+// records had been written by then starts without waiting for anything.
+//
+// DM (see above): 1 also where rows are not 16-byte aligned.
+template <int NS, int R, int DM>
 __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int lane,
                           uint64_t deadline, float4* sedge) {
   using LD = LDims<NS, R>;
+  using LE = LEdge<NS>;
+  constexpr int H = R / 2, AH = fwd_ahead<R>(), WB = fwd_block<R>();
   check_lengths(a, w, lane);
   if (!lp.ok && w.band == 0 && lane == 0) {
     atomicOr(a.status, ERR_BAD_PARAMS);
@@ -419,132 +644,150 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
   }
   const int jl = col0 + lane * R;
   const int nlive = min(max(L2 - jl, 0), R);
-  const bool has_dead = __any_sync(FULL, nlive < R);
+  const bool hd = col0 + 32 * R > L2;
   const float k = lp.k, gO = lp.xgo, gE = lp.xge;
-  const size_t Lm = (size_t)w.Lm;
-  float* eout = a.edge + w.ed0 + (size_t)band * w.edb;
-  const float* ein = (band > 0) ? eout - w.edb : nullptr;
+  float* eout = LE::base(a.edge, w.ed0 + (size_t)band * w.edb);
   const bool fault = a.fault_inject && band > 0;
-  if (fault) ein = nullptr;
+  const float* ein = (band > 0 && !fault) ? LE::base(a.edge, w.ed0 + (size_t)(band - 1) * w.edb) : nullptr;
   const bool keep_ck = a.ckpt != nullptr;
   float* ck = keep_ck ? a.ckpt + w.ck0 + (size_t)band * w.ckb : nullptr;
   const int nch = band_chunks(L1);
   const int KC = a.ck_every;
   float* ckmax = keep_ck ? ck + (size_t)((nch + KC - 1) / KC) * LD::LREC : nullptr;
+  int next_ck = 0;   // the next chunk whose record is kept
 
   LState<NS, R> s;
   lstate_zero(s);
+  float2 d[H];
+#pragma unroll
+  for (int j = 0; j < H; ++j) d[j] = dup2(0.f);
   float zm = (band == 0 && lane == 0) ? 1.f : 0.f, zc = 0.f;   // M[0,0]: the empty alignment
   int ze = 0;
 
-  // lane u < C holds the left band's edge record lane 0 needs at step u of a
-  // chunk (NS values, then the frame), loaded one chunk ahead
-  constexpr int NEF = NS + 1;
-  float eb[NEF], ebn[NEF];
-  auto load_edge = [&](int kc, float (&dst)[NEF]) {
-    const int i = kc * C_STEPS + lane + 1;
-    const bool ok = ein && lane < C_STEPS && i <= L1;
-#pragma unroll
-    for (int f = 0; f < NEF; ++f) dst[f] = ok ? ld_poll(ein + f * Lm + (i - 1)) : 0.f;
+  // lane u < WB holds the left band's edge record lane 0 needs at step u of a
+  // block: `ea` of the next block, `eb` of the one after
+  auto get_edge = [&](int bl) {
+    const int ie = bl * WB + lane + 1;
+    return LE::get(ein, ie, ein && lane < WB && ie <= L1);
   };
-  load_edge(0, eb);
+  float4 ea = get_edge(0), eb = get_edge(1);
+  bool ready = false;   // this block's records are in shared memory
+  Rows<R> rows;
+  rows.init(pr, jl, col0);
+  const float* src = rows.at(1 - lane);
+  float sb[AH][R];   // per-lane score ring, AH steps ahead
 #pragma unroll
-  for (int f = 0; f < NEF; ++f) ebn[f] = 0.f;
-  float sb[FPF][R];   // per-lane score ring, FPF steps ahead
+  for (int u = 0; u < AH; ++u) {
 #pragma unroll
-  for (int u = 0; u < FPF; ++u) {
-    const int i = u - lane + 1;
-    load_row<R>(pr, i, jl, i >= 1 && i <= L1, sb[u]);
+    for (int c = 0; c < R; ++c) sb[u][c] = 0.f;
+    rows.load(src, u - lane + 1, sb[u]);
+    src += rows.ld;
   }
 
-  for (int kc = 0; kc < nch; ++kc) {
-    // resolve this chunk's edge records before its first step: lane u < C
-    // polls its own record until the left band has written it (one bounded
-    // wait per chunk, not per row); fault injection waits on a word nobody
-    // writes and substitutes zeros
-    {
-      const int ie = kc * C_STEPS + lane + 1;
-      const bool mine = lane < C_STEPS && ie <= L1;
-      bool miss = false;
-#pragma unroll
-      for (int f = 0; f < NEF; ++f) miss |= is_sentinel(eb[f]);
-      miss = miss && ein && mine;
-      if (__any_sync(FULL, miss || (fault && mine))) {
-        if (fault && mine) {
-          poll_value(a.never_written, ld_poll(a.never_written), deadline, a.status, a.pair_done + w.p,
-                     0.f);
-#pragma unroll
-          for (int f = 0; f < NEF; ++f) eb[f] = 0.f;
-        } else if (miss) {
-          FieldVec<NEF> x;
-#pragma unroll
-          for (int f = 0; f < NEF; ++f) x.v[f] = eb[f];
-          x = poll_fields_v<NEF, 0>(x, ein + (ie - 1), Lm, deadline, a.status, a.pair_done + w.p);
-#pragma unroll
-          for (int f = 0; f < NEF; ++f) eb[f] = x.v[f];
-        }
-      }
-    }
-    // the resolved records go to shared memory, where lane 0 reads the one of
-    // each step (one load instead of NS + 1 shuffles per step)
-    __syncwarp();
-    if (lane < C_STEPS) sedge[lane] = make_float4(eb[0], eb[1], eb[NEF > 2 ? 2 : 0], eb[NEF > 3 ? 3 : 0]);
-    __syncwarp();
-    if (keep_ck && kc % KC == 0) lck_store<NS, R>(ck + (size_t)(kc / KC) * LD::LREC, lane, s);
-    int cmx = -(1 << 30);   // largest normalised frame of the lane's live rows in this chunk
-    if (kc + 1 < nch) load_edge(kc + 1, ebn);
+  int i = 1 - lane;   // the lane's row at the next step
 #pragma unroll 1
-    for (int u0 = 0; u0 < C_STEPS; u0 += FPF)
-#pragma unroll
-    for (int u = 0; u < FPF; ++u) {
-      const int cu = u0 + u;
-      const int t = kc * C_STEPS + cu;
-      const int i = t - lane + 1;
-      const bool act = (i >= 1) && (i <= L1);
-      float xl[NS];
-#pragma unroll
-      for (int q = 0; q < NS; ++q) xl[q] = __shfl_up_sync(FULL, s.vs[q], 1);
-      int xn = __shfl_up_sync(FULL, s.n, 1);
-      if (lane == 0) {   // the chunk's records are resolved (0 where there is no left band)
-        const float4 e4 = sedge[cu];
-        const float ev[4] = {e4.x, e4.y, e4.z, e4.w};
-#pragma unroll
-        for (int q = 0; q < NS; ++q) xl[q] = act ? ev[q] : 0.f;
-        xn = act ? __float_as_int(ev[NS]) : 0;
+  for (int bl = 0; bl * WB < nch * C_STEPS; ++bl) {
+    float4* se = sedge + (bl & 1) * WB;
+    __syncwarp();   // the buffers: the last block's reads are done, its writes are seen
+    if (!ready) {
+      // wait for the block's records: lane u < WB polls its own until the left
+      // band has written it (one bounded wait per block, not per row); fault
+      // injection waits on a word nobody writes and substitutes zeros
+      const int ie = bl * WB + lane + 1;
+      const bool mine = lane < WB && ie <= L1;
+      if (fault) {
+        if (mine)
+          poll_value(a.never_written, ld_poll(a.never_written), deadline, a.status, a.pair_done + w.p, 0.f);
+      } else if (ein && mine && LE::missing(ea)) {
+        ea = LE::wait(ein, ie, deadline, a.status, a.pair_done + w.p);
       }
-      float xs[R];
-      lscores<R>(sb[u], k, nlive, has_dead, xs);
-      {
-        const int ip = i + FPF;
-        load_row<R>(pr, ip, jl, ip >= 1 && ip <= L1, sb[u]);
-      }
-      int et;
-      float em[R], rs;
-      lcells<NS, R>(s, xl, xn, xs, i >= 1, gO, gE, nlive, has_dead, et, em, rs);
-      if (act) {
-        // partition: the row's live values (dead columns are 0) in the frame
-        // ze (the largest normalised frame so far), Kahan-compensated
-        if (s.n > ze) {
-          const float f = p2i(ze - s.n);
-          zm *= f; zc *= f; ze = s.n;
-        }
-        const float y = rs * p2i(et - ze) - zc;
-        const float tt = zm + y;
-        zc = (tt - zm) - y;
-        zm = tt;
-        cmx = max(cmx, s.n);
-        if (lane == 31) {
+      __syncwarp();
+      if (lane < WB) se[lane] = LE::open(ea);
+      __syncwarp();
+    }
+    // the next block's records, if they are there (fault injection: never)
+    ready = __all_sync(FULL, !LE::missing(eb)) && !fault;
+    if (ready && lane < WB) sedge[((bl + 1) & 1) * WB + lane] = LE::open(eb);
+    ea = eb;
+    eb = get_edge(bl + 2);
+    const bool in_block = rows.inside(bl * (WB / C_STEPS)) && rows.inside((bl + 1) * (WB / C_STEPS) - 1 + AH / C_STEPS);
 #pragma unroll
-          for (int q = 0; q < NS; ++q) eout[q * Lm + (i - 1)] = s.vs[q];
-          eout[NS * Lm + (i - 1)] = __int_as_float(s.n);
+    for (int h = 0; h < WB / C_STEPS; ++h) {
+    const int kc = bl * (WB / C_STEPS) + h;
+    if (keep_ck && kc == next_ck && kc < nch) {
+      lck_store<NS, R>(ck, lane, s, col(d, 0));
+      ck += LD::LREC;
+      next_ck += KC;
+    }
+    int cmx = -(1 << 30);   // largest normalised frame of the lane's live rows in this chunk
+    float rsv[C_STEPS];
+    int ev[C_STEPS];
+    // the chunk's steps.  Inside chunks (every lane on a row of the pair, now
+    // and for the rows requested) run without a branch, so that the steps'
+    // loads, emissions and chains overlap
+    auto steps = [&](auto inside_c, auto vec_c) {
+      constexpr bool IN = decltype(inside_c)::value, VEC = decltype(vec_c)::value;
+      constexpr int DD = IN || DM == 2 ? DM : 1;
+#pragma unroll
+      for (int cu = 0; cu < C_STEPS; ++cu) {
+        const bool act = IN || (unsigned)(i + cu - 1) < (unsigned)L1;
+        const float4 e4 = se[h * C_STEPS + cu];   // 0 where there is no left band
+        float xd = 0.f;
+        if constexpr (NS == 3) {
+          xd = __shfl_up_sync(FULL, s.od, 1);
+          xd = lane == 0 ? e4.x : xd;
         }
+        float xc = __shfl_up_sync(FULL, s.oc, 1);
+        int xe = __shfl_up_sync(FULL, s.e, 1);
+        int xn = __shfl_up_sync(FULL, s.n, 1);
+        xc = lane == 0 ? e4.y : xc;
+        xe = lane == 0 ? __float_as_int(e4.z) : xe;
+        xn = lane == 0 ? __float_as_int(e4.w) : xn;
+        float2 xs[H], E[H];
+        lemit<R, DD>(sb[(h * C_STEPS + cu) % AH], k, nlive, hd, xs, E);
+        if constexpr (IN) rows.template fetch<VEC>(src, sb[(h * C_STEPS + cu) % AH]);
+        else rows.load(src, i + cu + AH, sb[(h * C_STEPS + cu) % AH]);
+        src += rows.ld;
+        rsv[cu] = 0.f;
+        ev[cu] = 0;
+        if (act) {
+          lcells<NS, R, DD>(s, xd, xc, xe, xn, E, gO, gE, nlive, hd, d, rsv[cu]);
+          ev[cu] = s.e;
+          cmx = max(cmx, s.n);
+          if (lane == 31) LE::put(eout, i + cu, s.od, s.oc, s.e, s.n, sexp(rsv[cu]));
+        }
+      }
+    };
+    bool done = false;
+    if constexpr (split_code<R>()) {
+      if (in_block) {
+        done = true;
+        if (DM != 1 || rows.vec) steps(std::true_type{}, std::true_type{});
+        else if constexpr (DM == 1) steps(std::true_type{}, std::false_type{});
       }
     }
+    if (!done) steps(std::false_type{}, std::false_type{});
+    i += C_STEPS;
+    // partition: the chunk's row sums in the frame ze (the largest normalised
+    // frame so far), Kahan-compensated from chunk to chunk
+    {
+      const int zn = max(ze, cmx);
+      const float f = p2b(ze - zn + 127);
+      float y = 0.f;
 #pragma unroll
-    for (int f = 0; f < NEF; ++f) eb[f] = ebn[f];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cmx = max(cmx, __shfl_xor_sync(FULL, cmx, o));
-    if (keep_ck && lane == 0) ckmax[kc] = __int_as_float(cmx);
+      for (int cu = 0; cu < C_STEPS; ++cu) y = fmaf(rsv[cu], p2b(ev[cu] - zn + 127), y);
+      zm *= f;
+      y -= zc * f;
+      const float tt = zm + y;
+      zc = (tt - zm) - y;
+      zm = tt;
+      ze = zn;
+    }
+    if (keep_ck) {
+      cmx = __reduce_max_sync(FULL, cmx);
+      if (lane == 0 && kc < nch) ckmax[kc] = __int_as_float(cmx);
+    }
+    }
   }
   // warp-combine (frame, sum) pairs, fixed shuffle tree
 #pragma unroll
@@ -559,11 +802,11 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
 }
 
 #ifndef SWB_LFWD_MINB
-#define SWB_LFWD_MINB 5
+#define SWB_LFWD_MINB 4
 #endif
 template <int NS, int R>
 __global__ void __launch_bounds__(128, (R >= 8 ? 4 : SWB_LFWD_MINB)) lfwd_kernel(Args a) {
-  __shared__ float4 s_edge[4][C_STEPS];   // per warp: the left band's records of a chunk
+  __shared__ float4 s_edge[4][2 * fwd_block<R>()];   // per warp: the left band's records of two blocks
   const int lane = threadIdx.x & 31;
   const LParams lp = lparams<NS>(a);
   const uint64_t deadline = gtimer() + a.spin_limit_ns;
@@ -573,7 +816,12 @@ __global__ void __launch_bounds__(128, (R >= 8 ? 4 : SWB_LFWD_MINB)) lfwd_kernel
     if (lane == 0) task = (int)atomicAdd(a.counters + 0, 1u);
     task = __shfl_sync(FULL, task, 0);
     if (task >= ntasks) break;
-    lfwd_band<NS, R>(a, lp, place_of<NS, R>(a, task, false), lane, deadline, s_edge[threadIdx.x >> 5]);
+    const Place w = place_of<NS, R>(a, task, false);
+    // a band whose last columns lie past the pair takes the variant that masks them
+    float4* se = s_edge[threadIdx.x >> 5];
+    if constexpr (!split_code<R>()) lfwd_band<NS, R, 2>(a, lp, w, lane, deadline, se);
+    else if ((w.band + 1) * 32 * R > w.pr.L2 || !w.pr.vec) lfwd_band<NS, R, 1>(a, lp, w, lane, deadline, se);
+    else lfwd_band<NS, R, 0>(a, lp, w, lane, deadline, se);
   }
 }
 
@@ -664,9 +912,292 @@ __host__ __device__ constexpr int lbwd_smem_floats() {
   return (C_STEPS * LDims<NS, R>::FW + LDims<NS, R>::CKF) * 32 + 2 * C_STEPS * 4;
 }
 
+// Lane state of the outside recursion: the row below and the right
+// neighbour's held value.
+template <int R> struct BState {
+  static constexpr int H = R / 2;
+  float2 b[H];      // beta_I (linear: beta) of the lane's latest row, raw (frame fb)
+  float2 t[H];      // t = E beta_M of that row (normalised frame nb)
+  float ht, ob;     // the right neighbour's held t (frame hn); beta_D (beta) of column 0 (frame nb)
+  int fb, nb, hn;
+};
+template <int R> __device__ __forceinline__ void bstate_zero(BState<R>& s) {
+#pragma unroll
+  for (int k = 0; k < R / 2; ++k) { s.b[k] = dup2(0.f); s.t[k] = dup2(0.f); }
+  s.ht = 0.f; s.ob = 0.f;
+  s.fb = 0; s.nb = 0; s.hn = 0;
+}
+
+// The state as a record ([group][lane][4] floats).
+template <int R> struct BDims {
+  static constexpr int BKF = (2 * R + 5 + 3) / 4 * 4;
+  static constexpr int BREC = BKF * 32;
+};
+template <int R>
+__device__ __forceinline__ void bstate_store(float* rec, int lane, const BState<R>& s) {
+  constexpr int H = R / 2, K = BDims<R>::BKF;
+  float x[K];
+#pragma unroll
+  for (int k = 0; k < H; ++k) {
+    x[2 * k] = s.b[k].x; x[2 * k + 1] = s.b[k].y;
+    x[R + 2 * k] = s.t[k].x; x[R + 2 * k + 1] = s.t[k].y;
+  }
+  x[2 * R] = s.ht;
+  x[2 * R + 1] = s.ob;
+  x[2 * R + 2] = __int_as_float(s.fb);
+  x[2 * R + 3] = __int_as_float(s.nb);
+  x[2 * R + 4] = __int_as_float(s.hn);
+#pragma unroll
+  for (int f = 2 * R + 5; f < K; ++f) x[f] = 0.f;
+#pragma unroll
+  for (int g = 0; g < K / 4; ++g)
+    reinterpret_cast<float4*>(rec + g * 128)[lane] = make_float4(x[4 * g], x[4 * g + 1], x[4 * g + 2], x[4 * g + 3]);
+}
+template <int R>
+__device__ __forceinline__ void bstate_load(const float* rec, int lane, BState<R>& s) {
+  constexpr int H = R / 2, K = BDims<R>::BKF;
+  float x[K];
+#pragma unroll
+  for (int g = 0; g < K / 4; ++g) {
+    const float4 y = reinterpret_cast<const float4*>(rec + g * 128)[lane];
+    x[4 * g] = y.x; x[4 * g + 1] = y.y; x[4 * g + 2] = y.z; x[4 * g + 3] = y.w;
+  }
+#pragma unroll
+  for (int k = 0; k < H; ++k) {
+    s.b[k] = make_float2(x[2 * k], x[2 * k + 1]);
+    s.t[k] = make_float2(x[R + 2 * k], x[R + 2 * k + 1]);
+  }
+  s.ht = x[2 * R];
+  s.ob = x[2 * R + 1];
+  s.fb = __float_as_int(x[2 * R + 2]);
+  s.nb = __float_as_int(x[2 * R + 3]);
+  s.hn = __float_as_int(x[2 * R + 4]);
+}
+
+// The gradient sums of a band are formed per segment of kSeg chunks (plain
+// sums per lane, then a shuffle tree) and folded over the segments, last one
+// first, with compensation: the adjoint of a whole band and the segment
+// kernel give the same bits.
+constexpr int kSeg = 4;
+struct BandSum {
+  KSum a, b, m;
+  __device__ __forceinline__ void add(float x, float y, float z) {
+    if (x != 0.f || y != 0.f || z != 0.f) { a.add(x); b.add(y); m.add(z); }
+  }
+};
+
+// End of a segment: its gradient partials; the pair's last segment folds them
+// (lane l the bands l, l + 32, ...; then the bands in order).
+template <int NS>
+__device__ __forceinline__ void lfinish_seg(const Args& a, const Place& w, int lane, int seg, float Sh, float Sl,
+                                            float g0, float g1, float ps, PParams pp) {
+  const int p = w.p;
+  unsigned done = 0;
+  if (lane == 0) {
+    reinterpret_cast<float4*>(a.spart)[(w.slot0 + w.band) * a.nseg + seg] = make_float4(g0, g1, ps, 0.f);
+    __threadfence();
+    done = atomicAdd(a.pair_done + p, 1u);
+  }
+  done = __shfl_sync(FULL, done, 0);
+  if ((done & ~PAIR_TIMEOUT) != (unsigned)(w.nb * a.nseg) - 1) return;
+  __threadfence();
+  float o = 0.f, e = 0.f, m = 0.f;
+  for (int b0 = 0; b0 < w.nb; b0 += 32) {
+    BandSum s;
+    if (b0 + lane < w.nb) {
+      const float* x = a.spart + 4 * (w.slot0 + b0 + lane) * a.nseg;
+      for (int q = a.nseg - 1; q >= 0; --q) s.add(ld_poll(x + 4 * q), ld_poll(x + 4 * q + 1), ld_poll(x + 4 * q + 2));
+    }
+    for (int b = 0; b < min(32, w.nb - b0); ++b) {
+      o += __shfl_sync(FULL, s.a.s, b);
+      e += __shfl_sync(FULL, s.b.s, b);
+      m += __shfl_sync(FULL, s.m.s, b);
+    }
+  }
+  if (lane != 0) return;
+  if (done & PAIR_TIMEOUT) {   // a bounded wait of this pair expired
+    const float nan = __int_as_float(0x7fc00000);
+    a.value[p] = nan; a.g_open[p] = nan; a.g_T[p] = nan;
+    if (a.g_ext) a.g_ext[p] = nan;
+    return;
+  }
+  const float inv_k = 1.f / pp.k;         // = T * ln 2
+  const float S = (Sh + Sl) * inv_k, match = m * inv_k;
+  a.value[p] = S;
+  a.g_open[p] = o;
+  if (a.g_ext) a.g_ext[p] = NS == 3 ? e : 0.f;
+  a.g_T[p] = NS == 3 ? (S - (match + (o * pp.go + e * pp.ge))) / pp.T : (S - (match + o * pp.go)) / pp.T;
+}
+
+// One row of the outside recursion for one lane: (rb, rt, rn) are the right
+// lane's beta_D (linear: beta) of its column 0, its t and its normalised
+// frame; live: the row is inside the pair.  Returns, in the frame `ft`: vm =
+// beta_M (beta), sr = beta_I below + beta_D right and br = beta_D right per
+// column.  The state moves on with bfinish.
+template <int NS, int R, int DM>
+__device__ __forceinline__ void bcells(const BState<R>& s, float rb, int rn, bool live, float gO, float gE,
+                                       float gX, int nlive, bool hd, int& ft, float& fB,
+                                       float2 (&vm)[R / 2], float2 (&vi)[R / 2], float2 (&sr)[R / 2],
+                                       float2 (&br)[R / 2], float& vd0, float& mx) {
+  constexpr int H = R / 2;
+  // frames: the row is computed in ft >= every input's normalised frame
+  ft = max(max(s.nb, rn), s.hn);
+  const int q = 127 - ft;
+  fB = p2b(s.fb + q);
+  const float fT = p2b(s.nb + q), fR = p2b(rn + q), fH = p2b(s.hn + q);
+  const float one = live ? p2b(q) : 0.f;
+  float2 base[H];
+#pragma unroll
+  for (int k = 0; k < H; ++k) {   // 1 plus the diagonal successor's t
+    float2 oc = dup2(one);
+    if (masks<DM>(hd)) oc = make_float2(k < nlive ? one : 0.f, k + H < nlive ? one : 0.f);
+    base[k] = k == H - 1 ? fma2(make_float2(fT, fH), make_float2(s.t[0].y, s.ht), oc)
+                         : fma2(dup2(fT), s.t[k < H - 1 ? k + 1 : 0], oc);
+  }
+  const float b0 = fR * rb;   // right successor's beta_D (beta) of the last column
+  float2 v[H];                // beta_D (beta) per column
+  if constexpr (NS == 3) {
+    col(v, R - 1) = fmaf(gE, b0, col(base, R - 1));
+#pragma unroll
+    for (int c = R - 2; c >= 0; --c) col(v, c) = fmaf(gE, col(v, c + 1), col(base, c));
+  } else {
+    float2 x[H];
+    const float2 gOb = dup2(gO * fB);
+#pragma unroll
+    for (int k = 0; k < H; ++k) x[k] = fma2(gOb, s.b[k], base[k]);
+    col(v, R - 1) = fmaf(gO, b0, col(x, R - 1));
+#pragma unroll
+    for (int c = R - 2; c >= 0; --c) col(v, c) = fmaf(gO, col(v, c + 1), col(x, c));
+  }
+  vd0 = v[0].x;
+#pragma unroll
+  for (int k = 0; k < H; ++k) {
+    br[k] = k == H - 1 ? make_float2(v[0].y, b0) : v[k < H - 1 ? k + 1 : 0];
+    sr[k] = fma2(dup2(fB), s.b[k], br[k]);
+  }
+  float2 m[H];
+  if constexpr (NS == 3) {
+    const float2 gEb = dup2(gE * fB);
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+      vm[k] = fma2(dup2(gO), sr[k], base[k]);
+      vi[k] = fma2(gEb, s.b[k], base[k]);
+      m[k] = fma2(dup2(gX), sr[k], base[k]);   // >= beta_M, beta_I, beta_D
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < H; ++k) { vm[k] = v[k]; vi[k] = v[k]; m[k] = v[k]; }
+  }
+  float x[R];
+#pragma unroll
+  for (int c = 0; c < R; ++c) x[c] = col(m, c);
+#pragma unroll
+  for (int h = 1; h < R; h *= 2)
+#pragma unroll
+    for (int c = 0; c + h < R; c += 2 * h) x[c] = fmaxf(x[c], x[c + h]);
+  mx = x[0];
+}
+
+// The state after the row: t = E beta_M in the row's normalised frame.
+template <int R>
+__device__ __forceinline__ void bfinish(BState<R>& s, int ft, float mx, const float2 (&vm)[R / 2],
+                                        const float2 (&vi)[R / 2], float vd0, const float2 (&E)[R / 2],
+                                        float rt, int rn) {
+  constexpr int H = R / 2;
+  const int nn = max(ft - 126 + sexp(mx), 0);
+  const float bs = p2b(ft - nn + 127);
+#pragma unroll
+  for (int k = 0; k < H; ++k) {
+    s.t[k] = mul2(mul2(vm[k], dup2(bs)), E[k]);
+    s.b[k] = vi[k];
+  }
+  s.fb = ft;
+  s.nb = nn;
+  s.ob = vd0 * bs;
+  s.ht = rt;
+  s.hn = rn;
+}
+
+// ---- quiet chunks.  For a cell u of a chunk, alpha_u beta_u / Z sums, over
+// the chunk cells x where u's continuations stay inside, terms
+// alpha_x (1 + w beta_out) / Z (alpha_u W(u -> x) <= alpha_x: all weights are
+// positive), where beta_out are the successors outside the chunk: the row
+// below, the right neighbour's held t and, for lane 31, the right band's
+// records.  With at most 2^9 cells, alpha_x <= 2^ckm and
+// 1 + w beta_out <= 4 max(1, inflow), every posterior in the chunk and every
+// flow across its top and left edges is below 2^-SWB_LQUIET when
+// ckm + 11 + max(log2 inflow, 0) < log2 Z - SWB_LQUIET.  Such a chunk has zero
+// map rows and zero records to the left band, and passes zero beta up: the
+// flows it drops are among those bounded.  The right band's records are
+// resolved first, so the decision does not depend on timing.  zlog: log2 of Z
+// less SWB_LQUIET; pb: lane u < C the record of backward step u. ----
+template <int R>
+__device__ __forceinline__ bool lquiet(const BState<R>& s, int ckm, const float (&pb)[3], int lane, int zlog) {
+  int inl = s.hn + fexp(s.ht);
+  float mb = 0.f, mt = 0.f;   // largest beta and t of the row below
+#pragma unroll
+  for (int j = 0; j < R / 2; ++j) {
+    mb = fmaxf(mb, fmaxf(s.b[j].x, s.b[j].y));
+    mt = fmaxf(mt, fmaxf(s.t[j].x, s.t[j].y));
+  }
+  inl = max(inl, max(s.fb + fexp(mb), s.nb + fexp(mt)));
+  if (lane < C_STEPS) inl = max(inl, __float_as_int(pb[2]) + fexp(fmaxf(pb[0], pb[1])));
+  return __all_sync(FULL, ckm + 11 + max(inl, 0) < zlog);
+}
+// ---- quiet run.  After a quiet chunk only lane 31's held t (pt, pn) and the
+// right band's records enter the chunks above, so one round of loads decides
+// the next 32 / C chunks: lane l takes chunk kn - l / C at backward step
+// l % C (lane 31's row there), checking that record and the one of the row
+// below (lane l - 1's; lane 0: the held t).  A record not written yet ends
+// the run; that chunk is then decided by lquiet from the same values, so
+// results do not depend on timing.  Returns how many chunks from kn down (not
+// below k_lo) are quiet; r1, rn: the lane's record's t and frame. ----
+__device__ __forceinline__ int lquiet_run(const float* pin, size_t Lm, int L1, const float* ckmax, int kn, int k_lo,
+                                          int lane, float pt, int pn, int zlog, float& r1, int& rn) {
+  constexpr int RUN = 32 / C_STEPS;
+  const int j = lane / C_STEPS, u = lane - j * C_STEPS;
+  const int kq = kn - j;
+  float r0 = 0.f;
+  int cm = -(1 << 30);
+  bool written = true;
+  r1 = 0.f;
+  rn = 0;
+  if (kq >= k_lo) {
+    const int ir = kq * C_STEPS + C_STEPS - 1 - u - 30;
+    if (pin && ir >= 1 && ir <= L1) {
+      r0 = ld_poll(pin + 0 * (Lm + 1) + ir);
+      r1 = ld_poll(pin + 1 * (Lm + 1) + ir);
+      const float r2 = ld_poll(pin + 2 * (Lm + 1) + ir);
+      written = !is_sentinel(r0) && !is_sentinel(r1) && !is_sentinel(r2);
+      rn = __float_as_int(r2);
+    }
+    cm = __float_as_int(ckmax[kq]);
+  }
+  const int lg = written ? rn + fexp(fmaxf(r0, r1)) : 0;
+  const int lgu = __shfl_up_sync(FULL, lg, 1);
+  const bool wu = __shfl_up_sync(FULL, (int)written, 1) != 0;
+  const int lgb = lane == 0 ? pn + fexp(pt) : lgu;
+  const bool wb = lane == 0 || wu;
+  const bool q = kq >= k_lo && written && wb && cm + 11 + max(max(lg, lgb), 0) < zlog;
+  const unsigned ball = __ballot_sync(FULL, q);
+  constexpr unsigned grp = (1u << C_STEPS) - 1u;
+  int n = 0;
+  while (n < RUN && kn - n >= k_lo && ((ball >> (n * C_STEPS)) & grp) == grp) ++n;
+  return n;
+}
+// Zero records to the left band for the rows of chunk kq (lane 0's).
+__device__ __forceinline__ void zero_push(float* pout, size_t Lm, int L1, int kq, int lane) {
+  const int i = kq * C_STEPS + lane + 1;
+  if (pout && lane < C_STEPS && i <= L1) {
+    pout[0 * (Lm + 1) + i] = 0.f;
+    pout[1 * (Lm + 1) + i] = 0.f;
+    pout[2 * (Lm + 1) + i] = 0.f;
+  }
+}
+
 // Per band, checkpoint chunks in reverse.  Each chunk restores its checkpoint
 // and recomputes C steps of the forward, keeping every cell's raw values and
-// scaled score (and each step's frames) in shared memory; then the outside
+// scaled score (and each step's frame) in shared memory; then the outside
 // recursion runs the same C steps backwards.  Lane l + 1 is one step ahead of
 // lane l (it processes row i one step earlier); a lane receives from its right
 // neighbour that row's beta_D (beta, linear) of column 0 in the neighbour's
@@ -676,11 +1207,17 @@ __host__ __device__ constexpr int lbwd_smem_floats() {
 // buffer; lane 31 reads the right band's.  No atomics; the map is written row
 // by row (a quiet chunk writes its zero rows in whole row pieces); the
 // gradient sums are folded per pair in band order.
-template <int NS, int R, bool SPARSE = false>
+//
+// SEG: one segment of the band, chunks [k_lo, k_hi), starting from the state
+// the outside sweep (lbeta_band) kept for it; every record it reads has been
+// written by then, and it passes none on.
+template <int NS, int R, bool SPARSE, int DM, bool SEG = false>
 __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int lane, float* sm,
-                          uint64_t deadline) {
+                          uint64_t deadline, int seg = 0) {
   using LD = LDims<NS, R>;
-  constexpr int CKF = LD::CKF, LREC = LD::LREC, FW = LD::FW, NEF = NS + 1, NPF = 3;
+  using LE = LEdge<NS>;
+  constexpr int H = R / 2;
+  constexpr int CKF = LD::CKF, LREC = LD::LREC, FW = LD::FW, NPF = 3;
   const Pair& pr = w.pr;
   const int L1 = pr.L1, L2 = pr.L2;
   const int band = w.band;
@@ -690,22 +1227,24 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
   lpair_z(a, w, lane, ze, zm);
   lz_log2(ze, zm, Sh, Sl);
   const PParams pp{lp.go, lp.ge, lp.T, lp.k};
-  if (!(L1 > 0 && col0 < L2)) {
-    finish_pair_p<NS>(a, w, lane, Sh, Sl, 0.f, 0.f, 0.f, pp);
+  const int nch = band_chunks(L1);
+  const int k_lo = SEG ? seg * kSeg : 0, k_hi = SEG ? min(k_lo + kSeg, nch) : nch;
+  if (!(L1 > 0 && col0 < L2) || k_lo >= k_hi) {
+    if constexpr (SEG) lfinish_seg<NS>(a, w, lane, seg, Sh, Sl, 0.f, 0.f, 0.f, pp);
+    else finish_pair_p<NS>(a, w, lane, Sh, Sl, 0.f, 0.f, 0.f, pp);
     return;
   }
   const float invZ = 1.f / zm;
   const int jl = col0 + lane * R;
   const int nlive = min(max(L2 - jl, 0), R);
-  const bool has_dead = __any_sync(FULL, nlive < R);
+  const bool hd = col0 + 32 * R > L2;
   const float k = lp.k, gO = lp.xgo, gE = lp.xge, gX = fmaxf(gO, gE);
   const size_t Lm = (size_t)w.Lm;
-  const float* ein = (band > 0) ? a.edge + w.ed0 + (size_t)(band - 1) * w.edb : nullptr;
-  float* pout = (band > 0) ? a.bpush + w.bp0 + (size_t)band * w.bpb : nullptr;
+  const float* ein = (band > 0) ? LE::base(a.edge, w.ed0 + (size_t)(band - 1) * w.edb) : nullptr;
+  float* pout = (!SEG && band > 0) ? a.bpush + w.bp0 + (size_t)band * w.bpb : nullptr;
   const bool right_live = (col0 + 32 * R) < L2 && (band + 1) < w.nb;
   const float* pin = right_live ? a.bpush + w.bp0 + (size_t)(band + 1) * w.bpb : nullptr;
   const float* ck = a.ckpt + w.ck0 + (size_t)band * w.ckb;
-  const int nch = band_chunks(L1);
   const int KC = SPARSE ? a.ck_every : 1;   // checkpoint records every KC chunks
   const float* ckmax = ck + (size_t)((nch + KC - 1) / KC) * LREC;
 
@@ -714,22 +1253,26 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
   float* stg_ck = sm + C_STEPS * FW * 32;   // [CK4][lane][4]
   float4* s_eb = reinterpret_cast<float4*>(stg_ck + CKF * 32);   // [C] edge records
   float4* s_pb = s_eb + C_STEPS;                                 // [C] push records
+  Rows<R> rows;
+  rows.init(pr, jl, col0);
   float nsb[C_STEPS][R];   // the next chunk's score rows, requested a chunk ahead
+#pragma unroll
+  for (int u = 0; u < C_STEPS; ++u)
+#pragma unroll
+    for (int c = 0; c < R; ++c) nsb[u][c] = 0.f;
   int ckm;                 // the next chunk's largest normalised alpha frame
-  float ebr[NEF];          // lane u < C: left-band edge record of lane 0's row at recompute step u
+  float4 ebr;              // lane u < C: left-band edge record of lane 0's row at recompute step u
   float pbc[NPF], pbn[NPF];// lane u < C: right-band record lane 31 needs at backward step u
   auto load_ck = [&](int kc) {   // the record at or before chunk kc, and kc's alpha frame
-    const float* rec = ck + (size_t)(kc / KC) * LREC;
+    const float* rec = ck + (size_t)(SPARSE ? kc / KC : kc) * LREC;
 #pragma unroll
     for (int g = 0; g < LD::CK4; ++g) lcp16(stg_ck + g * 128 + lane * 4, rec + g * 128 + lane * 4, 16);
     lcp_commit();
     ckm = __float_as_int(ckmax[kc]);
   };
-  auto load_eb = [&](int kc) {
+  auto get_edge = [&](int kc) {
     const int i = kc * C_STEPS + lane + 1;
-    const bool ok = ein && lane < C_STEPS && i <= L1;
-#pragma unroll
-    for (int f = 0; f < NEF; ++f) ebr[f] = ok ? ein[f * Lm + (i - 1)] : 0.f;
+    return LE::get(ein, i, ein && lane < C_STEPS && i <= L1);
   };
   auto load_pb = [&](int kc, float (&dst)[NPF]) {
     const int i = kc * C_STEPS + C_STEPS - 1 - lane - 30;   // lane 31's row at backward step lane
@@ -738,418 +1281,519 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
     for (int f = 0; f < NPF; ++f) dst[f] = ok ? ld_poll(pin + f * (Lm + 1) + i) : 0.f;
   };
   auto load_sb = [&](int kc) {
+    const int i0 = kc * C_STEPS - lane + 1;
+    const float* src = rows.at(i0);
+    if (rows.vec && rows.inside(kc)) {
 #pragma unroll
-    for (int u = 0; u < C_STEPS; ++u) {
-      const int i = kc * C_STEPS + u - lane + 1;
-      load_row<R>(pr, i, jl, i >= 1 && i <= L1, nsb[u]);
+      for (int u = 0; u < C_STEPS; ++u) {
+        rows.template fetch<true>(src, nsb[u]);
+        src += rows.ld;
+      }
+    } else if (split_code<R>() && rows.inside(kc)) {
+#pragma unroll
+      for (int u = 0; u < C_STEPS; ++u) {
+        rows.template fetch<false>(src, nsb[u]);
+        src += rows.ld;
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < C_STEPS; ++u) {
+        rows.load(src, i0 + u, nsb[u]);
+        src += rows.ld;
+      }
     }
   };
-  load_ck(nch - 1);
-  load_eb(nch - 1);
-  load_sb(nch - 1);
-  load_pb(nch - 1, pbc);
+  load_ck(k_hi - 1);
+  ebr = get_edge(k_hi - 1);
+  load_sb(k_hi - 1);
+  load_pb(k_hi - 1, pbc);
 #pragma unroll
   for (int f = 0; f < NPF; ++f) pbn[f] = 0.f;
 
-  // ---- outside-recursion state: the row below (raw beta_I / beta in frame
-  // fb, t = E beta_M in frame nb), the right neighbour's held t and frame,
-  // and this lane's outputs of its latest row (for the left neighbour) ----
-  float bdn[R], tdn[R];
+  BState<R> bs;
+  if constexpr (SEG) bstate_load<R>(a.bck + ((w.slot0 + band) * a.nseg + seg) * BDims<R>::BREC, lane, bs);
+  else bstate_zero(bs);
+  BandSum gsum;
+  float cA = 0.f, cB = 0.f;   // the segment's plain sums
+  float2 cS = dup2(0.f);
+  auto flush = [&]() {        // at the end of a segment
+    float v0 = cA, v1 = cB, v2 = cS.x + cS.y;
 #pragma unroll
-  for (int c = 0; c < R; ++c) { bdn[c] = 0.f; tdn[c] = 0.f; }
-  int fb = 0, nb = 0;
-  float ht = 0.f;
-  int hn = 0;
-  float o_b = 0.f, o_t = 0.f;
-  int o_n = 0;
-  KSum gA, gB, gS;
+    for (int o = 16; o > 0; o >>= 1) {
+      v0 += __shfl_xor_sync(FULL, v0, o);
+      v1 += __shfl_xor_sync(FULL, v1, o);
+      v2 += __shfl_xor_sync(FULL, v2, o);
+    }
+    gsum.add(v0, v1, v2);
+    cA = 0.f; cB = 0.f; cS = dup2(0.f);
+  };
 
   // log2 of Z is at least zlog; a chunk is quiet (below) when every cell's
   // posterior and every flow out of it is below 2^-SWB_LQUIET
   const int zlog = ze + fexp(zm) - 1 - SWB_LQUIET;
-  for (int kc = nch - 1; kc >= 0; --kc) {
+#pragma unroll 1
+  for (int kc = k_hi - 1; kc >= k_lo; --kc) {
     const int t0 = kc * C_STEPS;
     lcp_wait_all();   // this chunk's staged checkpoint
     __syncwarp();
-    // ---- quiet chunk.  For a cell u of the chunk, alpha_u beta_u / Z sums,
-    // over the chunk cells x where u's continuations stay inside, terms
-    // alpha_x (1 + w beta_out) / Z (alpha_u W(u -> x) <= alpha_x: all weights
-    // are positive), where beta_out are the successors outside the chunk: the
-    // row below, the right neighbour's held t and, for lane 31, the right
-    // band's records.  With at most 2^9 cells, alpha_x <= 2^ckm and
-    // 1 + w beta_out <= 4 max(1, inflow), every posterior in the chunk and
-    // every flow across its top and left edges is below 2^-SWB_LQUIET when
-    // ckm + 11 + max(log2 inflow, 0) < log2 Z - SWB_LQUIET.  Such a chunk writes zero
-    // map rows and zero records to the left band, and passes zero beta up:
-    // the flows it drops are among those bounded.  The right band's records
-    // are resolved first, so the decision does not depend on timing. ----
-    {
-      {
-        bool miss = false;
+    if constexpr (!SEG) {   // the right band's records of this chunk
+      const bool miss = is_sentinel(pbc[0]) || is_sentinel(pbc[1]) || is_sentinel(pbc[2]);
+      if (__any_sync(FULL, miss) && miss) {
+        const int ir = kc * C_STEPS + C_STEPS - 1 - lane - 30;   // as in load_pb
+        FieldVec<NPF> x;
 #pragma unroll
-        for (int f = 0; f < NPF; ++f) miss |= is_sentinel(pbc[f]);
-        if (__any_sync(FULL, miss) && miss) {
-          const int ir = kc * C_STEPS + C_STEPS - 1 - lane - 30;   // as in load_pb
-          FieldVec<NPF> x;
+        for (int f = 0; f < NPF; ++f) x.v[f] = pbc[f];
+        x = poll_fields_v<NPF, 0>(x, pin + ir, Lm + 1, deadline, a.status, a.pair_done + w.p);
 #pragma unroll
-          for (int f = 0; f < NPF; ++f) x.v[f] = pbc[f];
-          x = poll_fields_v<NPF, 0>(x, pin + ir, Lm + 1, deadline, a.status, a.pair_done + w.p);
-#pragma unroll
-          for (int f = 0; f < NPF; ++f) pbc[f] = x.v[f];
-        }
+        for (int f = 0; f < NPF; ++f) pbc[f] = x.v[f];
       }
-      int inl = hn + fexp(ht);
-#pragma unroll
-      for (int c = 0; c < R; ++c) inl = max(inl, max(fb + fexp(bdn[c]), nb + fexp(tdn[c])));
-      if (lane < C_STEPS) {
-        const int pn = __float_as_int(pbc[2]);
-        inl = max(inl, pn + fexp(fmaxf(pbc[0], pbc[1])));
-      }
-      const bool ok = ckm + 11 + max(inl, 0) < zlog;
+      __syncwarp();
+    }
+    const bool quiet = lquiet<R>(bs, ckm, pbc, lane, zlog);
 #ifdef SWB_COUNT_QUIET   // measurement builds: quiet and computed chunks in header words 8, 9
-      {
-        const bool all_ok = __all_sync(FULL, ok);   // the vote runs on every lane
-        if (lane == 0) atomicAdd(a.counters + (all_ok ? 8 : 9), 1u);
-      }
+    if (lane == 0) atomicAdd(a.counters + (quiet ? 8 : 9), 1u);
 #endif
-      if (__all_sync(FULL, ok)) {
-        // zero map rows and left-band records for the rows of chunk kq
-        auto zero_chunk = [&](int kq) {
-          if constexpr (R % 4 == 0) zero_chunk_rows<R>(pr, kq, col0, lane);
+    if (quiet) {
+      auto zero_chunk = [&](int kq) {   // zero map rows and records
+        if constexpr (R % 4 == 0) zero_chunk_rows<R>(pr, kq, col0, lane);
+        else {
           for (int cu = 0; cu < C_STEPS; ++cu) {
             const int i = kq * C_STEPS + cu - lane + 1;
-            if (i >= 1 && i <= L1) {
-              if constexpr (R % 4 != 0) {
-                float z[R];
+            float z[R];
 #pragma unroll
-                for (int c = 0; c < R; ++c) z[c] = 0.f;
-                store_row<R>(pr, i, jl, z);
-              }
-              if (lane == 0 && pout) {
-                pout[0 * (Lm + 1) + i] = 0.f;
-                pout[1 * (Lm + 1) + i] = 0.f;
-                pout[2 * (Lm + 1) + i] = 0.f;
-              }
-            }
+            for (int c = 0; c < R; ++c) z[c] = 0.f;
+            if (i >= 1 && i <= L1) store_row<R>(pr, i, jl, z);
           }
-        };
-        zero_chunk(kc);
-        // the row above the chunk sees zero beta; lane 31 keeps the right
-        // band's t of its top chunk row as the held diagonal successor
-        float pt = __shfl_sync(FULL, pbc[1], C_STEPS - 1);
-        int pn = __shfl_sync(FULL, __float_as_int(pbc[2]), C_STEPS - 1);
-        // ---- quiet run.  After a quiet chunk only lane 31's held t and the
-        // right band's records enter the chunks above, so one round of loads
-        // decides the next 32 / C chunks: lane l takes chunk kn - l / C at
-        // backward step l % C (lane 31's row there), checking that record
-        // and the one of the row below (lane l - 1's; lane 0: the held t).
-        // A record not written yet ends the run; that chunk is then decided
-        // as above from the same values, so results do not depend on timing. ----
-        constexpr int RUN = 32 / C_STEPS;
-        int kn = kc - 1;
-        while (kn >= 0) {
-          const int j = lane / C_STEPS, u = lane - j * C_STEPS;
-          const int kq = kn - j;
-          float r0 = 0.f, r1 = 0.f;
-          int rn2 = 0, cm = -(1 << 30);
-          bool written = true;
-          if (kq >= 0) {
-            const int ir = kq * C_STEPS + C_STEPS - 1 - u - 30;
-            if (pin && ir >= 1 && ir <= L1) {
-              r0 = ld_poll(pin + 0 * (Lm + 1) + ir);
-              r1 = ld_poll(pin + 1 * (Lm + 1) + ir);
-              const float r2 = ld_poll(pin + 2 * (Lm + 1) + ir);
-              written = !is_sentinel(r0) && !is_sentinel(r1) && !is_sentinel(r2);
-              rn2 = __float_as_int(r2);
-            }
-            cm = __float_as_int(ckmax[kq]);
-          }
-          const int lg = written ? rn2 + fexp(fmaxf(r0, r1)) : 0;
-          const int lgu = __shfl_up_sync(FULL, lg, 1);
-          const bool wu = __shfl_up_sync(FULL, (int)written, 1) != 0;
-          const int lgb = lane == 0 ? pn + fexp(pt) : lgu;
-          const bool wb = lane == 0 || wu;
-          const bool q = kq >= 0 && written && wb && cm + 11 + max(max(lg, lgb), 0) < zlog;
-          const unsigned ball = __ballot_sync(FULL, q);
-          constexpr unsigned grp = (1u << C_STEPS) - 1u;
-          int n = 0;
-          while (n < RUN && kn - n >= 0 && ((ball >> (n * C_STEPS)) & grp) == grp) ++n;
-          for (int m = 0; m < n; ++m) zero_chunk(kn - m);
-          if (n > 0) {   // lane 31's held t: the record of its top row of the last zeroed chunk
-            const int src = (n - 1) * C_STEPS + C_STEPS - 1;
-            pt = __shfl_sync(FULL, r1, src);
-            pn = __shfl_sync(FULL, rn2, src);
-          }
-          kn -= n;
-          if (n < RUN) break;
         }
-#pragma unroll
-        for (int c = 0; c < R; ++c) { bdn[c] = 0.f; tdn[c] = 0.f; }
-        fb = 0; nb = 0;
-        o_b = 0.f; o_t = 0.f; o_n = 0;
-        ht = lane == 31 ? pt : 0.f;
-        hn = lane == 31 ? pn : 0;
-        if (kn >= 0) {   // inputs of the next chunk to run
-          load_ck(kn);
-          load_eb(kn);
-          load_sb(kn);
-          load_pb(kn, pbc);
+        zero_push(pout, Lm, L1, kq, lane);
+      };
+      zero_chunk(kc);
+      // the row above the chunk sees zero beta; lane 31 keeps the right
+      // band's t of its top chunk row as the held diagonal successor
+      float pt = __shfl_sync(FULL, pbc[1], C_STEPS - 1);
+      int pn = __shfl_sync(FULL, __float_as_int(pbc[2]), C_STEPS - 1);
+      int kn = kc - 1;
+      while (kn >= k_lo) {
+        float r1;
+        int rn;
+        const int n = lquiet_run(pin, Lm, L1, ckmax, kn, k_lo, lane, pt, pn, zlog, r1, rn);
+        for (int m = 0; m < n; ++m) zero_chunk(kn - m);
+        if (n > 0) {   // lane 31's held t: the record of its top row of the last zeroed chunk
+          pt = __shfl_sync(FULL, r1, n * C_STEPS - 1);
+          pn = __shfl_sync(FULL, rn, n * C_STEPS - 1);
         }
-        kc = kn + 1;   // the loop continues with chunk kn
-        continue;
+        kn -= n;
+        if (n < 32 / C_STEPS) break;
       }
+      if (!SEG && kc / kSeg != (kn + (kn < 0 ? -kSeg + 1 : 0)) / kSeg) flush();   // the run left the segment
+      bstate_zero(bs);
+      bs.ht = lane == 31 ? pt : 0.f;
+      bs.hn = lane == 31 ? pn : 0;
+      if (kn >= k_lo) {   // inputs of the next chunk to run
+        load_ck(kn);
+        ebr = get_edge(kn);
+        load_sb(kn);
+        load_pb(kn, pbc);
+      }
+      kc = kn + 1;   // the loop continues with chunk kn
+      continue;
     }
     // ---- restore the checkpoint and recompute the chunk ----
     LState<NS, R> st;
-    {
-      float ckr[CKF];
-      lck_load<NS, R>(stg_ck, lane, ckr);
-      lck_unpack<NS, R>(ckr, st, gO, gE, nlive, has_dead);
-    }
-    if (lane < C_STEPS) s_eb[lane] = make_float4(ebr[0], ebr[1], ebr[NEF > 2 ? 2 : 0], ebr[NEF > 3 ? 3 : 0]);
+    float2 d[H];
+#pragma unroll
+    for (int j = 0; j < H; ++j) d[j] = dup2(0.f);
+    lck_restore<NS, R, DM>(stg_ck, lane, st, gO, gE, nlive, hd, d);
+    if (lane < C_STEPS) s_eb[lane] = LE::open(ebr);
     __syncwarp();   // the staged checkpoint is read before the next chunk's copy is issued
-    if (SPARSE && kc % KC != 0) {
-      // sparse checkpoints: the restored state is that of chunk kc - kc % KC;
-      // run the forward over the chunks in between (the same steps as the
-      // forward kernel, so the state reached is bit for bit the same)
-      const int k0 = kc - kc % KC;
-      float ab[PF][R];
-#pragma unroll
-      for (int u = 0; u < PF; ++u) {
-        const int i = k0 * C_STEPS + u - lane + 1;
-        load_row<R>(pr, i, jl, i >= 1 && i <= L1, ab[u]);
-      }
-      for (int ka = k0; ka < kc; ++ka) {
-        float er[NEF];
-        {
-          const int ie = ka * C_STEPS + lane + 1;
-          const bool ok = ein && lane < C_STEPS && ie <= L1;
-#pragma unroll
-          for (int f = 0; f < NEF; ++f) er[f] = ok ? ein[f * Lm + (ie - 1)] : 0.f;
-        }
-#pragma unroll 1
-        for (int u0 = 0; u0 < C_STEPS; u0 += PF)
+    if constexpr (SPARSE) {
+      if (kc % KC != 0) {
+        // sparse checkpoints: the restored state is that of chunk kc - kc % KC;
+        // run the forward over the chunks in between (the same steps as the
+        // forward kernel, so the state reached is bit for bit the same)
+        const int k0 = kc - kc % KC;
+        float ab[PF][R];
+        int i = k0 * C_STEPS - lane + 1;
+        const float* src = rows.at(i);
 #pragma unroll
         for (int u = 0; u < PF; ++u) {
-          const int cu = u0 + u;
-          const int i = ka * C_STEPS + cu - lane + 1;
-          const bool act = (i >= 1) && (i <= L1);
-          float xl[NS];
 #pragma unroll
-          for (int q = 0; q < NS; ++q) xl[q] = __shfl_up_sync(FULL, st.vs[q], 1);
-          int xn = __shfl_up_sync(FULL, st.n, 1);
-          float ev[NEF];
+          for (int c = 0; c < R; ++c) ab[u][c] = 0.f;
+          rows.load(src, i + u, ab[u]);
+          src += rows.ld;
+        }
+#pragma unroll 1
+        for (int ka = k0; ka < kc; ++ka) {
+          float4 er = LE::open(get_edge(ka));
+#pragma unroll 1
+          for (int u0 = 0; u0 < C_STEPS; u0 += PF)
 #pragma unroll
-          for (int f = 0; f < NEF; ++f) ev[f] = __shfl_sync(FULL, er[f], cu);
-          if (lane == 0) {
-#pragma unroll
-            for (int q = 0; q < NS; ++q) xl[q] = act ? ev[q] : 0.f;
-            xn = act ? __float_as_int(ev[NS]) : 0;
+          for (int u = 0; u < PF; ++u) {
+            const int cu = u0 + u;
+            const bool act = (unsigned)(i - 1) < (unsigned)L1;
+            float xd = 0.f;
+            if constexpr (NS == 3) xd = __shfl_up_sync(FULL, st.od, 1);
+            float xc = __shfl_up_sync(FULL, st.oc, 1);
+            int xe = __shfl_up_sync(FULL, st.e, 1);
+            int xn = __shfl_up_sync(FULL, st.n, 1);
+            const float e0 = __shfl_sync(FULL, er.x, cu), e1 = __shfl_sync(FULL, er.y, cu);
+            const float e2 = __shfl_sync(FULL, er.z, cu), e3 = __shfl_sync(FULL, er.w, cu);
+            if (lane == 0) { xd = e0; xc = e1; xe = __float_as_int(e2); xn = __float_as_int(e3); }
+            float2 xs[H], E[H];
+            lemit<R, DM>(ab[u], k, nlive, hd, xs, E);
+            rows.load(src, i + PF, ab[u]);
+            src += rows.ld;
+            float rs;
+            if (act) lcells<NS, R, DM>(st, xd, xc, xe, xn, E, gO, gE, nlive, hd, d, rs);
+            ++i;
           }
-          float xs[R];
-          lscores<R>(ab[u], k, nlive, has_dead, xs);
-          {
-            const int ip = i + PF;
-            load_row<R>(pr, ip, jl, ip >= 1 && ip <= L1, ab[u]);
-          }
-          int et;
-          float em[R], rs;
-          lcells<NS, R>(st, xl, xn, xs, i >= 1, gO, gE, nlive, has_dead, et, em, rs);
         }
       }
     }
+    auto recompute = [&](auto inside_c) {
+      constexpr bool IN = decltype(inside_c)::value;
 #pragma unroll
     for (int cu = 0; cu < C_STEPS; ++cu) {
-      const int t = t0 + cu;
-      const int i = t - lane + 1;
-      const bool act = (i >= 1) && (i <= L1);
-      float xl[NS];
-#pragma unroll
-      for (int q = 0; q < NS; ++q) xl[q] = __shfl_up_sync(FULL, st.vs[q], 1);
+      const int i = t0 + cu - lane + 1;
+      const bool act = IN || (unsigned)(i - 1) < (unsigned)L1;
+      float xd = 0.f;
+      if constexpr (NS == 3) xd = __shfl_up_sync(FULL, st.od, 1);
+      float xc = __shfl_up_sync(FULL, st.oc, 1);
+      int xe = __shfl_up_sync(FULL, st.e, 1);
       int xn = __shfl_up_sync(FULL, st.n, 1);
       if (lane == 0) {
         const float4 e4 = s_eb[cu];
-        const float ev[4] = {e4.x, e4.y, e4.z, e4.w};
-#pragma unroll
-        for (int q = 0; q < NS; ++q) xl[q] = act ? ev[q] : 0.f;
-        xn = act ? __float_as_int(ev[NS]) : 0;
+        xd = e4.x; xc = e4.y; xe = __float_as_int(e4.z); xn = __float_as_int(e4.w);
       }
-      float xs[R];
-      lscores<R>(nsb[cu], k, nlive, has_dead, xs);
-      int et;
-      float em[R], rs;
-      lcells<NS, R>(st, xl, xn, xs, i >= 1, gO, gE, nlive, has_dead, et, em, rs);
+      float2 xs[H], E[H];
+      lemit<R, DM>(nsb[cu], k, nlive, hd, xs, E);
+      float rs;
+      if (act) lcells<NS, R, DM>(st, xd, xc, xe, xn, E, gO, gE, nlive, hd, d, rs);
       float* ent = sm + (size_t)cu * FW * 32;
-      if constexpr (R % 4 == 0) {
-        // field g's R columns as R / 4 float4 per lane: [g][quad][lane][4]
-        auto put = [&](int g, const float (&x)[R]) {
-#pragma unroll
-          for (int h = 0; h < R / 4; ++h)
-            reinterpret_cast<float4*>(ent + g * R * 32 + h * 128)[lane] =
-                make_float4(x[4 * h], x[4 * h + 1], x[4 * h + 2], x[4 * h + 3]);
-        };
-        put(0, st.v[0]);
-        if constexpr (NS == 3) {
-          put(1, st.v[1]);
-          put(2, st.v[2]);
+      // field g's R columns as pairs: [g][quad][lane][4] (2 columns: [g][lane][2])
+      auto put = [&](int g, const float2 (&x)[H]) {
+        if constexpr (R == 2) {
+          reinterpret_cast<float2*>(ent + g * 64)[lane] = x[0];
         } else {
-          put(1, em);
-        }
-        put(LD::NF - 1, xs);
-      } else {
 #pragma unroll
-        for (int c = 0; c < R; ++c) {
-          ent[(0 * R + c) * 32 + lane] = st.v[0][c];
-          if constexpr (NS == 3) {
-            ent[(1 * R + c) * 32 + lane] = st.v[1][c];
-            ent[(2 * R + c) * 32 + lane] = st.v[2][c];
-          } else {
-            ent[(1 * R + c) * 32 + lane] = em[c];
-          }
-          ent[((LD::NF - 1) * R + c) * 32 + lane] = xs[c];
+          for (int h = 0; h < H / 2; ++h)
+            reinterpret_cast<float4*>(ent + g * R * 32 + h * 128)[lane] =
+                make_float4(x[2 * h].x, x[2 * h].y, x[2 * h + 1].x, x[2 * h + 1].y);
         }
-      }
-      ent[LD::NF * R * 32 + lane] = __int_as_float(et);
-      ent[LD::NF * R * 32 + 32 + lane] = __int_as_float(st.n);
+      };
+      put(0, st.v[0]);
+      if constexpr (NS == 3) put(1, st.v[1]);
+      put(LD::NF - 2, d);
+      put(LD::NF - 1, xs);
+      ent[LD::NF * R * 32 + lane] = __int_as_float(st.e);
     }
-    if (kc > 0) {   // prefetch the next chunk's inputs while the outside recursion runs
+    };
+    const bool in = kc >= 32 / C_STEPS && (kc + 1) * C_STEPS <= L1;   // every lane on a row of the pair
+    if (split_code<R>() && in) recompute(std::true_type{});
+    else recompute(std::false_type{});
+    if (kc > k_lo) {   // prefetch the next chunk's inputs while the outside recursion runs
       load_ck(kc - 1);
-      load_eb(kc - 1);
+      ebr = get_edge(kc - 1);
       load_sb(kc - 1);
       load_pb(kc - 1, pbn);
     }
     if (lane < C_STEPS) s_pb[lane] = make_float4(pbc[0], pbc[1], pbc[2], 0.f);
     __syncwarp();
-    float cA = 0.f, cB = 0.f, cS = 0.f;   // this chunk's plain sums
+    int i = t0 + C_STEPS - lane;
+    float* mrow = pr.m + (long long)(i - 1) * pr.ld + jl;
     // ---- outside recursion over the chunk, last step first ----
 #pragma unroll 1
     for (int cu = 0; cu < C_STEPS; ++cu) {
-      const int ent_i = C_STEPS - 1 - cu;
-      const int t = t0 + ent_i;
-      const int i = t - lane + 1;
-      const bool act = (i >= 1) && (i <= L1);
-      const float* ent = sm + (size_t)ent_i * FW * 32;
+      const bool act = (unsigned)(i - 1) < (unsigned)L1;
+      const float* ent = sm + (size_t)(C_STEPS - 1 - cu) * FW * 32;
       // the right neighbour's latest row (row i): beta_D / beta of its column
       // 0, its t and frame; lane 31 takes the right band's record of row i
-      float rb = __shfl_down_sync(FULL, o_b, 1);
-      float rt = __shfl_down_sync(FULL, o_t, 1);
-      int rn = __shfl_down_sync(FULL, o_n, 1);
+      float rb = __shfl_down_sync(FULL, bs.ob, 1);
+      float rt = __shfl_down_sync(FULL, bs.t[0].x, 1);
+      int rn = __shfl_down_sync(FULL, bs.nb, 1);
       if (lane == 31) {   // resolved at the chunk's start (the quiet-chunk test polls them)
         const float4 p4 = s_pb[cu];
         rb = p4.x; rt = p4.y; rn = __float_as_int(p4.z);
       }
-      // frames: the row is computed in ft >= every input's normalised frame
-      const int ft = max(max(nb, rn), hn);
-      const float fBd = p2i(fb - ft), fTd = p2i(nb - ft), fR = p2i(rn - ft), fH = p2i(hn - ft);
-      const float st1 = p2i(-ft);
-      const int ea = __float_as_int(ent[LD::NF * R * 32 + lane]);
-      const int na = __float_as_int(ent[LD::NF * R * 32 + 32 + lane]);
-      const float as = p2i(ea - na);                       // raw alpha -> normalised
-      const float sc = p2any(na + ft - ze) * invZ; // real alpha * beta / Z factor
-      float fa[LD::NF][R];
-      if constexpr (R % 4 == 0) {
-#pragma unroll
-        for (int g = 0; g < LD::NF; ++g)
-#pragma unroll
-          for (int h = 0; h < R / 4; ++h) {
-            const float4 y = reinterpret_cast<const float4*>(ent + g * R * 32 + h * 128)[lane];
-            fa[g][4 * h] = y.x; fa[g][4 * h + 1] = y.y; fa[g][4 * h + 2] = y.z; fa[g][4 * h + 3] = y.w;
-          }
-      } else {
-#pragma unroll
-        for (int g = 0; g < LD::NF; ++g)
-#pragma unroll
-          for (int c = 0; c < R; ++c) fa[g][c] = ent[(g * R + c) * 32 + lane];
-      }
-      const float one = act ? st1 : 0.f;
-      // per-row factors folded out of the cells: the frame of the row below
-      // (fBd), alpha's normalisation (as) and the posterior scale (sc)
-      const float asc = as * sc, gEb = gE * fBd, gOb = gO * fBd;
-      float br = fR * rb;   // right successor's beta_D (beta)
-      float nbv[R], nmv[R], pm[R], mxv[R];
-      float so = 0.f, sxi = 0.f, sxd = 0.f, sp = 0.f;   // sums of raw alpha x beta
-#pragma unroll
-      for (int c = R - 1; c >= 0; --c) {
-        const float oc = c < nlive ? one : 0.f;
-        // plus the diagonal successor's t
-        const float base = c == R - 1 ? fmaf(fH, ht, oc) : fmaf(fTd, tdn[c + 1], oc);
-        const float sr = fmaf(fBd, bdn[c], br);   // beta_I (beta) below + beta_D right
-        if constexpr (NS == 3) {
-          const float vm = fmaf(gO, sr, base);
-          const float vi = fmaf(gEb, bdn[c], base);
-          const float vd = fmaf(gE, br, base);
-          const float P = fminf((fa[0][c] * asc) * vm, 1.f);   // a posterior: rounding may pass 1
-          pm[c] = P;
-          so = fmaf(fa[0][c], sr, so);
-          sxi = fmaf(fa[1][c], bdn[c], sxi);
-          sxd = fmaf(fa[2][c], br, sxd);
-          sp = fmaf(P, fa[3][c], sp);
-          nbv[c] = vi;
-          nmv[c] = vm;
-          mxv[c] = fmaf(gX, sr, base);   // >= vm, vi, vd
-          br = vd;
+      auto get = [&](int g, float2 (&x)[H]) {
+        if constexpr (R == 2) {
+          x[0] = reinterpret_cast<const float2*>(ent + g * 64)[lane];
         } else {
-          const float vb = fmaf(gO, br, fmaf(gOb, bdn[c], base));   // one fma on the column chain
-          const float P = fminf((fa[1][c] * asc) * vb, 1.f);
-          pm[c] = P;
-          so = fmaf(fa[0][c], sr, so);
-          sp = fmaf(P, fa[2][c], sp);
-          nbv[c] = vb;
-          nmv[c] = vb;
-          mxv[c] = vb;
-          br = vb;
+#pragma unroll
+          for (int h = 0; h < H / 2; ++h) {
+            const float4 y = reinterpret_cast<const float4*>(ent + g * R * 32 + h * 128)[lane];
+            x[2 * h] = make_float2(y.x, y.y);
+            x[2 * h + 1] = make_float2(y.z, y.w);
+          }
         }
+      };
+      const int ea = __float_as_int(ent[LD::NF * R * 32 + lane]);
+      float2 fm[H], fd[H], xs[H], E[H];
+      get(0, fm);
+      get(LD::NF - 2, fd);
+      get(LD::NF - 1, xs);
+#pragma unroll
+      for (int j = 0; j < H; ++j) E[j] = make_float2(ex2(xs[j].x), ex2(xs[j].y));
+      int ft;
+      float fB, vd0, mx;
+      float2 vm[H], vi[H], sr[H], br[H], P[H];
+      bcells<NS, R, DM>(bs, rb, rn, act, gO, gE, gX, nlive, hd, ft, fB, vm, vi, sr, br, vd0, mx);
+      // raw alpha (frame ea) times raw beta (frame ft), over Z
+      const float asc = p2any(ea + ft - ze) * invZ;
+      float2 so = dup2(0.f);
+#pragma unroll
+      for (int j = 0; j < H; ++j) {
+        const float2 p = mul2(mul2(NS == 3 ? fm[j] : fd[j], dup2(asc)), vm[j]);
+        P[j] = make_float2(fminf(p.x, 1.f), fminf(p.y, 1.f));   // a posterior: rounding may pass 1
+        so = fma2(fm[j], sr[j], so);
+        cS = fma2(P[j], xs[j], cS);
       }
-      // normalise: t = E beta_M in the row's normalised frame
-#pragma unroll
-      for (int h = 1; h < R; h *= 2)   // pairwise maximum: a short dependency chain
-#pragma unroll
-        for (int c = 0; c + h < R; c += 2 * h) mxv[c] = fmaxf(mxv[c], mxv[c + h]);
-      const int nn = max(ft + fexp(mxv[0]), 0);
-      const float bs = p2i(ft - nn);
-#pragma unroll
-      for (int c = 0; c < R; ++c) {
-        tdn[c] = (nmv[c] * bs) * ex2(fa[LD::NF - 1][c]);
-        bdn[c] = nbv[c];
-      }
-      fb = ft;
-      nb = nn;
-      o_b = br * bs;   // column 0's beta_D (beta), normalised
-      o_t = tdn[0];
-      o_n = nn;
-      ht = rt;
-      hn = rn;
+      cA = fmaf((so.x + so.y) * asc, gO, cA);
       if constexpr (NS == 3) {
-        cA = fmaf(so * asc, gO, cA);
-        cB = fmaf(fmaf(sxi, fBd, sxd) * asc, gE, cB);
-      } else {
-        cA = fmaf(so * asc, gO, cA);
+        float2 fi[H];
+        get(1, fi);
+        float2 sxi = dup2(0.f), sxd = dup2(0.f);
+#pragma unroll
+        for (int j = 0; j < H; ++j) {
+          sxi = fma2(fi[j], bs.b[j], sxi);
+          sxd = fma2(fd[j], br[j], sxd);
+        }
+        cB = fmaf(fmaf(sxi.x + sxi.y, fB, sxd.x + sxd.y) * asc, gE, cB);
       }
-      cS += sp;
+      bfinish<R>(bs, ft, mx, vm, vi, vd0, E, rt, rn);
       if (act) {
-        store_row<R>(pr, i, jl, pm);
+        store_pairs<R>(mrow, jl, pr, P);
         if (lane == 0 && pout) {
-          pout[0 * (Lm + 1) + i] = o_b;
-          pout[1 * (Lm + 1) + i] = o_t;
-          pout[2 * (Lm + 1) + i] = __int_as_float(o_n);
+          pout[0 * (Lm + 1) + i] = bs.ob;
+          pout[1 * (Lm + 1) + i] = bs.t[0].x;
+          pout[2 * (Lm + 1) + i] = __int_as_float(bs.nb);
         }
       }
+      --i;
+      mrow -= pr.ld;
     }
 #pragma unroll
     for (int f = 0; f < NPF; ++f) pbc[f] = pbn[f];
-    gA.add(cA);
-    gB.add(cB);
-    gS.add(cS);
+    if (!SEG && kc % kSeg == 0) flush();
     __syncwarp();
   }
-  float v0 = gA.s, v1 = gB.s, v2 = gS.s;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v0 += __shfl_xor_sync(FULL, v0, o);
-    v1 += __shfl_xor_sync(FULL, v1, o);
-    v2 += __shfl_xor_sync(FULL, v2, o);
+  if constexpr (SEG) {
+    flush();
+    lfinish_seg<NS>(a, w, lane, seg, Sh, Sl, gsum.a.s, gsum.b.s, gsum.m.s, pp);
+  } else {
+    finish_pair_p<NS>(a, w, lane, Sh, Sl, gsum.a.s, gsum.b.s, gsum.m.s, pp);
   }
-  finish_pair_p<NS>(a, w, lane, Sh, Sl, v0, v1, v2, pp);
+}
+
+// ---------------------------------------------------------------------------
+// the outside sweep and the segments
+// ---------------------------------------------------------------------------
+// In a batch too small to fill the GPU the adjoint's time is its longest
+// chain: per band, chunk after chunk, a restore, a recompute and an outside
+// pass.  There the outside recursion, which needs nothing of alpha but the
+// quiet-chunk test, runs as a sweep of its own (lbeta_kernel) that skips the
+// quiet chunks and keeps its state at the top of every kSeg-th chunk; then
+// every (band, segment) recomputes its chunks and writes its map rows
+// independently of the others (lseg_kernel).  The decisions, the states and
+// the sums are the adjoint's, so the results are its results bit for bit.
+
+template <int NS, int R, int DM>
+__device__ void lbeta_band(const Args& a, const LParams& lp, const Place& w, int lane, uint64_t deadline,
+                           float4* spush) {
+  using LD = LDims<NS, R>;
+  constexpr int H = R / 2, AH = fwd_ahead<R>(), SUB = AH / C_STEPS, NPF = 3;
+  const Pair& pr = w.pr;
+  const int L1 = pr.L1, L2 = pr.L2;
+  const int band = w.band;
+  const int col0 = band * 32 * R;
+  if (!(L1 > 0 && col0 < L2)) return;
+  int ze;
+  float zm;
+  lpair_z(a, w, lane, ze, zm);
+  const int zlog = ze + fexp(zm) - 1 - SWB_LQUIET;
+  const int jl = col0 + lane * R;
+  const int nlive = min(max(L2 - jl, 0), R);
+  const bool hd = col0 + 32 * R > L2;
+  const float k = lp.k, gO = lp.xgo, gE = lp.xge, gX = fmaxf(gO, gE);
+  const size_t Lm = (size_t)w.Lm;
+  float* pout = (band > 0) ? a.bpush + w.bp0 + (size_t)band * w.bpb : nullptr;
+  const bool right_live = (col0 + 32 * R) < L2 && (band + 1) < w.nb;
+  const float* pin = right_live ? a.bpush + w.bp0 + (size_t)(band + 1) * w.bpb : nullptr;
+  const int nch = band_chunks(L1), KC = a.ck_every;
+  const float* ckmax = a.ckpt + w.ck0 + (size_t)band * w.ckb + (size_t)((nch + KC - 1) / KC) * LD::LREC;
+  float* rec = a.bck + (w.slot0 + band) * (size_t)a.nseg * BDims<R>::BREC;
+
+  BState<R> bs;
+  bstate_zero(bs);
+  auto get_push = [&](int kc) {   // lane u < C: the right band's record lane 31 needs at backward step u
+    const int i = kc * C_STEPS + C_STEPS - 1 - lane - 30;
+    FieldVec<NPF> x;
+    const bool ok = pin && lane < C_STEPS && i >= 1 && i <= L1;
+#pragma unroll
+    for (int f = 0; f < NPF; ++f) x.v[f] = ld_poll_if(pin + f * (Lm + 1) + i, ok);
+    return x;
+  };
+  // the state at the top of a segment whose chunks above were quiet
+  auto store_zero = [&](int kq, float pt, int pn) {
+    BState<R> z;
+    bstate_zero(z);
+    z.ht = lane == 31 ? pt : 0.f;
+    z.hn = lane == 31 ? pn : 0;
+    bstate_store<R>(rec + (size_t)(kq / kSeg) * BDims<R>::BREC, lane, z);
+  };
+  Rows<R> rows;
+  rows.init(pr, jl, col0);
+  float sb[AH][R];
+#pragma unroll
+  for (int u = 0; u < AH; ++u)
+#pragma unroll
+    for (int c = 0; c < R; ++c) sb[u][c] = 0.f;
+  int kc = nch - 1;
+  FieldVec<NPF> ea, eb;
+  int ckm = 0, i = 0;
+  const float* src = rows.base;
+  // chunk kc's inputs, at the start and after a quiet run
+  auto prime = [&]() {
+    i = (kc + 1) * C_STEPS - lane;   // the lane's row at the next step
+    src = rows.at(i);
+    ea = get_push(kc);
+    eb = get_push(kc - 1);
+    ckm = __float_as_int(ckmax[kc]);
+#pragma unroll
+    for (int u = 0; u < AH; ++u) {
+      rows.load(src, i - u, sb[u]);
+      src -= rows.ld;
+    }
+  };
+  // one chunk; true after a quiet one (kc moved past the quiet run)
+  auto chunk = [&](auto sub_c) -> bool {
+    constexpr int S0 = decltype(sub_c)::value * C_STEPS;
+    const bool miss = is_sentinel(ea.v[0]) || is_sentinel(ea.v[1]) || is_sentinel(ea.v[2]);
+    if (__any_sync(FULL, miss)) {
+      if (miss)
+        ea = poll_fields_v<NPF, 0>(ea, pin + (kc * C_STEPS + C_STEPS - 1 - lane - 30), Lm + 1, deadline, a.status,
+                                   a.pair_done + w.p);
+      __syncwarp();
+    }
+    if (kc == nch - 1 || (kc + 1) % kSeg == 0) bstate_store<R>(rec + (size_t)(kc / kSeg) * BDims<R>::BREC, lane, bs);
+    if (lquiet<R>(bs, ckm, ea.v, lane, zlog)) {
+      zero_push(pout, Lm, L1, kc, lane);
+      float pt = __shfl_sync(FULL, ea.v[1], C_STEPS - 1);
+      int pn = __shfl_sync(FULL, __float_as_int(ea.v[2]), C_STEPS - 1);
+      int kn = kc - 1;
+      while (kn >= 0) {
+        float r1;
+        int rn;
+        const int n = lquiet_run(pin, Lm, L1, ckmax, kn, 0, lane, pt, pn, zlog, r1, rn);
+        for (int m = 0; m < n; ++m) {
+          if ((kn - m + 1) % kSeg == 0) store_zero(kn - m, pt, pn);
+          zero_push(pout, Lm, L1, kn - m, lane);
+          pt = __shfl_sync(FULL, r1, m * C_STEPS + C_STEPS - 1);
+          pn = __shfl_sync(FULL, rn, m * C_STEPS + C_STEPS - 1);
+        }
+        kn -= n;
+        if (n < 32 / C_STEPS) break;
+      }
+      bstate_zero(bs);
+      bs.ht = lane == 31 ? pt : 0.f;
+      bs.hn = lane == 31 ? pn : 0;
+      kc = kn;
+      return true;
+    }
+    if (lane < C_STEPS) spush[lane] = make_float4(ea.v[0], ea.v[1], ea.v[2], 0.f);
+    __syncwarp();
+    ea = eb;
+    eb = get_push(kc - 2);
+    if (kc > 0) ckm = __float_as_int(ckmax[kc - 1]);
+    auto steps = [&](auto inside_c, auto vec_c) {
+      constexpr bool IN = decltype(inside_c)::value, VEC = decltype(vec_c)::value;
+      constexpr int DD = IN ? DM : 1;
+#pragma unroll
+      for (int cu = 0; cu < C_STEPS; ++cu) {
+        const bool act = IN || (unsigned)(i - cu - 1) < (unsigned)L1;
+        const float4 p4 = spush[cu];
+        float rb = __shfl_down_sync(FULL, bs.ob, 1);
+        float rt = __shfl_down_sync(FULL, bs.t[0].x, 1);
+        int rn = __shfl_down_sync(FULL, bs.nb, 1);
+        rb = lane == 31 ? p4.x : rb;
+        rt = lane == 31 ? p4.y : rt;
+        rn = lane == 31 ? __float_as_int(p4.z) : rn;
+        float2 xs[H], E[H];
+        lemit<R, DD>(sb[S0 + cu], k, nlive, hd, xs, E);
+        if constexpr (IN) rows.template fetch<VEC>(src, sb[S0 + cu]);
+        else rows.load(src, i - cu - AH, sb[S0 + cu]);
+        src -= rows.ld;
+        int ft;
+        float fB, vd0, mx;
+        float2 vm[H], vi[H], sr[H], br[H];
+        bcells<NS, R, DD>(bs, rb, rn, act, gO, gE, gX, nlive, hd, ft, fB, vm, vi, sr, br, vd0, mx);
+        bfinish<R>(bs, ft, mx, vm, vi, vd0, E, rt, rn);
+        if (act && lane == 0 && pout) {
+          pout[0 * (Lm + 1) + i - cu] = bs.ob;
+          pout[1 * (Lm + 1) + i - cu] = bs.t[0].x;
+          pout[2 * (Lm + 1) + i - cu] = __int_as_float(bs.nb);
+        }
+      }
+    };
+    if (rows.inside(kc) && rows.inside(kc - SUB)) {
+      if (DM != 1 || rows.vec) steps(std::true_type{}, std::true_type{});
+      else if constexpr (DM == 1) steps(std::true_type{}, std::false_type{});
+    } else {
+      steps(std::false_type{}, std::false_type{});
+    }
+    i -= C_STEPS;
+    --kc;
+    __syncwarp();   // spush is free for the next chunk
+    return false;
+  };
+  bool jumped = true;
+#pragma unroll 1
+  while (kc >= 0) {
+    if (jumped) prime();
+    jumped = chunk(std::integral_constant<int, 0>{});
+    if constexpr (SUB > 1) {
+      if (!jumped && kc >= 0) jumped = chunk(std::integral_constant<int, 1 % SUB>{});
+    }
+  }
+}
+
+template <int NS, int R>
+__global__ void __launch_bounds__(128) lbeta_kernel(Args a) {
+  __shared__ float4 s_push[4][C_STEPS];
+  const int lane = threadIdx.x & 31;
+  const LParams lp = lparams<NS>(a);
+  const uint64_t deadline = gtimer() + a.spin_limit_ns;
+  const int ntasks = a.B * a.nb;
+  while (true) {
+    int task = 0;
+    if (lane == 0) task = (int)atomicAdd(a.counters + 1, 1u);
+    task = __shfl_sync(FULL, task, 0);
+    if (task >= ntasks) break;
+    const Place w = place_of<NS, R>(a, task, true);
+    if ((w.band + 1) * 32 * R > w.pr.L2 || !w.pr.vec)
+      lbeta_band<NS, R, 1>(a, lp, w, lane, deadline, s_push[threadIdx.x >> 5]);
+    else
+      lbeta_band<NS, R, 0>(a, lp, w, lane, deadline, s_push[threadIdx.x >> 5]);
+    __syncwarp();
+  }
+}
+
+// The segments of every band (a.nseg per band): one warp each.
+template <int NS, int R, bool SPARSE>
+__global__ void __launch_bounds__(32) lseg_kernel(Args a) {
+  extern __shared__ float smem[];
+  const int lane = threadIdx.x;
+  const LParams lp = lparams<NS>(a);
+  const int ntasks = a.B * a.nb * a.nseg;
+  for (int task = blockIdx.x; task < ntasks; task += gridDim.x) {
+    const int slot = task / a.nseg, seg = task - slot * a.nseg;
+    const Place w = place_of<NS, R>(a, slot, false);
+    if constexpr (!split_code<R>()) lbwd_band<NS, R, SPARSE, 2, true>(a, lp, w, lane, smem, 0, seg);
+    else if ((w.band + 1) * 32 * R > w.pr.L2) lbwd_band<NS, R, SPARSE, 1, true>(a, lp, w, lane, smem, 0, seg);
+    else lbwd_band<NS, R, SPARSE, 0, true>(a, lp, w, lane, smem, 0, seg);
+    lcp_wait_all();
+    __syncwarp();
+  }
 }
 
 // Before a separate adjoint launch on a workspace the forward filled: the
@@ -1177,7 +1821,10 @@ __global__ void __launch_bounds__(32 * WARPS) lbwd_kernel(Args a) {
     if (lane == 0) task = (int)atomicAdd(a.counters + 1, 1u);
     task = __shfl_sync(FULL, task, 0);
     if (task >= ntasks) break;
-    lbwd_band<NS, R, SPARSE>(a, lp, place_of<NS, R>(a, task, true), lane, sm, deadline);
+    const Place w = place_of<NS, R>(a, task, true);
+    if constexpr (!split_code<R>()) lbwd_band<NS, R, SPARSE, 2>(a, lp, w, lane, sm, deadline);
+    else if ((w.band + 1) * 32 * R > w.pr.L2) lbwd_band<NS, R, SPARSE, 1>(a, lp, w, lane, sm, deadline);
+    else lbwd_band<NS, R, SPARSE, 0>(a, lp, w, lane, sm, deadline);
   }
 }
 

