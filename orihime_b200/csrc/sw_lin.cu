@@ -234,22 +234,29 @@ constexpr int ZF_NONE = -(1 << 28);
 template <int GM> __host__ __device__ constexpr int zero_frame() { return GM == 1 ? ZF_NONE : 0; }
 template <int GM> __device__ __forceinline__ int floor_frame(int n) { return GM == 1 ? n : max(n, 0); }
 // Frames in cross-band records are biased so that no word is the sentinel.
-template <int GM> __host__ __device__ constexpr int frame_bias() { return GM == 1 ? (1 << 29) : 0; }
+template <int GM> __host__ __device__ constexpr int frame_bias() { return GM ? (1 << 29) : 0; }
 
 // ---- spread.  A lane keeps its columns of a row under one frame, so a value
-// more than 2^-126 below the row's largest loses bits or all of it.  The
+// far enough below the row's largest loses bits or all of it.  The
 // double-float log-domain kernels do not, so the models that they otherwise
-// serve (GM 1 and 2) watch the spread of each lane's row, and a pair in which
-// it may have mattered is run again in the log domain:
-// * the forward flags a pair when a value of some lane's row lies more than
-//   2^-SPREAD_A below the row's frame (Saigo-Vert: values below 2^-45 of the empty alignment do not
-//   count, as any continuation of theirs weighs less than a fresh start);
-//   A score beyond the clamp counts as spread too.
-// * the adjoint flags a pair when a value of beta lies more than 2^-SPREAD_B
-//   below its row's frame where it may count: where 2^-126 of that frame times
-//   the row's alpha is over 2^-45 of Z (with a bit of its own: bands of the
-//   pair that have not started must not stop, their neighbours wait for them).
-constexpr int SPREAD_A = 110, SPREAD_B = 100;
+// serve (GM 1 and 2) place their rows HEADROOM bits higher in fp32's range
+// (scores up to XHEAD fit on top of it), which leaves 2^-174 below a row's
+// inputs, and watch what is left; a pair in which it may have mattered is run
+// again in the log domain:
+// * the forward flags a pair when a raw value of some lane's row is below
+//   2^-SPREAD (Saigo-Vert: values below 2^-45 of the empty alignment do not
+//   count, as any continuation of theirs weighs less than a fresh start), or
+//   when a score passes XHEAD;
+// * the adjoint flags a pair when a raw value of beta is below 2^-SPREAD where
+//   it may count: where 2^-126 of the row's frame times the row's alpha is
+//   over 2^-45 of Z (with a bit of its own: bands of the pair that have not
+//   started must not stop, their neighbours wait for them).
+// Of 1024 pairs of 32 to 1024 rows and columns at T = 0.5, one or two come
+// within 2^-110 of a row's largest value, and each such pair run again costs a
+// whole chain of log-domain steps; hence the headroom.
+template <int GM> __host__ __device__ constexpr int headroom() { return GM ? 48 : 0; }
+template <int GM> __host__ __device__ constexpr float score_max() { return GM ? 70.f : XMAX; }
+constexpr int SPREAD = 124;
 __device__ __forceinline__ void flag_redo(const Args& a, int p, int lane, unsigned flag) {
   if (lane == 0) {
     atomicOr(a.pair_done + p, flag);
@@ -444,7 +451,8 @@ __device__ __forceinline__ void lcells(LState<NS, R>& s, float xd, float xc, int
   // the row's frame is at least every input's normalised frame, so that every
   // converted input is <= 1 (a raw value's frame exceeds its normalised frame
   // by at most 126)
-  const int et = max(max(s.n, xn), s.nd);
+  int et = max(max(s.n, xn), s.nd);
+  if constexpr (GM != 0) et = max(max(et - headroom<GM>(), s.e - 127), xe - 127);   // (conversions stay below 2^128)
   s.nd = xn;
   const int q = 127 - et;
   const float fU = p2b(s.e + q), fL = p2b(xe + q);
@@ -512,7 +520,7 @@ __device__ __forceinline__ void lblank(bool act, float2 (&xs)[R / 2], float2 (&E
 
 // Scaled scores and emissions of one step as pairs: clamped at XMAX, NEG
 // (E = 0) in columns past the pair.
-template <int R, int DM>
+template <int R, int DM, int GM>
 __device__ __forceinline__ void lemit(const float (&sb)[R], float k, int nlive, bool hd, float2 (&xs)[R / 2],
                                       float2 (&E)[R / 2]) {
   constexpr int H = R / 2;
@@ -520,8 +528,8 @@ __device__ __forceinline__ void lemit(const float (&sb)[R], float k, int nlive, 
 #pragma unroll
   for (int c = 0; c < R; c += 2) {
     const float2 t = mul2(make_float2(sb[c], sb[c + 1]), dup2(k));
-    x[c] = fminf(t.x, XMAX);
-    x[c + 1] = fminf(t.y, XMAX);
+    x[c] = fminf(t.x, score_max<GM>());
+    x[c + 1] = fminf(t.y, score_max<GM>());
   }
   if (masks<DM>(hd)) {
 #pragma unroll
@@ -645,7 +653,7 @@ __device__ __forceinline__ float ld_poll_if(const float* p, bool ok) {
 // 16-byte boundary of its edge slice (2 NS floats per row hold them with the
 // padding; slices start at even offsets).
 template <int NS, int GM = 0> struct LEdge {
-  static constexpr int BIAS = frame_bias<GM>(), B16 = GM == 1 ? (1 << 23) : 0;   // affine; linear
+  static constexpr int BIAS = frame_bias<GM>(), B16 = GM ? (1 << 23) : 0;   // affine; linear
   __device__ static __forceinline__ float* base(float* edge, size_t off) {
     return edge + (NS == 3 ? (off + 3) / 4 * 4 : off);
   }
@@ -841,7 +849,7 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
     if (ready && lane < WB)
       sedge[((bl + 1) & 1) * WB + lane] = ein || GM != 1 ? LE::open(eb) : LE::column0(lp, (bl + 1) * WB + lane + 1);
     if constexpr (GM != 0) {   // the pair is to be run again in the log domain: leave it
-      if (__any_sync(FULL, spread > SPREAD_A)) flag_redo(a, w.p, lane, PAIR_REDO);
+      if (__any_sync(FULL, spread > SPREAD)) flag_redo(a, w.p, lane, PAIR_REDO);
       if (stop) return;
       stop = __any_sync(FULL, lane == 0 && redo_set(a, w.p));
     }
@@ -881,7 +889,7 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
         xe = lane == 0 ? __float_as_int(e4.z) : xe;
         xn = lane == 0 ? __float_as_int(e4.w) : xn;
         float2 xs[H], E[H];
-        lemit<R, DD>(sb[(h * C_STEPS + cu) % AH], k, nlive, hd, xs, E);
+        lemit<R, DD, GM>(sb[(h * C_STEPS + cu) % AH], k, nlive, hd, xs, E);
         if constexpr (IN) rows.template fetch<VEC>(src, sb[(h * C_STEPS + cu) % AH]);
         else rows.load(src, i + cu + AH, sb[(h * C_STEPS + cu) % AH]);
         src += rows.ld;
@@ -897,7 +905,7 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
             float top = xs[0].x;   // a clamped score (the log domain takes any)
 #pragma unroll
             for (int j = 0; j < H; ++j) top = fmaxf(top, fmaxf(xs[j].x, xs[j].y));
-            if (top >= XMAX) spread = 127;
+            if (top >= score_max<GM>()) spread = 127;
             if (DD == 0 || nlive > 0) spread = max(spread, 127 - x);   // 1 in the row's frame against its least value
           }
           const int rx = sexp(rsv[cu]);
@@ -940,7 +948,7 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
     }
   }
   if constexpr (GM != 0) {
-    if (__any_sync(FULL, spread > SPREAD_A)) flag_redo(a, w.p, lane, PAIR_REDO);
+    if (__any_sync(FULL, spread > SPREAD)) flag_redo(a, w.p, lane, PAIR_REDO);
   }
   if constexpr (GM == 1) {   // the terminal cell (L1, L2): Z of the pair, in its band's partial
     const int q = L2 - 1 - jl;
@@ -1282,6 +1290,7 @@ __device__ __forceinline__ void bcells(const BState<R>& s, float rb, int rn, boo
   constexpr int H = R / 2;
   // frames: the row is computed in ft >= every input's normalised frame
   ft = max(max(s.nb, rn), s.hn);
+  if constexpr (GM != 0) ft = max(ft - headroom<GM>(), s.fb - 127);
   if (GM == 1 && live && term >= 0) ft = max(ft, 0);
   const int q = 127 - ft;
   fB = p2b(s.fb + q);
@@ -1698,7 +1707,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
             const float e2 = __shfl_sync(FULL, er.z, cu), e3 = __shfl_sync(FULL, er.w, cu);
             if (lane == 0) { xd = e0; xc = e1; xe = __float_as_int(e2); xn = __float_as_int(e3); }
             float2 xs[H], E[H];
-            lemit<R, DM>(ab[u], k, nlive, hd, xs, E);
+            lemit<R, DM, GM>(ab[u], k, nlive, hd, xs, E);
             rows.load(src, i + PF, ab[u]);
             src += rows.ld;
             float rs;
@@ -1722,7 +1731,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
         xd = e4.x; xc = e4.y; xe = __float_as_int(e4.z); xn = __float_as_int(e4.w);
       }
       float2 xs[H], E[H];
-      lemit<R, DM>(nsb[cu], k, nlive, hd, xs, E);
+      lemit<R, DM, GM>(nsb[cu], k, nlive, hd, xs, E);
       lblank<R>(act, xs, E);
       float rs;
       if (act) lcells<NS, R, DM, GM>(st, xd, xc, xe, xn, E, gO, gE, nlive, hd, d, rs);
@@ -1800,17 +1809,22 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
       float2 vm[H], vi[H], sr[H], br[H], P[H];
       bcells<NS, R, DM, GM>(bs, rb, rn, GM == 1 ? i == L1 : act, term, gO, gE, gX, nlive, hd, ft, fB, vm, vi, sr, br, vd0, mx);
       // raw alpha (frame ea) times raw beta (frame ft), over Z
-      const float asc = p2any(ea + ft - ze) * invZ;
+      // (with headroom the product's exponent may leave the range of one
+      // factor: half goes to each side)
+      const int ax = ea + ft - ze;
+      const float asc = p2any(GM ? ax >> 1 : ax) * invZ, bsc = GM ? p2any(ax - (ax >> 1)) : 1.f;
       if constexpr (GM != 0) {   // a beta near the end of the range where alpha makes it count
         const int bx = 127 - sexp(min2<DM>(vm, nlive, hd));
-        lost = lost || (act && (DM == 0 || nlive > 0) && bx > SPREAD_B && ea - 126 + (ew & 255) + ft - 81 > zlog + SWB_LQUIET);
+        lost = lost || (act && (DM == 0 || nlive > 0) && bx > SPREAD && ea - 126 + (ew & 255) + ft - 81 > zlog + SWB_LQUIET);
       }
       float2 so = dup2(0.f);
 #pragma unroll
       for (int j = 0; j < H; ++j) {
-        const float2 p = mul2(mul2(NS == 3 ? fm[j] : fd[j], dup2(asc)), vm[j]);
+        const float2 q = mul2(NS == 3 ? fm[j] : fd[j], dup2(asc));
+        const float2 p = mul2(q, GM ? mul2(vm[j], dup2(bsc)) : vm[j]);
         P[j] = make_float2(fminf(p.x, 1.f), fminf(p.y, 1.f));   // a posterior: rounding may pass 1
-        if (GM != 1 || NS == 3) so = fma2(fm[j], sr[j], so);
+        if constexpr (GM == 0) so = fma2(fm[j], sr[j], so);
+        else if constexpr (NS == 3) so = fma2(q, sr[j], so);   // scaled first: raw values fill the range here
         // (an excluded cell, score -inf, has posterior 0)
         cS = fma2(P[j], GM == 0 ? xs[j] : make_float2(fmaxf(xs[j].x, NEG), fmaxf(xs[j].y, NEG)), cS);
         if constexpr (GM == 1) cP = add2(cP, P[j]);
@@ -1823,14 +1837,15 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
         float2 sdi = dup2(0.f);
 #pragma unroll
         for (int j = 0; j < H; ++j) {
-          so = fma2(fi[j], br[j], so);
-          if constexpr (GM == 1) sdi = fma2(fd[j], bs.b[j], sdi);
+          so = fma2(mul2(fi[j], dup2(asc)), br[j], so);
+          if constexpr (GM == 1) sdi = fma2(mul2(fd[j], dup2(asc)), bs.b[j], sdi);
         }
-        float o = fmaf(sdi.x + sdi.y, fB, so.x + so.y) * asc * gO;
+        float o = fmaf(sdi.x + sdi.y, fB, so.x + so.y) * bsc * gO;
         if constexpr (GM == 1) {
           if (band == 0 && lane == 0 && act) {
             const float4 e4 = s_eb[C_STEPS - 1 - cu];
-            o = fmaf(e4.x * vd0, p2any(__float_as_int(e4.z) + ft - ze) * invZ, o);
+            const int x = __float_as_int(e4.z) + ft - ze;
+            o = fmaf(e4.x * (p2any(x >> 1) * invZ), vd0 * p2any(x - (x >> 1)), o);
           }
         }
         if (GM == 2 || act) cA += o;
@@ -1843,10 +1858,11 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
         float2 sxi = dup2(0.f), sxd = dup2(0.f);
 #pragma unroll
         for (int j = 0; j < H; ++j) {
-          sxi = fma2(fi[j], bs.b[j], sxi);
-          sxd = fma2(fd[j], br[j], sxd);
+          sxi = fma2(GM ? mul2(fi[j], dup2(asc)) : fi[j], bs.b[j], sxi);
+          sxd = fma2(GM ? mul2(fd[j], dup2(asc)) : fd[j], br[j], sxd);
         }
-        cB = fmaf(fmaf(sxi.x + sxi.y, fB, sxd.x + sxd.y) * asc, gE, cB);
+        const float x = fmaf(sxi.x + sxi.y, fB, sxd.x + sxd.y);
+        cB = fmaf(x * (GM ? bsc : asc), gE, cB);
       }
       bfinish<R, GM>(bs, ft, mx, vm, vi, vd0, E, rt, rn);
       if constexpr (GM == 1 && NS == 3) {
@@ -1856,9 +1872,10 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
 #pragma unroll
           for (int j = 0; j < H; ++j) d0[j] = dup2(0.f);
           lstate_row0<NS, R, DM>(z, d0, lp, jl, nlive, hd);
+          const int x = z.e + bs.fb - ze;
 #pragma unroll
-          for (int j = 0; j < H; ++j) o = fma2(d0[j], bs.b[j], o);
-          cA = fmaf((o.x + o.y) * gO, p2any(z.e + bs.fb - ze) * invZ, cA);
+          for (int j = 0; j < H; ++j) o = fma2(mul2(d0[j], dup2(p2any(x >> 1) * invZ)), mul2(bs.b[j], dup2(p2any(x - (x >> 1)))), o);
+          cA = fmaf(o.x + o.y, gO, cA);
         }
       }
       if (act) {
@@ -2028,7 +2045,7 @@ __device__ void lbeta_band(const Args& a, const LParams& lp, const Place& w, int
         rt = lane == 31 ? p4.y : rt;
         rn = lane == 31 ? __float_as_int(p4.z) : rn;
         float2 xs[H], E[H];
-        lemit<R, DD>(sb[S0 + cu], k, nlive, hd, xs, E);
+        lemit<R, DD, GM>(sb[S0 + cu], k, nlive, hd, xs, E);
         if constexpr (!IN) lblank<R>(act, xs, E);
         if constexpr (IN) rows.template fetch<VEC>(src, sb[S0 + cu]);
         else rows.load(src, i - cu - AH, sb[S0 + cu]);
