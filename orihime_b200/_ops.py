@@ -557,8 +557,9 @@ def _aux_plan(fam, B, L1, L2, dev, params):
     else:
         fn = getattr(_LIB, _AUX[fam][0])
     nbytes = int(fn(B, L1, L2))
-    # the free-memory query is a host call; under stream capture use the floor
-    free = 0 if _capturing() else torch.cuda.mem_get_info(dev)[0]
+    # the free-memory query (a driver call that can take milliseconds) matters
+    # only above the budget's floor; under stream capture use the floor
+    free = 0 if nbytes <= 2 << 30 or _capturing() else torch.cuda.mem_get_info(dev)[0]
     budget = min(AUX_BUDGET_MAX, max(2 << 30, free // 2))
     g = B
     if nbytes > budget:

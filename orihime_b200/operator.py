@@ -65,6 +65,16 @@ def _as_float(value: Param) -> float:
     return float(value.detach().reshape(()).item()) if isinstance(value, Tensor) else float(value)
 
 
+def _as_floats(params: Sequence[Param]) -> list[float]:
+    """The parameters as floats.  Several scalar tensors on one device are read
+    together: one device-to-host copy (and wait) instead of one each."""
+    ts = [p for p in params if isinstance(p, Tensor)]
+    if len(ts) > 1 and not _interpreters() and all(t.is_cuda and t.dtype == ts[0].dtype and t.device == ts[0].device for t in ts):
+        got = iter(torch.stack([t.detach().reshape(()) for t in ts]).tolist())
+        return [float(next(got)) if isinstance(p, Tensor) else float(p) for p in params]
+    return [_as_float(p) for p in params]
+
+
 def _validate_domain(name: str, x: Tensor, params: Sequence[Param], param_names: Sequence[str]) -> None:
     limit = MAX_ABS_SCORE_TEMPERATURE_RATIO
     T = params[param_names.index("temp")]
@@ -95,11 +105,12 @@ def _validate_domain(name: str, x: Tensor, params: Sequence[Param], param_names:
 
 
 def _validate_and_normalize(name: str, x: Tensor, params: Sequence[Param],
-                            param_names: Sequence[str]) -> Tensor:
+                            param_names: Sequence[str], vals: Optional[Sequence[float]] = None) -> Tensor:
     """_validate_domain then normalize_mask, with the full-tensor questions of
     both answered by one fused device pass (swb_scan_scores) for fp32 CUDA
     inputs: the same checks in the same order with the same messages, the
-    same sentinel values, one host synchronisation instead of three or four."""
+    same sentinel values, one host synchronisation instead of three or four.
+    vals: the parameters as floats, when the caller has read them."""
     if not (x.is_cuda and x.dtype == torch.float32 and x.numel() > 0):
         _validate_domain(name, x, params, param_names)
         return normalize_mask(x, _as_float(params[param_names.index("temp")]))
@@ -107,8 +118,13 @@ def _validate_and_normalize(name: str, x: Tensor, params: Sequence[Param],
 
     limit = MAX_ABS_SCORE_TEMPERATURE_RATIO
     T = params[param_names.index("temp")]
-    _validate_temperature(T)
-    Tf = _as_float(T)
+    if vals is None or not isinstance(T, Tensor):
+        _validate_temperature(T)
+    if vals is None:
+        vals = _as_floats(params)
+    Tf = vals[param_names.index("temp")]
+    if not (math.isfinite(Tf) and Tf > 0):
+        raise RuntimeError("temperature must be finite and strictly positive")
     message = ("orihime's supported FP32 numerical domain requires every finite "
                f"|score or cost| / temperature to be <= {limit:g}")
     flags, amax = ops_mod.scan_scores(x.detach().contiguous(), limit * Tf, MASK_SENTINEL_MAGNITUDE)
@@ -116,11 +132,10 @@ def _validate_and_normalize(name: str, x: Tensor, params: Sequence[Param],
         raise RuntimeError(f"{name} contains an unsupported infinity; use -inf score masks")
     if flags & ops_mod.SCAN_DOMAIN:
         raise RuntimeError(f"{message}; {name} is out of domain")
-    for pname, value in zip(param_names, params):
+    for pname, value, v in zip(param_names, params, vals):
         if pname == "temp":
             continue
         _validate_scalar_parameter_shape(value, pname)
-        v = _as_float(value)
         if isinstance(value, Tensor):
             if not value.is_floating_point():
                 raise TypeError(f"{pname} tensor must have a floating-point dtype")
@@ -332,18 +347,27 @@ def _entropy_direction_error(op, pname: str) -> NotImplementedError:
         "DERIVATIVE_COVERAGE.md. Detach the parameter or use finite differences.")
 
 
-def _checked(op, x: Tensor, params, lengths):
+def _checked_values(op, x: Tensor, params, lengths):
     """The value-dependent part of the input contract on plain tensors:
     lengths within the padded shape, the temperature, the FP32 numerical
     domain and -inf masks.  Returns (normalised scores, the -inf cells or
-    None)."""
+    None, the parameters as floats)."""
     if lengths is not None:
         lim = torch.tensor(x.shape[1:], device=lengths.device, dtype=torch.int32)
         if not bool(((lengths >= 0) & (lengths <= lim)).all()):
             raise RuntimeError("lengths entries must lie within the padded input shape")
-    xn = _validate_and_normalize(op.primary_name, x, params, op.params)
+    T = params[op.params.index("temp")]
+    if not isinstance(T, Tensor):
+        _validate_temperature(T)
+    vals = tuple(_as_floats(params))
+    xn = _validate_and_normalize(op.primary_name, x, params, op.params, vals)
     neg = torch.isneginf(x) if xn is not x else None
-    return (xn if xn.is_contiguous() else xn.contiguous()), neg
+    return (xn if xn.is_contiguous() else xn.contiguous()), neg, vals
+
+
+def _checked(op, x: Tensor, params, lengths):
+    """_checked_values without the values."""
+    return _checked_values(op, x, params, lengths)[:2]
 
 
 def _fold_vmap(fn, info, in_dims, op, validate, lengths, scores, params):
@@ -366,6 +390,13 @@ def _fold_vmap(fn, info, in_dims, op, validate, lengths, scores, params):
     return out, tuple(0 for _ in out)
 
 
+# The `validate` argument of the Functions: True where forward runs the input
+# contract itself (under a torch.func transform), else the parameters' values,
+# which the eager caller has read and checked.
+def _values(validate, params) -> list[float]:
+    return list(validate) if isinstance(validate, tuple) else _as_floats(params)
+
+
 def _saved(ctx):
     """(scores, lengths, -inf mask or None) saved by setup_context."""
     saved = ctx.saved_tensors
@@ -380,12 +411,14 @@ def _save_inputs(ctx, inputs, output, nlead: int):
     copy forward returned), the lengths and the -inf mask, for backward and
     for jvp; output[:nlead] are the observable's own outputs."""
     op, validate, lengths, scores, *params = inputs
+    vals = _values(validate, params)
+    validate = validate is True
     extra = output[nlead:]
     if validate:
         scores = extra[0]
     neg = extra[1] if validate and len(extra) > 1 else None
     ctx.op, ctx.validate = op, validate
-    ctx.vals = [_as_float(p) for p in params]
+    ctx.vals = vals
     ctx.pmeta = _param_meta(params)
     ctx.has_lengths, ctx.has_neg = lengths is not None, neg is not None
     tensors = (scores,) + ((lengths,) if lengths is not None else ()) + ((neg,) if neg is not None else ())
@@ -398,9 +431,10 @@ class _ValueFn(torch.autograd.Function):
     @staticmethod
     def forward(op, validate, lengths, scores, *params):
         neg = None
-        if validate:
-            scores, neg = _checked(op, scores, params, lengths)
-        vals = [_as_float(p) for p in params]
+        if validate is True:
+            scores, neg, vals = _checked_values(op, scores, params, lengths)
+        else:
+            vals = _values(validate, params)
         value, smap, *grads = op.fam.full(scores, *vals, lengths)
         if neg is not None:
             smap = smap.masked_fill(neg, 0.0)
@@ -468,10 +502,10 @@ class _CheckpointedValueFn(torch.autograd.Function):
     [B, L1, L2] is kept between the two."""
 
     @staticmethod
-    def forward(ctx, fam, lengths, ws_value, scores, *params):
+    def forward(ctx, fam, lengths, vals, ws_value, scores, *params):
         value, ws = ws_value
         ctx.fam, ctx.lengths, ctx.ws = fam, lengths, ws
-        ctx.vals = [_as_float(p) for p in params]
+        ctx.vals = vals
         ctx.pmeta = _param_meta(params)
         ctx.save_for_backward(scores)
         return value
@@ -484,14 +518,14 @@ class _CheckpointedValueFn(torch.autograd.Function):
         (scores,) = ctx.saved_tensors
         _, smap, *grads = ops_mod.run_adjoint(ctx.fam.name, scores, ctx.lengths, ctx.vals,
                                               _checkpoint_every(scores), ctx.ws)
-        gs = gv.view(-1, 1, 1) * smap if ctx.needs_input_grad[3] else None
-        out = [None, None, None, gs]
+        gs = gv.view(-1, 1, 1) * smap if ctx.needs_input_grad[4] else None
+        out = [None, None, None, None, gs]
         for k, meta in enumerate(ctx.pmeta):
-            out.append(_param_grad((gv * grads[k]).sum(), meta, ctx.needs_input_grad[4 + k]))
+            out.append(_param_grad((gv * grads[k]).sum(), meta, ctx.needs_input_grad[5 + k]))
         return tuple(out)
 
 
-def _checkpointed_value(fam, lengths, scores, params):
+def _checkpointed_value(fam, lengths, scores, params, vals):
     """The checkpointed value op, or None where it does not apply (another
     family, a positive gap, a tensor off CUDA, under stream capture)."""
     if (fam.name not in ("sw", "sw_affine") or not scores.is_cuda
@@ -499,11 +533,10 @@ def _checkpointed_value(fam, lengths, scores, params):
         return None
     from . import _ops as ops_mod
 
-    vals = [_as_float(p) for p in params]
     got = ops_mod.run_checkpoint(fam.name, scores.detach(), lengths, vals, _checkpoint_every(scores))
     if got is None:
         return None
-    return _CheckpointedValueFn.apply(fam, lengths, got, scores, *params)
+    return _CheckpointedValueFn.apply(fam, lengths, vals, got, scores, *params)
 
 
 class _MapFn(torch.autograd.Function):
@@ -512,14 +545,15 @@ class _MapFn(torch.autograd.Function):
     @staticmethod
     def forward(op, validate, lengths, scores, *params):
         neg = None
-        if validate:
-            scores, neg = _checked(op, scores, params, lengths)
-        vals = [_as_float(p) for p in params]
+        if validate is True:
+            scores, neg, vals = _checked_values(op, scores, params, lengths)
+        else:
+            vals = _values(validate, params)
         _, smap = op.fam.forward(scores, *vals, lengths)
         if neg is not None:
             smap = smap.masked_fill(neg, 0.0)
         # the normalised scores may be the input itself: return a view of it
-        extra = (scores.view_as(scores),) if validate else ()
+        extra = (scores.view_as(scores),) if validate is True else ()
         if neg is not None:
             extra += (neg,)
         return (smap, *extra)
@@ -588,11 +622,12 @@ class _EntropyFn(torch.autograd.Function):
     @staticmethod
     def forward(op, validate, lengths, scores, *params):
         neg = None
-        if validate:
-            scores, neg = _checked(op, scores, params, lengths)
-        vals = [_as_float(p) for p in params]
+        if validate is True:
+            scores, neg, vals = _checked_values(op, scores, params, lengths)
+        else:
+            vals = _values(validate, params)
         ent = op.fam.grads(scores, *vals, lengths)[-1]
-        extra = (scores.view_as(scores),) if validate else ()
+        extra = (scores.view_as(scores),) if validate is True else ()
         if neg is not None:
             extra += (neg,)
         return (ent, *extra)
@@ -720,11 +755,12 @@ class Operator:
         return primary, params, lengths
 
     def _prepare(self, primary, params, lengths, mask, dtype):
-        """The whole input contract.  lengths stays None when the caller gave
-        none: the ops take that as full lengths, with no host round trip."""
+        """The whole input contract, and the parameters as floats (read once per
+        call).  lengths stays None when the caller gave none: the ops take that
+        as full lengths, with no host round trip."""
         primary, params, lengths = self._prepare_shapes(primary, params, lengths, mask, dtype)
-        primary, _ = _checked(self, primary, params, lengths)
-        return primary, params, lengths
+        primary, _, vals = _checked_values(self, primary, params, lengths)
+        return primary, params, lengths, vals
 
     def _compiled(self, kind, primary, params, lengths, mask, dtype) -> Tensor:
         """While Dynamo traces: the observable as one opaque op (_pt2)."""
@@ -739,8 +775,8 @@ class Operator:
         if _transforms_active():
             x, params, lengths = self._prepare_shapes(primary, params, lengths, mask, dtype)
             return _MapFn.apply(self, True, lengths, x, *params)[0]
-        x, params, lengths = self._prepare(primary, params, lengths, mask, dtype)
-        return _MapFn.apply(self, False, lengths, x, *params)[0]
+        x, params, lengths, vals = self._prepare(primary, params, lengths, mask, dtype)
+        return _MapFn.apply(self, vals, lengths, x, *params)[0]
 
     def value(self, primary, *params, lengths=None, mask=None, dtype=None) -> Tensor:
         if torch.compiler.is_compiling():
@@ -748,17 +784,17 @@ class Operator:
         if _transforms_active():
             x, params, lengths = self._prepare_shapes(primary, params, lengths, mask, dtype)
             return _ValueFn.apply(self, True, lengths, x, *params)[0]
-        x, params, lengths = self._prepare(primary, params, lengths, mask, dtype)
+        x, params, lengths, vals = self._prepare(primary, params, lengths, mask, dtype)
         needs_grad = torch.is_grad_enabled() and (
             x.requires_grad or any(isinstance(p, Tensor) and p.requires_grad for p in params))
         if not needs_grad:
             # no gradient can flow: the forward wavefront alone (same values,
             # no marginal map, about half the work)
-            return self.fam.value(x, *[_as_float(p) for p in params], lengths)
-        v = _checkpointed_value(self.fam, lengths, x, params)
+            return self.fam.value(x, *vals, lengths)
+        v = _checkpointed_value(self.fam, lengths, x, params, vals)
         if v is not None:
             return v
-        return _ValueFn.apply(self, False, lengths, x, *params)[0]
+        return _ValueFn.apply(self, vals, lengths, x, *params)[0]
 
     def entropy(self, primary, *params, lengths=None, mask=None, dtype=None) -> Tensor:
         if torch.compiler.is_compiling():
@@ -766,19 +802,17 @@ class Operator:
         if _transforms_active():
             x, params, lengths = self._prepare_shapes(primary, params, lengths, mask, dtype)
             return _EntropyFn.apply(self, True, lengths, x, *params)[0]
-        x, params, lengths = self._prepare(primary, params, lengths, mask, dtype)
-        return _EntropyFn.apply(self, False, lengths, x, *params)[0]
+        x, params, lengths, vals = self._prepare(primary, params, lengths, mask, dtype)
+        return _EntropyFn.apply(self, vals, lengths, x, *params)[0]
 
     # -- named ops tier (orihime/operator.py:2312-2400) --
     def vjp(self, primary, *params, grad_map, wrt, lengths=None, mask=None, dtype=None) -> Tensor:
-        x, params, lengths = self._prepare(primary, params, lengths, mask, dtype)
-        vals = [_as_float(p) for p in params]
+        x, params, lengths, vals = self._prepare(primary, params, lengths, mask, dtype)
         if wrt == self.primary_name:
             return self.fam.hvp(x, grad_map.contiguous(), *vals, lengths)
         k = self.params.index(wrt)
         return (grad_map * self.fam.sens[k](x, *vals, lengths)).sum()
 
     def sensitivity(self, primary, *params, wrt, lengths=None, mask=None, dtype=None) -> Tensor:
-        x, params, lengths = self._prepare(primary, params, lengths, mask, dtype)
-        vals = [_as_float(p) for p in params]
+        x, params, lengths, vals = self._prepare(primary, params, lengths, mask, dtype)
         return self.fam.sens[self.params.index(wrt)](x, *vals, lengths)
