@@ -46,19 +46,15 @@ bool valid_r(int r) { return r == 2 || r == 4; }
 // 8 columns per lane: the linear-domain kernels of the local families only
 bool valid_r_local(int r) { return r == 2 || r == 4 || r == 8; }
 constexpr int ridx(int r) { return r == 2 ? 0 : (r == 4 ? 1 : 2); }
-// Global alignments run in the linear domain while a lane's columns of the
-// boundary rows stay well within fp32's range (gap factors of 2^-30 or more);
-// the other models for any gaps <= 0.
-template <int G> bool lin_gaps(double xo, double xe) { return G != 1 || (xo >= -30.0 && xe >= -30.0); }
 // Whether a launch with these parameters runs the linear-domain kernels
-// (gaps <= 0, not forced to the log domain).
+// (the local families, gaps <= 0, not forced to the log domain).
 template <int NS, int G>
 bool lin_eligible(float go, float ge, float T, const swb_options* opt) {
-  if (!(T > 0.f) || !(T < INFINITY)) return false;
+  if (G != 0 || !(T > 0.f) || !(T < INFINITY)) return false;
   if (opt && opt->domain == SWB_DOMAIN_LOG) return false;
   const float k = 1.4426950408889634f / T;
   const double xo = (double)go * (double)k, xe = NS == 3 ? (double)ge * (double)k : 0.0;
-  return xo <= 0.0 && xe <= 0.0 && lin_gaps<G>(xo, xe);
+  return xo <= 0.0 && xe <= 0.0;
 }
 // Default columns per lane of the padded entry points, for the linear-domain
 // kernels: 2 on batches at most 64 columns wide (one band with every lane
@@ -119,7 +115,7 @@ struct SegPlan {
 template <int R>
 SegPlan seg_plan(const Layout& l, long long slots) {
   SegPlan p;
-  if (R == 8 || slots > kSegSlots) return p;
+  if (!swb::split_code<R>() || slots > kSegSlots) return p;
   p.nseg = (l.nchunks + swb::kSeg - 1) / swb::kSeg;
   p.off_state = l.total;
   p.off_part = p.off_state + align_up(sizeof(float) * (size_t)slots * p.nseg * swb::BDims<R>::BREC);
@@ -161,11 +157,10 @@ size_t plan_bytes_for(long long B, long long ntasks) {
 struct DevInfo {
   int sms = 0;
   int occ[2][5][2] = {};   // [kernel fwd/bwd][model_index][R == 4?]
-  int locc[2][5][3] = {};  // linear-domain kernels: [fwd/bwd][model_index][R: 2, 4, 8]
+  int locc[2][2][3] = {};  // linear-domain kernels: [fwd/bwd][NS == 3?][R: 2, 4, 8]
   int locc_sparse[2][3] = {};  // linear-domain adjoint, sparse checkpoints: [NS == 3?][R: 2, 4, 8]
-  int lfwd_split[5][3] = {};   // forward of small batches: [model_index][R: 2, 4]
-  int sweep[5][3] = {};        // outside sweep: [model_index][R: 2, 4, 8]
-  int seg[2][5][3] = {};       // segments: [sparse?][model_index][R: 2, 4, 8]
+  int sweep[2][3] = {};        // outside sweep: [NS == 3?][R: 2, 4, 8]
+  int seg[2][2][3] = {};       // segments: [sparse?][NS == 3?][R: 2, 4, 8]
   bool ready = false;
 };
 DevInfo g_dev[64];
@@ -182,32 +177,38 @@ template <int NS, int G> constexpr int model_index() {
 template <int NS, int R>
 size_t lbwd_smem() { return (size_t)kWarpsBwd * swb::lbwd_smem_floats<NS, R>() * sizeof(float); }
 
-template <int NS, int R, int G = 0>
+template <int NS, int R>
 cudaError_t setup_lin(DevInfo& d) {
-  constexpr int m = model_index<NS, G>();
-  constexpr int smem = (int)(kWarpsBwd * swb::lbwd_smem_floats<NS, R>() * sizeof(float));
-  auto occ = [&](int* out, auto* kernel, int threads, int bytes) {
-    cudaError_t e = bytes ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : cudaSuccess;
-    if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, kernel, threads, bytes);
-  };
-  cudaError_t e = occ(&d.locc[0][m][ridx(R)], swb::lfwd_kernel<NS, R, G, false>, 32 * kWarpsFwd, 0);
+  cudaError_t e = cudaFuncSetAttribute(swb::lbwd_kernel<NS, R, kWarpsBwd>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)lbwd_smem<NS, R>());
   if (e != cudaSuccess) return e;
-  if constexpr (R != 8) {
-    if ((e = occ(&d.lfwd_split[m][ridx(R)], swb::lfwd_kernel<NS, R, G, true>, 32 * kWarpsFwd, 0)) != cudaSuccess) return e;
-  }
-  e = occ(&d.locc[1][m][ridx(R)], swb::lbwd_kernel<NS, R, kWarpsBwd, false, G>, 32 * kWarpsBwd, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.locc[0][NS == 3][ridx(R)],
+                                                    swb::lfwd_kernel<NS, R>, 32 * kWarpsFwd, 0);
   if (e != cudaSuccess) return e;
-  if constexpr (R != 8) {
-    if ((e = occ(&d.sweep[m][ridx(R)], swb::lbeta_kernel<NS, R, G>, 128, 0)) != cudaSuccess ||
-        (e = occ(&d.seg[0][m][ridx(R)], swb::lseg_kernel<NS, R, false, G>, 32, smem)) != cudaSuccess)
-      return e;
-    if constexpr (G == 0) {
-      if ((e = occ(&d.seg[1][m][ridx(R)], swb::lseg_kernel<NS, R, true, G>, 32, smem)) != cudaSuccess) return e;
-    }
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &d.locc[1][NS == 3][ridx(R)], swb::lbwd_kernel<NS, R, kWarpsBwd>, 32 * kWarpsBwd,
+      lbwd_smem<NS, R>());
+  if (e != cudaSuccess) return e;
+  if constexpr (swb::split_code<R>()) {
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.sweep[NS == 3][ridx(R)], swb::lbeta_kernel<NS, R>, 128,
+                                                         0)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(swb::lseg_kernel<NS, R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)lbwd_smem<NS, R>())) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(swb::lseg_kernel<NS, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)lbwd_smem<NS, R>())) != cudaSuccess ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.seg[0][NS == 3][ridx(R)], swb::lseg_kernel<NS, R, false>,
+                                                         32, lbwd_smem<NS, R>())) != cudaSuccess ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.seg[1][NS == 3][ridx(R)], swb::lseg_kernel<NS, R, true>,
+                                                         32, lbwd_smem<NS, R>())) != cudaSuccess)
+    return e;
   }
-  if constexpr (G == 0) return occ(&d.locc_sparse[NS == 3][ridx(R)], swb::lbwd_kernel<NS, R, kWarpsBwd, true, G>, 32 * kWarpsBwd, smem);
-  return e;
+  e = cudaFuncSetAttribute(swb::lbwd_kernel<NS, R, kWarpsBwd, true>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lbwd_smem<NS, R>());
+  if (e != cudaSuccess) return e;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &d.locc_sparse[NS == 3][ridx(R)], swb::lbwd_kernel<NS, R, kWarpsBwd, true>, 32 * kWarpsBwd,
+      lbwd_smem<NS, R>());
 }
 
 template <int NS, int R, int G = 0>
@@ -237,8 +238,7 @@ int dev_info(DevInfo** out) {
         setup_pair<1, 2, 1>(d) || setup_pair<1, 4, 1>(d) || setup_pair<3, 2, 1>(d) ||
         setup_pair<3, 4, 1>(d) || setup_pair<3, 2, 2>(d) || setup_pair<3, 4, 2>(d) ||
         setup_lin<1, 2>(d) || setup_lin<1, 4>(d) || setup_lin<3, 2>(d) || setup_lin<3, 4>(d) ||
-        setup_lin<1, 8>(d) || setup_lin<3, 8>(d) || setup_lin<1, 2, 1>(d) || setup_lin<1, 4, 1>(d) ||
-        setup_lin<3, 2, 1>(d) || setup_lin<3, 4, 1>(d) || setup_lin<3, 2, 2>(d) || setup_lin<3, 4, 2>(d))
+        setup_lin<1, 8>(d) || setup_lin<3, 8>(d))
       return SWB_ERR_CUDA;
     d.ready = true;
   }
@@ -287,49 +287,20 @@ int static_scratch(void** out) {
   return SWB_OK;
 }
 
-// The forward: the variant for small batches (a padded batch with at most two
-// warps per scheduler: branch-free steps, records passed 8 rows at a time), or
-// the compact one.  Affine, 4 columns per lane, forward, split / compact, us:
-// 4 x 1024^2 233 / 280; 512 x 512^2 (2048 bands) 263 / 240.
-constexpr long long kSplitTasks = 1184;
-template <int NS, int R, int G>
-void launch_forward(const Args& a, const DevInfo& d, long long ntasks, int max_ctas, cudaStream_t st) {
-  constexpr int m = model_index<NS, G>();
-  const bool split = R != 8 && a.layout == 0 && ntasks <= kSplitTasks;
-  const int occ = split ? d.lfwd_split[m][ridx(R)] : d.locc[0][m][ridx(R)];
-  long long grid = std::min<long long>((ntasks + kWarpsFwd - 1) / kWarpsFwd, (long long)d.sms * std::max(occ, 1));
-  if (max_ctas > 0) grid = std::min<long long>(grid, max_ctas);
-  const int g = (int)std::max(1LL, grid);
-  if constexpr (R != 8) {
-    if (split) {
-      swb::lfwd_kernel<NS, R, G, true><<<g, 32 * kWarpsFwd, 0, st>>>(a);
-      return;
-    }
-  }
-  swb::lfwd_kernel<NS, R, G, false><<<g, 32 * kWarpsFwd, 0, st>>>(a);
-}
-
 // The outside sweep and the segments of a padded batch.
-template <int NS, int R, int G = 0>
+template <int NS, int R>
 int launch_segments(Args a, const DevInfo& d, const SegPlan& p, char* w, bool sparse, int max_ctas, cudaStream_t st) {
   a.bck = reinterpret_cast<float*>(w + p.off_state);
   a.spart = reinterpret_cast<float*>(w + p.off_part);
   a.nseg = p.nseg;
   const long long slots = (long long)a.B * a.nb, n = slots * p.nseg;
-  constexpr int m = model_index<NS, G>();
-  const int os = d.sweep[m][ridx(R)], og = d.seg[sparse][m][ridx(R)];
+  const int os = d.sweep[NS == 3][ridx(R)], og = d.seg[sparse][NS == 3][ridx(R)];
   long long gs = std::min<long long>((slots + 3) / 4, (long long)d.sms * std::max(os, 1));
   long long gg = std::min<long long>(n, (long long)d.sms * std::max(og, 1));
   if (max_ctas > 0) { gs = std::min<long long>(gs, max_ctas); gg = std::min<long long>(gg, max_ctas); }
-  swb::lbeta_kernel<NS, R, G><<<(int)std::max(1LL, gs), 128, 0, st>>>(a);
-  const int grid = (int)std::max(1LL, gg);
-  if constexpr (G == 0) {
-    if (sparse) {
-      swb::lseg_kernel<NS, R, true, G><<<grid, 32, lbwd_smem<NS, R>(), st>>>(a);
-      return cudaPeekAtLastError() == cudaSuccess ? SWB_OK : SWB_ERR_CUDA;
-    }
-  }
-  swb::lseg_kernel<NS, R, false, G><<<grid, 32, lbwd_smem<NS, R>(), st>>>(a);
+  swb::lbeta_kernel<NS, R><<<(int)std::max(1LL, gs), 128, 0, st>>>(a);
+  if (sparse) swb::lseg_kernel<NS, R, true><<<(int)std::max(1LL, gg), 32, lbwd_smem<NS, R>(), st>>>(a);
+  else swb::lseg_kernel<NS, R, false><<<(int)std::max(1LL, gg), 32, lbwd_smem<NS, R>(), st>>>(a);
   return cudaPeekAtLastError() == cudaSuccess ? SWB_OK : SWB_ERR_CUDA;
 }
 
@@ -359,13 +330,13 @@ int launch(Args a, const Layout& l, long long ntasks, size_t map_elems, bool cle
   // transition factor 2^(gap k) is at most 1, else in the log domain
   const double xo = (double)a.go * (double)a.k, xe = NS == 3 ? (double)a.ge * (double)a.k : 0.0;
   const int domain = opt ? opt->domain : SWB_DOMAIN_AUTO;
-  const bool lin = domain != SWB_DOMAIN_LOG && xo <= 0.0 && xe <= 0.0 && lin_gaps<G>(xo, xe);
+  const bool lin = G == 0 && domain != SWB_DOMAIN_LOG && xo <= 0.0 && xe <= 0.0;
   if (G == 0 && domain == SWB_DOMAIN_LINEAR && !lin) return SWB_ERR_ARG;
   a.xgo = (float)exp2(xo);
   a.xge = (float)exp2(xe);
   if (a.ck_every < 1) a.ck_every = 1;
   a.dparams = opt ? opt->params_device : nullptr;
-  if (a.dparams && (G != 0 || !lin)) return SWB_ERR_ARG;   // device parameters: the local models in the linear domain
+  if (a.dparams && !lin) return SWB_ERR_ARG;   // device parameters: linear-domain kernels only
 
   // per-call resets: counters, status and completion counts to 0, cross-band
   // buffers to the NaN sentinel, the map to 0 (cells outside lengths stay 0)
@@ -375,10 +346,10 @@ int launch(Args a, const Layout& l, long long ntasks, size_t map_elems, bool cle
       cudaMemsetAsync(a.map, 0, map_elems * sizeof(float), st) != cudaSuccess)
     return SWB_ERR_CUDA;
 
-  if (R == 8 && (G != 0 || !lin)) return SWB_ERR_ARG;   // 8 columns per lane: the local models, linear domain
+  if (R == 8 && !lin) return SWB_ERR_ARG;   // 8 columns per lane: linear domain only
   constexpr int m = model_index<NS, G>();
-  const int of = lin ? d->locc[0][m][ridx(R)] : d->occ[0][m][R == 4];
-  const int ob = lin ? d->locc[1][m][ridx(R)] : d->occ[1][m][R == 4];
+  const int of = lin ? d->locc[0][NS == 3][ridx(R)] : d->occ[0][m][R == 4];
+  const int ob = lin ? d->locc[1][NS == 3][ridx(R)] : d->occ[1][m][R == 4];
   const int cta_cap_f = d->sms * (of > 0 ? of : 1);
   const int cta_cap_b = d->sms * (ob > 0 ? ob : 1);
   const long long need_f = (ntasks + kWarpsFwd - 1) / kWarpsFwd;
@@ -392,52 +363,33 @@ int launch(Args a, const Layout& l, long long ntasks, size_t map_elems, bool cle
   if (grid_f < 1) grid_f = 1;
   if (grid_b < 1) grid_b = 1;
   if (lin) {
-    if constexpr (G == 0 || R != 8) {
+    if constexpr (G == 0) {
       SegPlan seg;
       if (a.layout == 0 && !value_only && !a.fault_inject) {
         seg = seg_plan<R>(l, ntasks);
         if (ws_bytes < seg.total) seg = SegPlan{};
       }
-      launch_forward<NS, R, G>(a, *d, ntasks, opt ? opt->max_ctas : 0, st);
+      swb::lfwd_kernel<NS, R><<<grid_f, 32 * kWarpsFwd, 0, st>>>(a);
       if (cudaPeekAtLastError() != cudaSuccess) return SWB_ERR_CUDA;
       if (opt && opt->split_event &&
           cudaEventRecord(reinterpret_cast<cudaEvent_t>(opt->split_event), st) != cudaSuccess)
         return SWB_ERR_CUDA;
       if (value_only) {
-        swb::lvalue_kernel<NS, R, G><<<(a.B + 3) / 4, 128, 0, st>>>(a);
-      } else {
-        bool done = false;
-        if constexpr (R != 8) {
-          if (seg.total) {
-            rc = launch_segments<NS, R, G>(a, *d, seg, w, false, opt ? opt->max_ctas : 0, st);
-            if (rc != SWB_OK) return rc;
-            done = true;
-          }
-        }
-        if (!done) swb::lbwd_kernel<NS, R, kWarpsBwd, false, G><<<grid_b, 32 * kWarpsBwd, lbwd_smem<NS, R>(), st>>>(a);
+        swb::lvalue_kernel<NS, R><<<(a.B + 3) / 4, 128, 0, st>>>(a);
+        return cudaPeekAtLastError() == cudaSuccess ? SWB_OK : SWB_ERR_CUDA;
       }
-      if (cudaPeekAtLastError() != cudaSuccess) return SWB_ERR_CUDA;
-      if constexpr (G == 0) return SWB_OK;
-      // global and Saigo-Vert models: pairs whose values spread too far for
-      // fp32 frames run again in the log domain (none, as a rule: three
-      // launches that return at once)
-      if constexpr (G != 0) {
-        swb::redo_kernel<NS, R, G><<<std::min(a.B, 2 * d->sms), 128, 0, st>>>(a);
-        a.redo = 1;
-        const int fl = d->occ[0][m][R == 4], bl = d->occ[1][m][R == 4];
-        grid_f = (int)std::max(1LL, std::min<long long>(need_f, (long long)d->sms * std::max(fl, 1)));
-        grid_b = (int)std::max(1LL, std::min<long long>(need_b, (long long)d->sms * std::max(bl, 1)));
-        if (opt && opt->max_ctas > 0) {
-          grid_f = std::min(grid_f, opt->max_ctas);
-          grid_b = std::min(grid_b, opt->max_ctas);
-        }
+      if constexpr (swb::split_code<R>()) {
+        if (seg.total)
+          return launch_segments<NS, R>(a, *d, seg, w, false, opt ? opt->max_ctas : 0, st);
       }
+      swb::lbwd_kernel<NS, R, kWarpsBwd><<<grid_b, 32 * kWarpsBwd, lbwd_smem<NS, R>(), st>>>(a);
+      return cudaPeekAtLastError() == cudaSuccess ? SWB_OK : SWB_ERR_CUDA;
     }
   }
   if constexpr (R != 8) {   // the log-domain kernels have 2 or 4 columns per lane
     swb::fwd_kernel<NS, R, G><<<grid_f, 32 * kWarpsFwd, 0, st>>>(a);
     if (cudaPeekAtLastError() != cudaSuccess) return SWB_ERR_CUDA;
-    if (!a.redo && opt && opt->split_event &&
+    if (opt && opt->split_event &&
         cudaEventRecord(reinterpret_cast<cudaEvent_t>(opt->split_event), st) != cudaSuccess)
       return SWB_ERR_CUDA;
     if (value_only) {
@@ -475,7 +427,7 @@ template <int NS, int G = 0>
 int launch_padded(const float* scores, const int* lengths, int B, int L1m, int L2m, float go,
                   float ge, float T, float* value, float* map, float* g_open, float* g_ext,
                   float* g_T, void* ws, size_t ws_bytes, void* stream, const swb_options* opt) {
-  const int r = pick_r(opt, B, L2m, G == 0 && lin_eligible<NS, G>(go, ge, T, opt));
+  const int r = pick_r(opt, B, L2m, lin_eligible<NS, G>(go, ge, T, opt));
   if (r == 2)
     return launch_padded_r<NS, 2, G>(scores, lengths, B, L1m, L2m, go, ge, T, value, map, g_open,
                                      g_ext, g_T, ws, ws_bytes, stream, opt);
@@ -891,7 +843,10 @@ int ck_forward_r(const float* scores, const int* lengths, int B, int L1m, int L2
   if (cudaMemsetAsync(w, 0, l.off_part, st) != cudaSuccess) return SWB_ERR_CUDA;
   if (cudaMemsetAsync(w + l.off_sent, 0xff, l.sent_bytes, st) != cudaSuccess) return SWB_ERR_CUDA;
   const long long ntasks = (long long)B * l.nb;
-  launch_forward<NS, R, 0>(a, *d, ntasks, 0, st);
+  const int of = d->locc[0][NS == 3][ridx(R)];
+  const long long cap = (long long)d->sms * (of > 0 ? of : 1);
+  const int grid = (int)std::max(1LL, std::min((ntasks + kWarpsFwd - 1) / kWarpsFwd, cap));
+  swb::lfwd_kernel<NS, R><<<grid, 32 * kWarpsFwd, 0, st>>>(a);
   swb::lvalue_kernel<NS, R><<<(B + 3) / 4, 128, 0, st>>>(a);
   return cudaPeekAtLastError() == cudaSuccess ? SWB_OK : SWB_ERR_CUDA;
 }
@@ -921,10 +876,10 @@ int ck_adjoint_r(const float* scores, const int* lengths, int B, int L1m, int L2
   if (lengths && map_elems > 0 && cudaMemsetAsync(map, 0, map_elems * sizeof(float), st) != cudaSuccess)
     return SWB_ERR_CUDA;
   const long long ntasks = (long long)B * l.nb;
-  const int ob = kc > 1 ? d->locc_sparse[NS == 3][ridx(R)] : d->locc[1][model_index<NS, 0>()][ridx(R)];
+  const int ob = kc > 1 ? d->locc_sparse[NS == 3][ridx(R)] : d->locc[1][NS == 3][ridx(R)];
   const long long cap = (long long)d->sms * (ob > 0 ? ob : 1);
   const int grid = (int)std::max(1LL, std::min((ntasks + kWarpsBwd - 1) / kWarpsBwd, cap));
-  if constexpr (R != 8) {
+  if constexpr (swb::split_code<R>()) {
     const SegPlan seg = seg_plan<R>(l, ntasks);
     if (seg.total && ws_bytes >= seg.total) return launch_segments<NS, R>(a, *d, seg, w, kc > 1, 0, st);
   }
@@ -1287,8 +1242,8 @@ int swb_nw_forward(const float* scores, const int* lengths, int B, int L1max, in
 
 size_t swb_nw_affine_workspace_bytes(int B, int L1max, int L2max) {
   if (B <= 0) return 0;
-  return std::max(with_segments<2>(layout_for<3, 2, 1>(B, L1max, L2max), B),
-                  with_segments<4>(layout_for<3, 4, 1>(B, L1max, L2max), B));
+  return std::max(layout_for<3, 2, 1>(B, L1max, L2max).total,
+                  layout_for<3, 4, 1>(B, L1max, L2max).total);
 }
 
 int swb_nw_affine_forward(const float* scores, const int* lengths, int B, int L1max, int L2max,
@@ -1330,8 +1285,8 @@ int swb_nw_affine_ragged_value(const float* scores, const void* host_plan, const
 
 size_t swb_sv_affine_workspace_bytes(int B, int L1max, int L2max) {
   if (B <= 0) return 0;
-  return std::max(with_segments<2>(layout_for<3, 2, 2>(B, L1max, L2max), B),
-                  with_segments<4>(layout_for<3, 4, 2>(B, L1max, L2max), B));
+  return std::max(layout_for<3, 2, 2>(B, L1max, L2max).total,
+                  layout_for<3, 4, 2>(B, L1max, L2max).total);
 }
 
 int swb_sv_affine_forward(const float* scores, const int* lengths, int B, int L1max, int L2max,

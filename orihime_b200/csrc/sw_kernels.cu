@@ -76,10 +76,6 @@ struct KSum {
 // ops: into its output map), so a timeout shows in the results without any
 // host synchronisation; the status word records it as well.
 constexpr unsigned PAIR_TIMEOUT = 0x80000000u;
-// Bit 30: the linear-domain forward leaves the pair to the log-domain kernels;
-// bit 29: its adjoint does.
-constexpr unsigned PAIR_REDO = 0x40000000u, PAIR_LOST = 0x20000000u;
-constexpr unsigned PAIR_FLAGS = PAIR_TIMEOUT | PAIR_REDO | PAIR_LOST;
 
 __device__ __forceinline__ void mark_timeout(unsigned* status, unsigned* flag) {
   atomicOr(status, ERR_WAIT_TIMEOUT);
@@ -942,7 +938,6 @@ __device__ void fwd_band(const Args& a, const Place& w, int lane, uint64_t deadl
 
 template <int NS, int R, int GM = 0>
 __global__ void __launch_bounds__(128) fwd_kernel(Args a) {
-  if (a.redo && a.status[1] == 0u) return;   // no pair to run again
   const int lane = threadIdx.x & 31;
   const uint64_t deadline = gtimer() + a.spin_limit_ns;
   const int ntasks = (a.layout == 0) ? a.B * a.nb : a.ntasks;
@@ -951,9 +946,7 @@ __global__ void __launch_bounds__(128) fwd_kernel(Args a) {
     if (lane == 0) task = (int)atomicAdd(a.counters + 0, 1u);
     task = __shfl_sync(FULL, task, 0);
     if (task >= ntasks) break;
-    const Place w = place_of<NS, R, GM>(a, task, false);
-    if (a.redo && !(a.pair_done[w.p] & PAIR_REDO)) continue;
-    fwd_band<NS, R, GM>(a, w, lane, deadline);
+    fwd_band<NS, R, GM>(a, place_of<NS, R, GM>(a, task, false), lane, deadline);
   }
 }
 
@@ -1046,7 +1039,7 @@ __global__ void __launch_bounds__(128) value_kernel(Args a) {
   constexpr bool G = GM == 1;
   const int lane = threadIdx.x & 31;
   const int q = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (q >= a.B || (a.redo && !(a.pair_done[q] & PAIR_REDO))) return;
+  if (q >= a.B) return;
   Place w;
   if (a.layout == 0) {
     w = place_of<NS, R, GM>(a, q * a.nb, false);
@@ -1104,7 +1097,7 @@ __device__ void finish_pair_p(const Args& a, const Place& w, int lane, float Sh,
     gp[0] = g0sum; gp[1] = g1sum; gp[2] = pssum; gp[3] = 0.f;
     __threadfence();
     unsigned done = atomicAdd(a.pair_done + p, 1u);
-    if ((done & ~PAIR_FLAGS) == (unsigned)w.nb - 1) {
+    if ((done & ~PAIR_TIMEOUT) == (unsigned)w.nb - 1) {
       __threadfence();
       if (done & PAIR_TIMEOUT) {   // a bounded wait of this pair expired
         const float nan = __int_as_float(0x7fc00000);
@@ -1633,7 +1626,6 @@ __host__ __device__ constexpr int bwd_smem_floats() {
 
 template <int NS, int R, int WARPS, int GM = 0>
 __global__ void __launch_bounds__(32 * WARPS) bwd_kernel(Args a) {
-  if (a.redo && a.status[1] == 0u) return;   // no pair to run again
   extern __shared__ float smem[];
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
@@ -1645,9 +1637,7 @@ __global__ void __launch_bounds__(32 * WARPS) bwd_kernel(Args a) {
     if (lane == 0) task = (int)atomicAdd(a.counters + 1, 1u);
     task = __shfl_sync(FULL, task, 0);
     if (task >= ntasks) break;
-    const Place p = place_of<NS, R, GM>(a, task, true);
-    if (a.redo && !(a.pair_done[p.p] & PAIR_REDO)) continue;
-    bwd_band<NS, R, GM>(a, p, lane, sm, deadline);
+    bwd_band<NS, R, GM>(a, place_of<NS, R, GM>(a, task, true), lane, sm, deadline);
   }
 }
 

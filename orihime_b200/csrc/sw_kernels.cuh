@@ -109,7 +109,7 @@ struct Args {
   float* g_T;
   // workspace (see layout_for in sw_capi.cu)
   unsigned* counters;         // [0] forward task counter, [1] adjoint task counter
-  unsigned* status;           // [0] error bits, [1] some pair is flagged PAIR_REDO
+  unsigned* status;           // error bits
   unsigned* pair_done;        // [B]
   float* part;                // [B*nb][2] partition partials (ref, sum)
   float* gpart;               // [B*nb][4] gradient partials
@@ -120,7 +120,6 @@ struct Args {
   float* bck;                 // [B*nb][nseg] outside-recursion states
   float* spart;               // [B*nb][nseg][4] gradient partials
   int nseg;                   // segments per band
-  int redo;                   // log-domain kernels: 1 runs only the pairs flagged PAIR_REDO
   unsigned long long spin_limit_ns;
   int fault_inject;           // 1: band>0 waits on a word nobody writes (tests only)
   float* never_written;       // target of fault_inject polls

@@ -136,31 +136,6 @@ __device__ __forceinline__ void zero_chunk_rows(const Pair& pr, int kc, int col0
   }
 }
 
-// Parameters of a linear-domain launch: the launch's floats, or read from the
-// device parameter array when there is one (a stream capture with tensor
-// parameters: each replay reads their current values).  k and the transition
-// factors are formed exactly as the host forms them.  ok is false for a
-// temperature that is not finite and positive or a positive gap: the linear
-// domain needs every transition factor <= 1.
-struct LParams {
-  float go, ge, T, k, xgo, xge;
-  bool ok;
-};
-template <int NS>
-__device__ __forceinline__ LParams lparams(const Args& a) {
-  LParams p{a.go, a.ge, a.T, a.k, a.xgo, a.xge, true};
-  if (a.dparams) {
-    p.go = a.dparams[0];
-    p.ge = NS == 3 ? a.dparams[1] : 0.f;
-    p.T = a.dparams[NS == 3 ? 2 : 1];
-    p.k = 1.4426950408889634f / p.T;
-    p.xgo = (float)exp2((double)p.go * (double)p.k);
-    p.xge = (float)exp2((double)p.ge * (double)p.k);
-    p.ok = p.T > 0.f && p.T < INFINITY && p.go * p.k <= 0.f && p.ge * p.k <= 0.f;
-  }
-  return p;
-}
-
 // ---------------------------------------------------------------------------
 // packed columns
 // ---------------------------------------------------------------------------
@@ -190,17 +165,6 @@ template <int H> __device__ __forceinline__ float sum2(const float2 (&p)[H]) {
 // 2^d as bits for d + 127 given: 0 below the exponent range.
 __device__ __forceinline__ float p2b(int d127) { return __int_as_float(max(d127, 0) << 23); }
 
-// Columns past the pair (DM): 0 the band has none, 1 it may have some and they
-// are masked without a branch, 2 a warp-uniform branch on whether it has any.
-// Kernels that run with every scheduler full keep one copy of their steps (2,
-// and no copy for chunks inside the pair): with several the instruction cache
-// misses cost more than the branches (4096 ragged pairs at 8 columns per lane,
-// forward + adjoint: 7.0 ms against 5.0).  The sweeps of small batches (SPLIT)
-// run a warp or two per scheduler, and there a branch costs its latency.
-template <int DM> __device__ __forceinline__ bool masks(bool has_dead) {
-  return DM == 1 || (DM == 2 && has_dead);
-}
-
 // Checkpoint floats per lane (CKF, padded to float4), one checkpoint record
 // (LREC: CK4 groups of [lane][4]) and adjoint shared-memory floats per lane
 // per step (FW).  A band's checkpoint region holds ceil(nchunks / ck_every)
@@ -222,64 +186,6 @@ template <int NS, int R> struct LDims {
   static constexpr int FW = NF * R + 1;
 };
 
-// Model variants (template argument GM, as in sw_kernels.cu): 0 the local
-// models, 1 the global ones, 2 Saigo-Vert.  Against the recurrences above:
-// * global (soft Needleman-Wunsch): no fresh start and one end, the cell
-//   (L1, L2); A[i,j] = E A_diag + G (A_up + A_left), and with affine gaps also
-//   I from D above and D from I on the left, at the open factor.  Row 0 and
-//   column 0 hold the boundary gaps.  Frames are not floored at 0 (there is no
-//   weight 1 to keep), ZF stands for "no value yet".
-// * Saigo-Vert: D also from I on the left (open factor), and only M ends.
-constexpr int ZF_NONE = -(1 << 28);
-template <int GM> __host__ __device__ constexpr int zero_frame() { return GM == 1 ? ZF_NONE : 0; }
-template <int GM> __device__ __forceinline__ int floor_frame(int n) { return GM == 1 ? n : max(n, 0); }
-// Frames in cross-band records are biased so that no word is the sentinel.
-template <int GM> __host__ __device__ constexpr int frame_bias() { return GM ? (1 << 29) : 0; }
-
-// ---- spread.  A lane keeps its columns of a row under one frame, so a value
-// far enough below the row's largest loses bits or all of it.  The
-// double-float log-domain kernels do not, so the models that they otherwise
-// serve (GM 1 and 2) place their rows HEADROOM bits higher in fp32's range
-// (scores up to XHEAD fit on top of it), which leaves 2^-174 below a row's
-// inputs, and watch what is left; a pair in which it may have mattered is run
-// again in the log domain:
-// * the forward flags a pair when a raw value of some lane's row is below
-//   2^-SPREAD (Saigo-Vert: values below 2^-45 of the empty alignment do not
-//   count, as any continuation of theirs weighs less than a fresh start), or
-//   when a score passes XHEAD;
-// * the adjoint flags a pair when a raw value of beta is below 2^-SPREAD where
-//   it may count: where 2^-126 of the row's frame times the row's alpha is
-//   over 2^-45 of Z (with a bit of its own: bands of the pair that have not
-//   started must not stop, their neighbours wait for them).
-// Of 1024 pairs of 32 to 1024 rows and columns at T = 0.5, one or two come
-// within 2^-110 of a row's largest value, and each such pair run again costs a
-// whole chain of log-domain steps; hence the headroom.
-template <int GM> __host__ __device__ constexpr int headroom() { return GM ? 48 : 0; }
-template <int GM> __host__ __device__ constexpr float score_max() { return GM ? 70.f : XMAX; }
-constexpr int SPREAD = 124;
-__device__ __forceinline__ void flag_redo(const Args& a, int p, int lane, unsigned flag) {
-  if (lane == 0) {
-    atomicOr(a.pair_done + p, flag);
-    atomicOr(a.status + 1, 1u);
-  }
-}
-__device__ __forceinline__ unsigned ld_flag(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ bool redo_set(const Args& a, int p) { return (ld_flag(a.pair_done + p) & PAIR_REDO) != 0; }
-// Smallest live column of a row of sums.
-template <int DM, int H> __device__ __forceinline__ float min2(const float2 (&p)[H], int nlive, bool hd) {
-  float m = INFINITY;
-#pragma unroll
-  for (int k = 0; k < H; ++k) {
-    const bool x = !masks<DM>(hd) || k < nlive, y = !masks<DM>(hd) || k + H < nlive;
-    m = fminf(m, fminf(x ? p[k].x : INFINITY, y ? p[k].y : INFINITY));
-  }
-  return m;
-}
-
 // Lane state of the forward wavefront.
 template <int NS, int R> struct LState {
   static constexpr int H = R / 2;
@@ -293,7 +199,7 @@ template <int NS, int R> struct LState {
 // Exponent bound of a non-negative sum: x <= 2^(sexp(x) - 126).
 __device__ __forceinline__ int sexp(float x) { return (int)(__float_as_uint(x) >> 23); }
 
-template <int NS, int R, int GM>
+template <int NS, int R>
 __device__ __forceinline__ void lstate_zero(LState<NS, R>& s) {
   constexpr int H = R / 2;
 #pragma unroll
@@ -302,51 +208,19 @@ __device__ __forceinline__ void lstate_zero(LState<NS, R>& s) {
     if constexpr (NS == 3) { s.v[1][k] = dup2(0.f); s.c[k] = dup2(0.f); }
   }
   s.ds = 0.f; s.od = 0.f; s.oc = 0.f;
-  s.e = zero_frame<GM>(); s.n = s.e; s.nd = s.e;
+  s.e = 0; s.n = 0; s.nd = 0;
 }
 
-// 2^x as a mantissa in (0.5, 1] under the frame e (x may be far out of range).
-__device__ __forceinline__ float split2(double x, int& e) {
-  const double f = ceil(x);
-  e = (int)f;
-  return exp2f((float)(x - f));
-}
-// log2 of the boundary gap of length n >= 1 (affine: open, then extensions).
-template <int NS> __device__ __forceinline__ double gap_log2(const LParams& lp, int n) {
-  const double o = (double)lp.go * (double)lp.k;
-  return NS == 3 ? o + (double)(n - 1) * ((double)lp.ge * (double)lp.k) : (double)n * o;
-}
-
-// Global alignment: the lane's columns of row 0 (jl columns lie to the left).
-template <int NS, int R, int DM>
-__device__ __forceinline__ void lstate_row0(LState<NS, R>& s, float2 (&d)[R / 2], const LParams& lp, int jl,
-                                            int nlive, bool hd) {
-  constexpr int H = R / 2;
-  lstate_zero<NS, R, 1>(s);
-  if (nlive > 0) {
-    split2(gap_log2<NS>(lp, jl + 1), s.e);
-    float2 x[H];
-#pragma unroll
-    for (int c = 0; c < R; ++c) {   // D as ldchain rebuilds it from its first column
-      if (NS == 3 && c > 0) col(x, c) = lp.xge * col(x, c - 1);
-      else col(x, c) = exp2f((float)(gap_log2<NS>(lp, jl + 1 + c) - (double)s.e));
-    }
-    if (masks<DM>(hd)) {
-#pragma unroll
-      for (int c = 0; c < R; ++c)
-        if (c >= nlive) col(x, c) = 0.f;
-    }
-#pragma unroll
-    for (int k = 0; k < H; ++k) {
-      if constexpr (NS == 3) { d[k] = x[k]; s.c[k] = x[k]; }
-      else s.v[0][k] = x[k];
-    }
-    const double left = jl > 0 ? gap_log2<NS>(lp, jl) : 0.0;   // the cell (0, jl)
-    s.ds = exp2f((float)(left - (double)s.e));
-    s.nd = (int)ceil(left);
-    s.n = s.e - 126 + sexp(sum2(x));
-    s.oc = x[H - 1].y;
-  }
+// Columns past the pair (DM): 0 the band has none, 1 it may have some and they
+// are masked without a branch, 2 a warp-uniform branch on whether it has any.
+// The kernels at 8 columns per lane, which run with every scheduler full,
+// keep one copy of their steps (2, and no copy for chunks inside the pair):
+// with several the instruction cache misses cost more than the branches
+// (4096 ragged pairs, forward + adjoint: 7.0 ms against 5.0).  The narrower
+// ones run few warps, and there a branch costs its latency.
+template <int R> __host__ __device__ constexpr bool split_code() { return R < 8; }
+template <int DM> __device__ __forceinline__ bool masks(bool has_dead) {
+  return DM == 1 || (DM == 2 && has_dead);
 }
 
 // D of a row from its first column's D and the row's M: D runs along the
@@ -368,13 +242,6 @@ __device__ __forceinline__ void ldchain(const float2 (&m)[R / 2], float d0, floa
     for (int c = 0; c < R; ++c)
       if (c >= nlive) col(d, c) = 0.f;
   }
-}
-
-// What D opens from: M, and I where the model lets D follow I.
-template <int R, int GM>
-__device__ __forceinline__ void dsource(const float2 (&m)[R / 2], const float2 (&iv)[R / 2], float2 (&o)[R / 2]) {
-#pragma unroll
-  for (int k = 0; k < R / 2; ++k) o[k] = GM ? add2(m[k], iv[k]) : m[k];
 }
 
 template <int NS, int R>
@@ -401,7 +268,7 @@ __device__ __forceinline__ void lck_store(float* rec, int lane, const LState<NS,
 // Restores the lane state of a record (`rec` + lane: global or staged in
 // shared memory), rebuilding D, the sums and the normalised frame with the
 // operations lcells used for that row; `d` is the row's D.
-template <int NS, int R, int DM, int GM>
+template <int NS, int R, int DM>
 __device__ __forceinline__ void lck_restore(const float* rec, int lane, LState<NS, R>& s, float gO, float gE,
                                             int nlive, bool hd, float2 (&d)[R / 2]) {
   using L = LDims<NS, R>;
@@ -422,9 +289,7 @@ __device__ __forceinline__ void lck_restore(const float* rec, int lane, LState<N
   s.nd = __float_as_int(x[V + 2]);
   float rs;
   if constexpr (NS == 3) {
-    float2 ds[H];
-    dsource<R, GM>(s.v[0], s.v[1], ds);
-    ldchain<NS, R, DM>(ds, x[V + 3], gO, gE, nlive, hd, d, s.od);
+    ldchain<NS, R, DM>(s.v[0], x[V + 3], gO, gE, nlive, hd, d, s.od);
 #pragma unroll
     for (int k = 0; k < H; ++k) s.c[k] = add2(add2(s.v[0][k], s.v[1][k]), d[k]);
     s.oc = s.c[H - 1].y;
@@ -434,7 +299,7 @@ __device__ __forceinline__ void lck_restore(const float* rec, int lane, LState<N
     s.oc = s.v[0][H - 1].y;
     rs = sum2(s.v[0]);
   }
-  s.n = floor_frame<GM>(s.e - 126 + sexp(rs));
+  s.n = max(s.e - 126 + sexp(rs), 0);
 }
 
 // One step of the forward wavefront for one lane: (xd, xc) are the left
@@ -443,7 +308,7 @@ __device__ __forceinline__ void lck_restore(const float* rec, int lane, LState<N
 // frame et (its raw frame from then on) and returns the row's sum over its
 // columns and states in `rs`.
 // Affine: M, I and `d` = D; linear: A and `d` = the emission part.
-template <int NS, int R, int DM, int GM>
+template <int NS, int R, int DM>
 __device__ __forceinline__ void lcells(LState<NS, R>& s, float xd, float xc, int xe, int xn,
                                        const float2 (&E)[R / 2], float gO, float gE, int nlive, bool hd,
                                        float2 (&d)[R / 2], float& rs) {
@@ -451,26 +316,22 @@ __device__ __forceinline__ void lcells(LState<NS, R>& s, float xd, float xc, int
   // the row's frame is at least every input's normalised frame, so that every
   // converted input is <= 1 (a raw value's frame exceeds its normalised frame
   // by at most 126)
-  int et = max(max(s.n, xn), s.nd);
-  if constexpr (GM != 0) et = max(max(et - headroom<GM>(), s.e - 127), xe - 127);   // (conversions stay below 2^128)
+  const int et = max(max(s.n, xn), s.nd);
   s.nd = xn;
   const int q = 127 - et;
   const float fU = p2b(s.e + q), fL = p2b(xe + q);
-  const float2 fU2 = dup2(fU), st2 = dup2(GM == 1 ? 0.f : p2b(q));   // st: the fresh-start term 1 in frame et
+  const float2 fU2 = dup2(fU), st2 = dup2(p2b(q));   // st: the fresh-start term 1 in frame et
   if constexpr (NS == 3) {
     float2 m[H];
 #pragma unroll
     for (int k = 0; k < H; ++k) {
       const float2 p = k == 0 ? make_float2(s.ds, s.c[H - 1].x) : s.c[k > 0 ? k - 1 : 0];
-      m[k] = GM == 1 ? mul2(E[k], mul2(fU2, p)) : mul2(E[k], fma2(fU2, p, st2));
+      m[k] = mul2(E[k], fma2(fU2, p, st2));
     }
     const float2 gOu = dup2(gO * fU), gEu = dup2(gE * fU);
 #pragma unroll
-    for (int k = 0; k < H; ++k)   // I opens from M above (global: and from D above)
-      s.v[1][k] = fma2(gOu, GM == 1 ? add2(s.v[0][k], d[k]) : s.v[0][k], mul2(gEu, s.v[1][k]));
-    float2 ds[H];
-    dsource<R, GM>(m, s.v[1], ds);
-    ldchain<NS, R, DM>(ds, xd * fL, gO, gE, nlive, hd, d, s.od);
+    for (int k = 0; k < H; ++k) s.v[1][k] = fma2(gOu, s.v[0][k], mul2(gEu, s.v[1][k]));
+    ldchain<NS, R, DM>(m, xd * fL, gO, gE, nlive, hd, d, s.od);
 #pragma unroll
     for (int k = 0; k < H; ++k) {
       s.v[0][k] = m[k];
@@ -485,7 +346,7 @@ __device__ __forceinline__ void lcells(LState<NS, R>& s, float xd, float xc, int
 #pragma unroll
     for (int k = 0; k < H; ++k) {
       const float2 p = k == 0 ? make_float2(s.ds, s.v[0][H - 1].x) : s.v[0][k > 0 ? k - 1 : 0];
-      d[k] = GM == 1 ? mul2(E[k], mul2(fU2, p)) : mul2(E[k], fma2(fU2, p, st2));
+      d[k] = mul2(E[k], fma2(fU2, p, st2));
     }
 #pragma unroll
     for (int k = 0; k < H; ++k) x[k] = fma2(gU, s.v[0][k], d[k]);
@@ -504,23 +365,12 @@ __device__ __forceinline__ void lcells(LState<NS, R>& s, float xd, float xc, int
   // the row sum over columns and states bounds every value of the row (all
   // are >= 0) and is the row's partition term
   s.e = et;
-  s.n = floor_frame<GM>(1 - q + sexp(rs));
-}
-
-// Rows outside the pair have E = 0 in the outside recursion: the scores there
-// are whatever was loaded last, and a lane's state above row 1 enters the
-// quiet-chunk test of its warp.
-template <int R>
-__device__ __forceinline__ void lblank(bool act, float2 (&xs)[R / 2], float2 (&E)[R / 2]) {
-#pragma unroll
-  for (int j = 0; j < R / 2; ++j) {
-    if (!act) { xs[j] = dup2(NEG); E[j] = dup2(0.f); }
-  }
+  s.n = max(1 - q + sexp(rs), 0);
 }
 
 // Scaled scores and emissions of one step as pairs: clamped at XMAX, NEG
 // (E = 0) in columns past the pair.
-template <int R, int DM, int GM>
+template <int R, int DM>
 __device__ __forceinline__ void lemit(const float (&sb)[R], float k, int nlive, bool hd, float2 (&xs)[R / 2],
                                       float2 (&E)[R / 2]) {
   constexpr int H = R / 2;
@@ -528,8 +378,8 @@ __device__ __forceinline__ void lemit(const float (&sb)[R], float k, int nlive, 
 #pragma unroll
   for (int c = 0; c < R; c += 2) {
     const float2 t = mul2(make_float2(sb[c], sb[c + 1]), dup2(k));
-    x[c] = fminf(t.x, score_max<GM>());
-    x[c + 1] = fminf(t.y, score_max<GM>());
+    x[c] = fminf(t.x, XMAX);
+    x[c + 1] = fminf(t.y, XMAX);
   }
   if (masks<DM>(hd)) {
 #pragma unroll
@@ -652,16 +502,15 @@ __device__ __forceinline__ float ld_poll_if(const float* p, bool ok) {
 // float2 (oc, the two frames packed).  A band's records start at the next
 // 16-byte boundary of its edge slice (2 NS floats per row hold them with the
 // padding; slices start at even offsets).
-template <int NS, int GM = 0> struct LEdge {
-  static constexpr int BIAS = frame_bias<GM>(), B16 = GM ? (1 << 23) : 0;   // affine; linear
+template <int NS> struct LEdge {
   __device__ static __forceinline__ float* base(float* edge, size_t off) {
     return edge + (NS == 3 ? (off + 3) / 4 * 4 : off);
   }
   __device__ static __forceinline__ void put(float* b, int i, float od, float oc, int e, int n, int rs_exp) {
     if constexpr (NS == 3) {
-      reinterpret_cast<float4*>(b)[i - 1] = make_float4(od, oc, __int_as_float(e + BIAS), __int_as_float(n + BIAS));
+      reinterpret_cast<float4*>(b)[i - 1] = make_float4(od, oc, __int_as_float(e), __int_as_float(n));
     } else {
-      reinterpret_cast<float2*>(b)[i - 1] = make_float2(oc, __uint_as_float(((unsigned)(e + B16) << 8) | (unsigned)rs_exp));
+      reinterpret_cast<float2*>(b)[i - 1] = make_float2(oc, __uint_as_float(((unsigned)e << 8) | (unsigned)rs_exp));
     }
   }
   // record i (0 where !ok), a strong load; no branch
@@ -687,28 +536,18 @@ template <int NS, int GM = 0> struct LEdge {
   }
   // (od, oc, e, n) of a resolved record
   __device__ static __forceinline__ float4 open(const float4& v) {
-    if constexpr (NS == 3)
-      return make_float4(v.x, v.y, __int_as_float(__float_as_int(v.z) - BIAS), __int_as_float(__float_as_int(v.w) - BIAS));
+    if constexpr (NS == 3) return v;
     const unsigned w = __float_as_uint(v.y);
-    const int e = (int)(w >> 8) - B16;
-    return make_float4(0.f, v.x, __int_as_float(e), __int_as_float(floor_frame<GM>(e - 126 + (int)(w & 0xffu))));
-  }
-  // The record that column 0 of a global alignment stands for at row i (a gap
-  // of length i), as `open` gives it; column 0 of the other models is empty.
-  __device__ static __forceinline__ float4 column0(const LParams& lp, int i) {
-    if constexpr (GM != 1) return make_float4(0.f, 0.f, 0.f, 0.f);
-    int e;
-    const float m = split2(gap_log2<NS>(lp, i), e);
-    return make_float4(lp.xgo * m, m, __int_as_float(e), __int_as_float(e));
+    const int e = (int)(w >> 8);
+    return make_float4(0.f, v.x, __int_as_float(e), __int_as_float(max(e - 126 + (int)(w & 0xffu), 0)));
   }
   // Bounded wait for record i; on expiry the status word and the pair's flag
-  // are set and the record reads as 0 (also when the pair is to be run again).
+  // are set and the record reads as 0.
   __device__ static __noinline__ float4 wait(const float* b, int i, uint64_t deadline, unsigned* status,
                                              unsigned* flag) {
     for (int tries = 0;; ++tries) {
       const float4 v = get(b, i, true);
       if (!missing(v)) return v;
-      if (GM != 0 && (ld_flag(flag) & PAIR_REDO)) return make_float4(0.f, 0.f, 0.f, 0.f);
       if (gtimer() > deadline) {
         mark_timeout(status, flag);
         return make_float4(0.f, 0.f, 0.f, 0.f);
@@ -732,6 +571,31 @@ __device__ __forceinline__ void lscores(const float (&sb)[R], float k, int nlive
   }
 }
 
+// Parameters of a linear-domain launch: the launch's floats, or read from the
+// device parameter array when there is one (a stream capture with tensor
+// parameters: each replay reads their current values).  k and the transition
+// factors are formed exactly as the host forms them.  ok is false for a
+// temperature that is not finite and positive or a positive gap: the linear
+// domain needs every transition factor <= 1.
+struct LParams {
+  float go, ge, T, k, xgo, xge;
+  bool ok;
+};
+template <int NS>
+__device__ __forceinline__ LParams lparams(const Args& a) {
+  LParams p{a.go, a.ge, a.T, a.k, a.xgo, a.xge, true};
+  if (a.dparams) {
+    p.go = a.dparams[0];
+    p.ge = NS == 3 ? a.dparams[1] : 0.f;
+    p.T = a.dparams[NS == 3 ? 2 : 1];
+    p.k = 1.4426950408889634f / p.T;
+    p.xgo = (float)exp2((double)p.go * (double)p.k);
+    p.xge = (float)exp2((double)p.ge * (double)p.k);
+    p.ok = p.T > 0.f && p.T < INFINITY && p.go * p.k <= 0.f && p.ge * p.k <= 0.f;
+  }
+  return p;
+}
+
 // ---------------------------------------------------------------------------
 // forward band task
 // ---------------------------------------------------------------------------
@@ -739,11 +603,11 @@ __device__ __forceinline__ void lscores(const float (&sb)[R], float k, int nlive
 // Score prefetch distance of the tangent kernels' forward (steps).
 constexpr int FPF = C_STEPS;
 // Score prefetch distance of the sweeps (steps): each row is requested this
-// many steps ahead; small batches, whose steps are shorter, look further.
-template <bool SPLIT> __host__ __device__ constexpr int fwd_ahead() { return SPLIT ? 8 : 4; }
+// many steps ahead; the narrow kernels, whose steps are shorter, look further.
+template <int R> __host__ __device__ constexpr int fwd_ahead() { return R == 8 ? 4 : 8; }
 // Steps per block of the forward: the left band's records are passed a block
 // at a time (about 220 cycles a time in a lone warp).
-template <bool SPLIT> __host__ __device__ constexpr int fwd_block() { return SPLIT ? 2 * C_STEPS : C_STEPS; }
+template <int R> __host__ __device__ constexpr int fwd_block() { return split_code<R>() ? 2 * C_STEPS : C_STEPS; }
 
 // Forward wavefront of one band: per-lane partition sums (plain within a
 // chunk, Kahan over chunks, in the lane's largest normalised frame), the
@@ -757,12 +621,12 @@ template <bool SPLIT> __host__ __device__ constexpr int fwd_block() { return SPL
 // records had been written by then starts without waiting for anything.
 //
 // DM (see above): 1 also where rows are not 16-byte aligned.
-template <int NS, int R, int DM, int GM, bool SPLIT>
+template <int NS, int R, int DM>
 __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int lane,
                           uint64_t deadline, float4* sedge) {
   using LD = LDims<NS, R>;
-  using LE = LEdge<NS, GM>;
-  constexpr int H = R / 2, AH = fwd_ahead<SPLIT>(), WB = fwd_block<SPLIT>();
+  using LE = LEdge<NS>;
+  constexpr int H = R / 2, AH = fwd_ahead<R>(), WB = fwd_block<R>();
   check_lengths(a, w, lane);
   if (!lp.ok && w.band == 0 && lane == 0) {
     atomicOr(a.status, ERR_BAD_PARAMS);
@@ -774,7 +638,7 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
   const size_t slot = w.slot0 + band;
   const int col0 = band * 32 * R;
   float* part = a.part + 2 * (size_t)slot;
-  if (!(L1 > 0 && col0 < L2) || (GM != 0 && redo_set(a, w.p))) {
+  if (!(L1 > 0 && col0 < L2)) {
     if (lane == 0) { part[0] = 0.f; part[1] = (band == 0) ? 1.f : 0.f; }
     return;
   }
@@ -793,12 +657,10 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
   int next_ck = 0;   // the next chunk whose record is kept
 
   LState<NS, R> s;
+  lstate_zero(s);
   float2 d[H];
 #pragma unroll
   for (int j = 0; j < H; ++j) d[j] = dup2(0.f);
-  if constexpr (GM == 1) lstate_row0<NS, R, DM>(s, d, lp, jl, nlive, hd);
-  else lstate_zero<NS, R, GM>(s);
-  int spread = 0;   // the lane's largest spread so far
   float zm = (band == 0 && lane == 0) ? 1.f : 0.f, zc = 0.f;   // M[0,0]: the empty alignment
   int ze = 0;
 
@@ -810,7 +672,6 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
   };
   float4 ea = get_edge(0), eb = get_edge(1);
   bool ready = false;   // this block's records are in shared memory
-  [[maybe_unused]] bool stop = false;
   Rows<R> rows;
   rows.init(pr, jl, col0);
   const float* src = rows.at(1 - lane);
@@ -841,18 +702,12 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
         ea = LE::wait(ein, ie, deadline, a.status, a.pair_done + w.p);
       }
       __syncwarp();
-      if (lane < WB) se[lane] = ein || GM != 1 ? LE::open(ea) : LE::column0(lp, ie);
+      if (lane < WB) se[lane] = LE::open(ea);
       __syncwarp();
     }
     // the next block's records, if they are there (fault injection: never)
     ready = __all_sync(FULL, !LE::missing(eb)) && !fault;
-    if (ready && lane < WB)
-      sedge[((bl + 1) & 1) * WB + lane] = ein || GM != 1 ? LE::open(eb) : LE::column0(lp, (bl + 1) * WB + lane + 1);
-    if constexpr (GM != 0) {   // the pair is to be run again in the log domain: leave it
-      if (__any_sync(FULL, spread > SPREAD)) flag_redo(a, w.p, lane, PAIR_REDO);
-      if (stop) return;
-      stop = __any_sync(FULL, lane == 0 && redo_set(a, w.p));
-    }
+    if (ready && lane < WB) sedge[((bl + 1) & 1) * WB + lane] = LE::open(eb);
     ea = eb;
     eb = get_edge(bl + 2);
     const bool in_block = rows.inside(bl * (WB / C_STEPS)) && rows.inside((bl + 1) * (WB / C_STEPS) - 1 + AH / C_STEPS);
@@ -889,35 +744,22 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
         xe = lane == 0 ? __float_as_int(e4.z) : xe;
         xn = lane == 0 ? __float_as_int(e4.w) : xn;
         float2 xs[H], E[H];
-        lemit<R, DD, GM>(sb[(h * C_STEPS + cu) % AH], k, nlive, hd, xs, E);
+        lemit<R, DD>(sb[(h * C_STEPS + cu) % AH], k, nlive, hd, xs, E);
         if constexpr (IN) rows.template fetch<VEC>(src, sb[(h * C_STEPS + cu) % AH]);
         else rows.load(src, i + cu + AH, sb[(h * C_STEPS + cu) % AH]);
         src += rows.ld;
         rsv[cu] = 0.f;
         ev[cu] = 0;
         if (act) {
-          lcells<NS, R, DD, GM>(s, xd, xc, xe, xn, E, gO, gE, nlive, hd, d, rsv[cu]);
-          if constexpr (GM != 0) {
-            float lo;
-            if constexpr (NS == 3) lo = min2<DD>(s.c, nlive, hd);
-            else lo = min2<DD>(s.v[0], nlive, hd);
-            const int x = GM == 2 ? max(sexp(lo), 81 - s.e) : sexp(lo);
-            float top = xs[0].x;   // a clamped score (the log domain takes any)
-#pragma unroll
-            for (int j = 0; j < H; ++j) top = fmaxf(top, fmaxf(xs[j].x, xs[j].y));
-            if (top >= score_max<GM>()) spread = 127;
-            if (DD == 0 || nlive > 0) spread = max(spread, 127 - x);   // 1 in the row's frame against its least value
-          }
-          const int rx = sexp(rsv[cu]);
-          if constexpr (GM == 2) rsv[cu] = sum2(s.v[0]);   // only M ends an alignment
+          lcells<NS, R, DD>(s, xd, xc, xe, xn, E, gO, gE, nlive, hd, d, rsv[cu]);
           ev[cu] = s.e;
           cmx = max(cmx, s.n);
-          if (lane == 31) LE::put(eout, i + cu, s.od, s.oc, s.e, s.n, rx);
+          if (lane == 31) LE::put(eout, i + cu, s.od, s.oc, s.e, s.n, sexp(rsv[cu]));
         }
       }
     };
     bool done = false;
-    if constexpr (SPLIT) {
+    if constexpr (split_code<R>()) {
       if (in_block) {
         done = true;
         if (DM != 1 || rows.vec) steps(std::true_type{}, std::true_type{});
@@ -928,7 +770,7 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
     i += C_STEPS;
     // partition: the chunk's row sums in the frame ze (the largest normalised
     // frame so far), Kahan-compensated from chunk to chunk
-    if constexpr (GM != 1) {
+    {
       const int zn = max(ze, cmx);
       const float f = p2b(ze - zn + 127);
       float y = 0.f;
@@ -947,24 +789,6 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
     }
     }
   }
-  if constexpr (GM != 0) {
-    if (__any_sync(FULL, spread > SPREAD)) flag_redo(a, w.p, lane, PAIR_REDO);
-  }
-  if constexpr (GM == 1) {   // the terminal cell (L1, L2): Z of the pair, in its band's partial
-    const int q = L2 - 1 - jl;
-    if (q >= 0 && q < R) {
-      float v = 0.f;
-#pragma unroll
-      for (int c = 0; c < R; ++c) {
-        float x;
-        if constexpr (NS == 3) x = col(s.c, c);
-        else x = col(s.v[0], c);
-        v = c == q ? x : v;
-      }
-      part[0] = (float)s.e;
-      part[1] = v;
-    }
-  } else {
   // warp-combine (frame, sum) pairs, fixed shuffle tree
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -975,15 +799,14 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
     ze = m;
   }
   if (lane == 0) { part[0] = (float)ze; part[1] = zm; }
-  }
 }
 
 #ifndef SWB_LFWD_MINB
 #define SWB_LFWD_MINB 4
 #endif
-template <int NS, int R, int GM, bool SPLIT>
-__global__ void __launch_bounds__(128, SWB_LFWD_MINB) lfwd_kernel(Args a) {
-  __shared__ float4 s_edge[4][2 * fwd_block<SPLIT>()];   // per warp: the left band's records of two blocks
+template <int NS, int R>
+__global__ void __launch_bounds__(128, (R >= 8 ? 4 : SWB_LFWD_MINB)) lfwd_kernel(Args a) {
+  __shared__ float4 s_edge[4][2 * fwd_block<R>()];   // per warp: the left band's records of two blocks
   const int lane = threadIdx.x & 31;
   const LParams lp = lparams<NS>(a);
   const uint64_t deadline = gtimer() + a.spin_limit_ns;
@@ -993,12 +816,12 @@ __global__ void __launch_bounds__(128, SWB_LFWD_MINB) lfwd_kernel(Args a) {
     if (lane == 0) task = (int)atomicAdd(a.counters + 0, 1u);
     task = __shfl_sync(FULL, task, 0);
     if (task >= ntasks) break;
-    const Place w = place_of<NS, R, GM>(a, task, false);
+    const Place w = place_of<NS, R>(a, task, false);
     // a band whose last columns lie past the pair takes the variant that masks them
     float4* se = s_edge[threadIdx.x >> 5];
-    if constexpr (!SPLIT) lfwd_band<NS, R, 2, GM, false>(a, lp, w, lane, deadline, se);
-    else if ((w.band + 1) * 32 * R > w.pr.L2 || !w.pr.vec) lfwd_band<NS, R, 1, GM, true>(a, lp, w, lane, deadline, se);
-    else lfwd_band<NS, R, 0, GM, true>(a, lp, w, lane, deadline, se);
+    if constexpr (!split_code<R>()) lfwd_band<NS, R, 2>(a, lp, w, lane, deadline, se);
+    else if ((w.band + 1) * 32 * R > w.pr.L2 || !w.pr.vec) lfwd_band<NS, R, 1>(a, lp, w, lane, deadline, se);
+    else lfwd_band<NS, R, 0>(a, lp, w, lane, deadline, se);
   }
 }
 
@@ -1008,13 +831,7 @@ __global__ void __launch_bounds__(128, SWB_LFWD_MINB) lfwd_kernel(Args a) {
 
 // Z of pair w as (integer frame ze, mantissa zm): Z = zm * 2^ze, combined
 // from the band partials in a fixed order (deterministic).
-template <int R = 4, int GM = 0>
 __device__ __forceinline__ void lpair_z(const Args& a, const Place& w, int lane, int& ze, float& zm) {
-  if constexpr (GM == 1) {   // the terminal cell's band holds it
-    const float* q = a.part + 2 * (w.slot0 + max(w.pr.L2 - 1, 0) / (32 * R));
-    ze = (int)q[0];
-    zm = q[1];
-  } else {
   int ref = 0;
   float s = 0.f;
   for (int b = lane; b < w.nb; b += 32) {
@@ -1037,7 +854,6 @@ __device__ __forceinline__ void lpair_z(const Args& a, const Place& w, int lane,
   }
   ze = ref;
   zm = s;
-  }
 }
 
 // S' = log2 Z as a double-float (Sh, Sl): the integer part joins the frame
@@ -1057,34 +873,27 @@ __device__ __forceinline__ void lz_log2(int ze, float zm, float& Sh, float& Sl) 
 }
 
 // Value-only calls: one warp per pair folds the band partials into S.
-template <int NS, int R, int GM = 0>
+template <int NS, int R>
 __global__ void __launch_bounds__(128) lvalue_kernel(Args a) {
   const int lane = threadIdx.x & 31;
   const int q = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (q >= a.B) return;
   Place w;
   if (a.layout == 0) {
-    w = place_of<NS, R, GM>(a, q * a.nb, false);
+    w = place_of<NS, R>(a, q * a.nb, false);
   } else {
     const long long* pw = a.plan_pairs + (size_t)q * PLAN_PAIR_WORDS;
     w.p = q;
     w.nb = (int)pw[PW_NB];
     w.slot0 = (size_t)pw[PW_SLOT0];
-    w.pr.L1 = (int)pw[PW_L1];
-    w.pr.L2 = (int)pw[PW_L2];
   }
   if (a.pair_done[w.p] & PAIR_TIMEOUT) {   // a bounded wait of this pair expired
     if (lane == 0) a.value[w.p] = __int_as_float(0x7fc00000);
     return;
   }
-  if (GM == 1 && (w.pr.L1 == 0 || w.pr.L2 == 0)) {
-    float dgo, dge;
-    if (lane == 0) a.value[w.p] = empty_global_value<NS>(a, w.pr.L1 + w.pr.L2, dgo, dge);
-    return;
-  }
   int ze;
   float zm, Sh, Sl;
-  lpair_z<R, GM>(a, w, lane, ze, zm);
+  lpair_z(a, w, lane, ze, zm);
   lz_log2(ze, zm, Sh, Sl);
   if (lane == 0) a.value[w.p] = (Sh + Sl) * (1.f / lparams<NS>(a).k);
 }
@@ -1112,11 +921,11 @@ template <int R> struct BState {
   float ht, ob;     // the right neighbour's held t (frame hn); beta_D (beta) of column 0 (frame nb)
   int fb, nb, hn;
 };
-template <int R, int GM> __device__ __forceinline__ void bstate_zero(BState<R>& s) {
+template <int R> __device__ __forceinline__ void bstate_zero(BState<R>& s) {
 #pragma unroll
   for (int k = 0; k < R / 2; ++k) { s.b[k] = dup2(0.f); s.t[k] = dup2(0.f); }
   s.ht = 0.f; s.ob = 0.f;
-  s.fb = zero_frame<GM>(); s.nb = s.fb; s.hn = s.fb;
+  s.fb = 0; s.nb = 0; s.hn = 0;
 }
 
 // The state as a record ([group][lane][4] floats).
@@ -1171,96 +980,28 @@ __device__ __forceinline__ void bstate_load(const float* rec, int lane, BState<R
 // kernel give the same bits.
 constexpr int kSeg = 4;
 struct BandSum {
-  KSum a, b, m;   // m's compensation goes into the fold as well
+  KSum a, b, m;
   __device__ __forceinline__ void add(float x, float y, float z) {
     if (x != 0.f || y != 0.f || z != 0.f) { a.add(x); b.add(y); m.add(z); }
   }
 };
 
-// A pair's outputs from its sums: o = expected gap opens (linear gap: steps),
-// e = extensions, m = the sum of posteriors times scaled scores.  Global
-// alignments: every path has L1 + L2 gap and twice its match steps, so e comes
-// in as the sum of posteriors and the gap counts follow; a path that does not
-// start with a match at (1, 1) opens a boundary gap.
-// dS/dT is a small difference of large terms, formed in 64 bits.
-template <int NS, int GM>
-__device__ __forceinline__ void lwrite(const Args& a, const Place& w, float Sh, float Sl, double o, double e, double m,
-                                       bool bad, PParams pp) {
-  const int p = w.p;
-  if (bad) {   // a bounded wait of this pair expired
-    const float nan = __int_as_float(0x7fc00000);
-    a.value[p] = nan; a.g_open[p] = nan; a.g_T[p] = nan;
-    if (a.g_ext) a.g_ext[p] = nan;
-    return;
-  }
-  if constexpr (GM == 1) {
-    const int n = w.pr.L1 + w.pr.L2;
-    if (w.pr.L1 == 0 || w.pr.L2 == 0) {   // the terminal is a boundary cell
-      float dgo, dge;
-      a.value[p] = empty_global_value<NS>(a, n, dgo, dge);
-      a.g_open[p] = dgo;
-      if (a.g_ext) a.g_ext[p] = dge;
-      a.g_T[p] = 0.f;
-      return;
-    }
-    const double gaps = (double)n - 2.0 * e;
-    if (NS == 3) {
-      o += 1.0 - (double)ld_poll(w.pr.m);
-      e = gaps - o;
-    } else {
-      o = gaps;
-    }
-  }
-  const float inv_k = 1.f / pp.k;         // = T * ln 2
-  a.value[p] = (Sh + Sl) * inv_k;
-  a.g_open[p] = (float)o;
-  if (a.g_ext) a.g_ext[p] = NS == 3 ? (float)e : 0.f;
-  const double ln2T = 0.69314718055994530942 * (double)pp.T;
-  const double S = ((double)Sh + (double)Sl) * ln2T;
-  a.g_T[p] = (float)((S - (m * ln2T + o * (double)pp.go + (NS == 3 ? e * (double)pp.ge : 0.0))) / (double)pp.T);
-}
-
-// End of a band: its gradient partials; the pair's last band folds them in
-// band order, so the result is deterministic.
-template <int NS, int GM>
-__device__ __forceinline__ void lfinish_band(const Args& a, const Place& w, int lane, float Sh, float Sl,
-                                             const BandSum& s, PParams pp) {
-  __threadfence();   // the map's first cell (global alignments)
-  __syncwarp();
-  if (lane != 0) return;
-  float* gp = a.gpart + 4 * (w.slot0 + w.band);
-  gp[0] = s.a.s; gp[1] = s.b.s; gp[2] = s.m.s; gp[3] = -s.m.c;
-  __threadfence();
-  const unsigned done = atomicAdd(a.pair_done + w.p, 1u);
-  if ((done & ~PAIR_FLAGS) != (unsigned)w.nb - 1) return;
-  __threadfence();
-  double o = 0.0, e = 0.0, m = 0.0;
-  for (int b = 0; b < w.nb; ++b) {
-    const float* q = a.gpart + 4 * (w.slot0 + b);
-    o += (double)ld_poll(q);
-    e += (double)ld_poll(q + 1);
-    m += (double)ld_poll(q + 2) + (double)ld_poll(q + 3);
-  }
-  lwrite<NS, GM>(a, w, Sh, Sl, o, e, m, (done & PAIR_TIMEOUT) != 0, pp);
-}
-
 // End of a segment: its gradient partials; the pair's last segment folds them
 // (lane l the bands l, l + 32, ...; then the bands in order).
-template <int NS, int GM>
+template <int NS>
 __device__ __forceinline__ void lfinish_seg(const Args& a, const Place& w, int lane, int seg, float Sh, float Sl,
                                             float g0, float g1, float ps, PParams pp) {
-  __threadfence();   // the map's first cell (global alignments)
-  __syncwarp();
+  const int p = w.p;
   unsigned done = 0;
   if (lane == 0) {
     reinterpret_cast<float4*>(a.spart)[(w.slot0 + w.band) * a.nseg + seg] = make_float4(g0, g1, ps, 0.f);
     __threadfence();
-    done = atomicAdd(a.pair_done + w.p, 1u);
+    done = atomicAdd(a.pair_done + p, 1u);
   }
   done = __shfl_sync(FULL, done, 0);
-  if ((done & ~PAIR_FLAGS) != (unsigned)(w.nb * a.nseg) - 1) return;
+  if ((done & ~PAIR_TIMEOUT) != (unsigned)(w.nb * a.nseg) - 1) return;
   __threadfence();
-  double o = 0.0, e = 0.0, m = 0.0;
+  float o = 0.f, e = 0.f, m = 0.f;
   for (int b0 = 0; b0 < w.nb; b0 += 32) {
     BandSum s;
     if (b0 + lane < w.nb) {
@@ -1268,59 +1009,60 @@ __device__ __forceinline__ void lfinish_seg(const Args& a, const Place& w, int l
       for (int q = a.nseg - 1; q >= 0; --q) s.add(ld_poll(x + 4 * q), ld_poll(x + 4 * q + 1), ld_poll(x + 4 * q + 2));
     }
     for (int b = 0; b < min(32, w.nb - b0); ++b) {
-      o += (double)__shfl_sync(FULL, s.a.s, b);
-      e += (double)__shfl_sync(FULL, s.b.s, b);
-      m += (double)__shfl_sync(FULL, s.m.s, b) + (double)(-__shfl_sync(FULL, s.m.c, b));
+      o += __shfl_sync(FULL, s.a.s, b);
+      e += __shfl_sync(FULL, s.b.s, b);
+      m += __shfl_sync(FULL, s.m.s, b);
     }
   }
-  if (lane == 0) lwrite<NS, GM>(a, w, Sh, Sl, o, e, m, (done & PAIR_TIMEOUT) != 0, pp);
+  if (lane != 0) return;
+  if (done & PAIR_TIMEOUT) {   // a bounded wait of this pair expired
+    const float nan = __int_as_float(0x7fc00000);
+    a.value[p] = nan; a.g_open[p] = nan; a.g_T[p] = nan;
+    if (a.g_ext) a.g_ext[p] = nan;
+    return;
+  }
+  const float inv_k = 1.f / pp.k;         // = T * ln 2
+  const float S = (Sh + Sl) * inv_k, match = m * inv_k;
+  a.value[p] = S;
+  a.g_open[p] = o;
+  if (a.g_ext) a.g_ext[p] = NS == 3 ? e : 0.f;
+  a.g_T[p] = NS == 3 ? (S - (match + (o * pp.go + e * pp.ge))) / pp.T : (S - (match + o * pp.go)) / pp.T;
 }
 
 // One row of the outside recursion for one lane: (rb, rt, rn) are the right
 // lane's beta_D (linear: beta) of its column 0, its t and its normalised
-// frame; live: the row is inside the pair (global: it is the last row; term:
-// the terminal's column in this lane, or -1).  Returns, in the frame `ft`: vm =
+// frame; live: the row is inside the pair.  Returns, in the frame `ft`: vm =
 // beta_M (beta), sr = beta_I below + beta_D right and br = beta_D right per
 // column.  The state moves on with bfinish.
-template <int NS, int R, int DM, int GM>
-__device__ __forceinline__ void bcells(const BState<R>& s, float rb, int rn, bool live, int term, float gO, float gE,
+template <int NS, int R, int DM>
+__device__ __forceinline__ void bcells(const BState<R>& s, float rb, int rn, bool live, float gO, float gE,
                                        float gX, int nlive, bool hd, int& ft, float& fB,
                                        float2 (&vm)[R / 2], float2 (&vi)[R / 2], float2 (&sr)[R / 2],
                                        float2 (&br)[R / 2], float& vd0, float& mx) {
   constexpr int H = R / 2;
   // frames: the row is computed in ft >= every input's normalised frame
   ft = max(max(s.nb, rn), s.hn);
-  if constexpr (GM != 0) ft = max(ft - headroom<GM>(), s.fb - 127);
-  if (GM == 1 && live && term >= 0) ft = max(ft, 0);
   const int q = 127 - ft;
   fB = p2b(s.fb + q);
   const float fT = p2b(s.nb + q), fR = p2b(rn + q), fH = p2b(s.hn + q);
-  const float one = live && (GM != 1 || term >= 0) ? p2b(q) : 0.f;
-  // base: the diagonal successor's t, plus 1 where the alignment may end;
-  // nom: the same without M's end (Saigo-Vert: only M ends)
-  float2 base[H], nom[H];
+  const float one = live ? p2b(q) : 0.f;
+  float2 base[H];
 #pragma unroll
-  for (int k = 0; k < H; ++k) {
+  for (int k = 0; k < H; ++k) {   // 1 plus the diagonal successor's t
     float2 oc = dup2(one);
-    if constexpr (GM == 1) oc = make_float2(k == term ? one : 0.f, k + H == term ? one : 0.f);
-    else if (masks<DM>(hd)) oc = make_float2(k < nlive ? one : 0.f, k + H < nlive ? one : 0.f);
-    const float2 f = k == H - 1 ? make_float2(fT, fH) : dup2(fT);
-    const float2 t = k == H - 1 ? make_float2(s.t[0].y, s.ht) : s.t[k < H - 1 ? k + 1 : 0];
-    base[k] = fma2(f, t, oc);
-    nom[k] = GM == 2 ? mul2(f, t) : base[k];
+    if (masks<DM>(hd)) oc = make_float2(k < nlive ? one : 0.f, k + H < nlive ? one : 0.f);
+    base[k] = k == H - 1 ? fma2(make_float2(fT, fH), make_float2(s.t[0].y, s.ht), oc)
+                         : fma2(dup2(fT), s.t[k < H - 1 ? k + 1 : 0], oc);
   }
   const float b0 = fR * rb;   // right successor's beta_D (beta) of the last column
   float2 v[H];                // beta_D (beta) per column
-  const float2 gEb = dup2(gE * fB), gOb = dup2(gO * fB);
   if constexpr (NS == 3) {
-    float2 x[H];              // global: D also goes on to I below
+    col(v, R - 1) = fmaf(gE, b0, col(base, R - 1));
 #pragma unroll
-    for (int k = 0; k < H; ++k) x[k] = GM == 1 ? fma2(gOb, s.b[k], nom[k]) : nom[k];
-    col(v, R - 1) = fmaf(gE, b0, col(x, R - 1));
-#pragma unroll
-    for (int c = R - 2; c >= 0; --c) col(v, c) = fmaf(gE, col(v, c + 1), col(x, c));
+    for (int c = R - 2; c >= 0; --c) col(v, c) = fmaf(gE, col(v, c + 1), col(base, c));
   } else {
     float2 x[H];
+    const float2 gOb = dup2(gO * fB);
 #pragma unroll
     for (int k = 0; k < H; ++k) x[k] = fma2(gOb, s.b[k], base[k]);
     col(v, R - 1) = fmaf(gO, b0, col(x, R - 1));
@@ -1335,11 +1077,11 @@ __device__ __forceinline__ void bcells(const BState<R>& s, float rb, int rn, boo
   }
   float2 m[H];
   if constexpr (NS == 3) {
+    const float2 gEb = dup2(gE * fB);
 #pragma unroll
     for (int k = 0; k < H; ++k) {
       vm[k] = fma2(dup2(gO), sr[k], base[k]);
-      // I goes on to I below and, but for the local model, to D on the right
-      vi[k] = fma2(gEb, s.b[k], GM ? fma2(dup2(gO), br[k], nom[k]) : base[k]);
+      vi[k] = fma2(gEb, s.b[k], base[k]);
       m[k] = fma2(dup2(gX), sr[k], base[k]);   // >= beta_M, beta_I, beta_D
     }
   } else {
@@ -1357,12 +1099,12 @@ __device__ __forceinline__ void bcells(const BState<R>& s, float rb, int rn, boo
 }
 
 // The state after the row: t = E beta_M in the row's normalised frame.
-template <int R, int GM>
+template <int R>
 __device__ __forceinline__ void bfinish(BState<R>& s, int ft, float mx, const float2 (&vm)[R / 2],
                                         const float2 (&vi)[R / 2], float vd0, const float2 (&E)[R / 2],
                                         float rt, int rn) {
   constexpr int H = R / 2;
-  const int nn = floor_frame<GM>(ft - 126 + sexp(mx));
+  const int nn = max(ft - 126 + sexp(mx), 0);
   const float bs = p2b(ft - nn + 127);
 #pragma unroll
   for (int k = 0; k < H; ++k) {
@@ -1389,11 +1131,8 @@ __device__ __forceinline__ void bfinish(BState<R>& s, int ft, float mx, const fl
 // flows it drops are among those bounded.  The right band's records are
 // resolved first, so the decision does not depend on timing.  zlog: log2 of Z
 // less SWB_LQUIET; pb: lane u < C the record of backward step u. ----
-// Global alignments: the only fresh weight is the terminal's, so the 1 counts
-// in its chunk alone (own).
-template <int R, int GM>
-__device__ __forceinline__ bool lquiet(const BState<R>& s, int ckm, const float (&pb)[3], int lane, int zlog,
-                                       bool own) {
+template <int R>
+__device__ __forceinline__ bool lquiet(const BState<R>& s, int ckm, const float (&pb)[3], int lane, int zlog) {
   int inl = s.hn + fexp(s.ht);
   float mb = 0.f, mt = 0.f;   // largest beta and t of the row below
 #pragma unroll
@@ -1403,7 +1142,7 @@ __device__ __forceinline__ bool lquiet(const BState<R>& s, int ckm, const float 
   }
   inl = max(inl, max(s.fb + fexp(mb), s.nb + fexp(mt)));
   if (lane < C_STEPS) inl = max(inl, __float_as_int(pb[2]) + fexp(fmaxf(pb[0], pb[1])));
-  return __all_sync(FULL, ckm + 11 + (GM != 1 || own ? max(inl, 0) : inl) < zlog);
+  return __all_sync(FULL, ckm + 11 + max(inl, 0) < zlog);
 }
 // ---- quiet run.  After a quiet chunk only lane 31's held t (pt, pn) and the
 // right band's records enter the chunks above, so one round of loads decides
@@ -1412,11 +1151,9 @@ __device__ __forceinline__ bool lquiet(const BState<R>& s, int ckm, const float 
 // below (lane l - 1's; lane 0: the held t).  A record not written yet ends
 // the run; that chunk is then decided by lquiet from the same values, so
 // results do not depend on timing.  Returns how many chunks from kn down (not
-// below k_lo) are quiet; r1, rn: the lane's record's t and frame.  Chunk `own`
-// (a global alignment's terminal) ends it too. ----
-template <int GM>
+// below k_lo) are quiet; r1, rn: the lane's record's t and frame. ----
 __device__ __forceinline__ int lquiet_run(const float* pin, size_t Lm, int L1, const float* ckmax, int kn, int k_lo,
-                                          int lane, float pt, int pn, int zlog, int own, float& r1, int& rn) {
+                                          int lane, float pt, int pn, int zlog, float& r1, int& rn) {
   constexpr int RUN = 32 / C_STEPS;
   const int j = lane / C_STEPS, u = lane - j * C_STEPS;
   const int kq = kn - j;
@@ -1424,7 +1161,7 @@ __device__ __forceinline__ int lquiet_run(const float* pin, size_t Lm, int L1, c
   int cm = -(1 << 30);
   bool written = true;
   r1 = 0.f;
-  rn = zero_frame<GM>();
+  rn = 0;
   if (kq >= k_lo) {
     const int ir = kq * C_STEPS + C_STEPS - 1 - u - 30;
     if (pin && ir >= 1 && ir <= L1) {
@@ -1432,7 +1169,7 @@ __device__ __forceinline__ int lquiet_run(const float* pin, size_t Lm, int L1, c
       r1 = ld_poll(pin + 1 * (Lm + 1) + ir);
       const float r2 = ld_poll(pin + 2 * (Lm + 1) + ir);
       written = !is_sentinel(r0) && !is_sentinel(r1) && !is_sentinel(r2);
-      rn = __float_as_int(r2) - frame_bias<GM>();
+      rn = __float_as_int(r2);
     }
     cm = __float_as_int(ckmax[kq]);
   }
@@ -1441,7 +1178,7 @@ __device__ __forceinline__ int lquiet_run(const float* pin, size_t Lm, int L1, c
   const bool wu = __shfl_up_sync(FULL, (int)written, 1) != 0;
   const int lgb = lane == 0 ? pn + fexp(pt) : lgu;
   const bool wb = lane == 0 || wu;
-  const bool q = kq >= k_lo && (GM != 1 || kq != own) && written && wb && cm + 11 + (GM == 1 ? max(lg, lgb) : max(max(lg, lgb), 0)) < zlog;
+  const bool q = kq >= k_lo && written && wb && cm + 11 + max(max(lg, lgb), 0) < zlog;
   const unsigned ball = __ballot_sync(FULL, q);
   constexpr unsigned grp = (1u << C_STEPS) - 1u;
   int n = 0;
@@ -1449,13 +1186,12 @@ __device__ __forceinline__ int lquiet_run(const float* pin, size_t Lm, int L1, c
   return n;
 }
 // Zero records to the left band for the rows of chunk kq (lane 0's).
-template <int GM>
 __device__ __forceinline__ void zero_push(float* pout, size_t Lm, int L1, int kq, int lane) {
   const int i = kq * C_STEPS + lane + 1;
   if (pout && lane < C_STEPS && i <= L1) {
     pout[0 * (Lm + 1) + i] = 0.f;
     pout[1 * (Lm + 1) + i] = 0.f;
-    pout[2 * (Lm + 1) + i] = __int_as_float(zero_frame<GM>() + frame_bias<GM>());
+    pout[2 * (Lm + 1) + i] = 0.f;
   }
 }
 
@@ -1475,12 +1211,12 @@ __device__ __forceinline__ void zero_push(float* pout, size_t Lm, int L1, int kq
 // SEG: one segment of the band, chunks [k_lo, k_hi), starting from the state
 // the outside sweep (lbeta_band) kept for it; every record it reads has been
 // written by then, and it passes none on.
-template <int NS, int R, bool SPARSE, bool SEG, int GM>
+template <int NS, int R, bool SPARSE, int DM, bool SEG = false>
 __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int lane, float* sm,
-                          uint64_t deadline, int seg) {
+                          uint64_t deadline, int seg = 0) {
   using LD = LDims<NS, R>;
-  using LE = LEdge<NS, GM>;
-  constexpr int H = R / 2, DM = 2;
+  using LE = LEdge<NS>;
+  constexpr int H = R / 2;
   constexpr int CKF = LD::CKF, LREC = LD::LREC, FW = LD::FW, NPF = 3;
   const Pair& pr = w.pr;
   const int L1 = pr.L1, L2 = pr.L2;
@@ -1488,15 +1224,14 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
   const int col0 = band * 32 * R;
   int ze;
   float zm, Sh, Sl;
-  if (GM != 0 && redo_set(a, w.p)) return;   // run again in the log domain
-  lpair_z<R, GM>(a, w, lane, ze, zm);
+  lpair_z(a, w, lane, ze, zm);
   lz_log2(ze, zm, Sh, Sl);
   const PParams pp{lp.go, lp.ge, lp.T, lp.k};
   const int nch = band_chunks(L1);
   const int k_lo = SEG ? seg * kSeg : 0, k_hi = SEG ? min(k_lo + kSeg, nch) : nch;
   if (!(L1 > 0 && col0 < L2) || k_lo >= k_hi) {
-    if constexpr (SEG) lfinish_seg<NS, GM>(a, w, lane, seg, Sh, Sl, 0.f, 0.f, 0.f, pp);
-    else lfinish_band<NS, GM>(a, w, lane, Sh, Sl, BandSum{}, pp);
+    if constexpr (SEG) lfinish_seg<NS>(a, w, lane, seg, Sh, Sl, 0.f, 0.f, 0.f, pp);
+    else finish_pair_p<NS>(a, w, lane, Sh, Sl, 0.f, 0.f, 0.f, pp);
     return;
   }
   const float invZ = 1.f / zm;
@@ -1543,8 +1278,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
     const int i = kc * C_STEPS + C_STEPS - 1 - lane - 30;   // lane 31's row at backward step lane
     const bool ok = pin && lane < C_STEPS && i >= 1 && i <= L1;
 #pragma unroll
-    for (int f = 0; f < NPF; ++f) dst[f] = ld_poll_if(pin + f * (Lm + 1) + i, ok);
-    if (GM == 1 && !ok) dst[2] = __int_as_float(zero_frame<GM>() + frame_bias<GM>());
+    for (int f = 0; f < NPF; ++f) dst[f] = ok ? ld_poll(pin + f * (Lm + 1) + i) : 0.f;
   };
   auto load_sb = [&](int kc) {
     const int i0 = kc * C_STEPS - lane + 1;
@@ -1553,6 +1287,12 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
 #pragma unroll
       for (int u = 0; u < C_STEPS; ++u) {
         rows.template fetch<true>(src, nsb[u]);
+        src += rows.ld;
+      }
+    } else if (split_code<R>() && rows.inside(kc)) {
+#pragma unroll
+      for (int u = 0; u < C_STEPS; ++u) {
+        rows.template fetch<false>(src, nsb[u]);
         src += rows.ld;
       }
     } else {
@@ -1572,18 +1312,12 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
 
   BState<R> bs;
   if constexpr (SEG) bstate_load<R>(a.bck + ((w.slot0 + band) * a.nseg + seg) * BDims<R>::BREC, lane, bs);
-  else bstate_zero<R, GM>(bs);
-  // global: the terminal's column in this lane, and the chunks with row L1 of its lanes
-  const int term = GM == 1 && L2 - 1 - jl >= 0 && L2 - 1 - jl < R ? L2 - 1 - jl : -1;
-  const int tl = (L2 - 1 - col0) / R;   // the terminal's lane (32 or more: in another band)
-  const int ownc = GM == 1 && tl < 32 ? (L1 - 1 + tl) / C_STEPS : -1;
-  [[maybe_unused]] bool lost = false;
+  else bstate_zero(bs);
   BandSum gsum;
   float cA = 0.f, cB = 0.f;   // the segment's plain sums
   float2 cS = dup2(0.f);
-  [[maybe_unused]] float2 cP = dup2(0.f);   // global: posteriors
   auto flush = [&]() {        // at the end of a segment
-    float v0 = cA, v1 = GM == 1 ? cP.x + cP.y : cB, v2 = cS.x + cS.y;
+    float v0 = cA, v1 = cB, v2 = cS.x + cS.y;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       v0 += __shfl_xor_sync(FULL, v0, o);
@@ -1591,7 +1325,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
       v2 += __shfl_xor_sync(FULL, v2, o);
     }
     gsum.add(v0, v1, v2);
-    cA = 0.f; cB = 0.f; cS = dup2(0.f); cP = dup2(0.f);
+    cA = 0.f; cB = 0.f; cS = dup2(0.f);
   };
 
   // log2 of Z is at least zlog; a chunk is quiet (below) when every cell's
@@ -1615,8 +1349,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
       }
       __syncwarp();
     }
-    pbc[2] = __int_as_float(__float_as_int(pbc[2]) - frame_bias<GM>());
-    const bool quiet = lquiet<R, GM>(bs, ckm, pbc, lane, zlog, kc == ownc);
+    const bool quiet = lquiet<R>(bs, ckm, pbc, lane, zlog);
 #ifdef SWB_COUNT_QUIET   // measurement builds: quiet and computed chunks in header words 8, 9
     if (lane == 0) atomicAdd(a.counters + (quiet ? 8 : 9), 1u);
 #endif
@@ -1632,7 +1365,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
             if (i >= 1 && i <= L1) store_row<R>(pr, i, jl, z);
           }
         }
-        zero_push<GM>(pout, Lm, L1, kq, lane);
+        zero_push(pout, Lm, L1, kq, lane);
       };
       zero_chunk(kc);
       // the row above the chunk sees zero beta; lane 31 keeps the right
@@ -1643,7 +1376,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
       while (kn >= k_lo) {
         float r1;
         int rn;
-        const int n = lquiet_run<GM>(pin, Lm, L1, ckmax, kn, k_lo, lane, pt, pn, zlog, ownc, r1, rn);
+        const int n = lquiet_run(pin, Lm, L1, ckmax, kn, k_lo, lane, pt, pn, zlog, r1, rn);
         for (int m = 0; m < n; ++m) zero_chunk(kn - m);
         if (n > 0) {   // lane 31's held t: the record of its top row of the last zeroed chunk
           pt = __shfl_sync(FULL, r1, n * C_STEPS - 1);
@@ -1653,9 +1386,9 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
         if (n < 32 / C_STEPS) break;
       }
       if (!SEG && kc / kSeg != (kn + (kn < 0 ? -kSeg + 1 : 0)) / kSeg) flush();   // the run left the segment
-      bstate_zero<R, GM>(bs);
+      bstate_zero(bs);
       bs.ht = lane == 31 ? pt : 0.f;
-      bs.hn = lane == 31 ? pn : zero_frame<GM>();
+      bs.hn = lane == 31 ? pn : 0;
       if (kn >= k_lo) {   // inputs of the next chunk to run
         load_ck(kn);
         ebr = get_edge(kn);
@@ -1670,8 +1403,8 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
     float2 d[H];
 #pragma unroll
     for (int j = 0; j < H; ++j) d[j] = dup2(0.f);
-    lck_restore<NS, R, DM, GM>(stg_ck, lane, st, gO, gE, nlive, hd, d);
-    if (lane < C_STEPS) s_eb[lane] = ein || GM != 1 ? LE::open(ebr) : LE::column0(lp, t0 + lane + 1);
+    lck_restore<NS, R, DM>(stg_ck, lane, st, gO, gE, nlive, hd, d);
+    if (lane < C_STEPS) s_eb[lane] = LE::open(ebr);
     __syncwarp();   // the staged checkpoint is read before the next chunk's copy is issued
     if constexpr (SPARSE) {
       if (kc % KC != 0) {
@@ -1691,7 +1424,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
         }
 #pragma unroll 1
         for (int ka = k0; ka < kc; ++ka) {
-          float4 er = ein || GM != 1 ? LE::open(get_edge(ka)) : LE::column0(lp, ka * C_STEPS + lane + 1);
+          float4 er = LE::open(get_edge(ka));
 #pragma unroll 1
           for (int u0 = 0; u0 < C_STEPS; u0 += PF)
 #pragma unroll
@@ -1707,20 +1440,22 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
             const float e2 = __shfl_sync(FULL, er.z, cu), e3 = __shfl_sync(FULL, er.w, cu);
             if (lane == 0) { xd = e0; xc = e1; xe = __float_as_int(e2); xn = __float_as_int(e3); }
             float2 xs[H], E[H];
-            lemit<R, DM, GM>(ab[u], k, nlive, hd, xs, E);
+            lemit<R, DM>(ab[u], k, nlive, hd, xs, E);
             rows.load(src, i + PF, ab[u]);
             src += rows.ld;
             float rs;
-            if (act) lcells<NS, R, DM, GM>(st, xd, xc, xe, xn, E, gO, gE, nlive, hd, d, rs);
+            if (act) lcells<NS, R, DM>(st, xd, xc, xe, xn, E, gO, gE, nlive, hd, d, rs);
             ++i;
           }
         }
       }
     }
+    auto recompute = [&](auto inside_c) {
+      constexpr bool IN = decltype(inside_c)::value;
 #pragma unroll
     for (int cu = 0; cu < C_STEPS; ++cu) {
       const int i = t0 + cu - lane + 1;
-      const bool act = (unsigned)(i - 1) < (unsigned)L1;
+      const bool act = IN || (unsigned)(i - 1) < (unsigned)L1;
       float xd = 0.f;
       if constexpr (NS == 3) xd = __shfl_up_sync(FULL, st.od, 1);
       float xc = __shfl_up_sync(FULL, st.oc, 1);
@@ -1731,10 +1466,9 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
         xd = e4.x; xc = e4.y; xe = __float_as_int(e4.z); xn = __float_as_int(e4.w);
       }
       float2 xs[H], E[H];
-      lemit<R, DM, GM>(nsb[cu], k, nlive, hd, xs, E);
-      lblank<R>(act, xs, E);
+      lemit<R, DM>(nsb[cu], k, nlive, hd, xs, E);
       float rs;
-      if (act) lcells<NS, R, DM, GM>(st, xd, xc, xe, xn, E, gO, gE, nlive, hd, d, rs);
+      if (act) lcells<NS, R, DM>(st, xd, xc, xe, xn, E, gO, gE, nlive, hd, d, rs);
       float* ent = sm + (size_t)cu * FW * 32;
       // field g's R columns as pairs: [g][quad][lane][4] (2 columns: [g][lane][2])
       auto put = [&](int g, const float2 (&x)[H]) {
@@ -1751,15 +1485,12 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
       if constexpr (NS == 3) put(1, st.v[1]);
       put(LD::NF - 2, d);
       put(LD::NF - 1, xs);
-      if constexpr (GM == 0) {
-        ent[LD::NF * R * 32 + lane] = __int_as_float(st.e);
-      } else {   // the raw frame and the exponent of the row's sum
-        float all;
-        if constexpr (NS == 3) all = sum2(st.c);
-        else all = sum2(st.v[0]);
-        ent[LD::NF * R * 32 + lane] = __int_as_float((int)((unsigned)st.e << 8) | sexp(all));
-      }
+      ent[LD::NF * R * 32 + lane] = __int_as_float(st.e);
     }
+    };
+    const bool in = kc >= 32 / C_STEPS && (kc + 1) * C_STEPS <= L1;   // every lane on a row of the pair
+    if (split_code<R>() && in) recompute(std::true_type{});
+    else recompute(std::false_type{});
     if (kc > k_lo) {   // prefetch the next chunk's inputs while the outside recursion runs
       load_ck(kc - 1);
       ebr = get_edge(kc - 1);
@@ -1796,8 +1527,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
           }
         }
       };
-      const int ew = __float_as_int(ent[LD::NF * R * 32 + lane]);
-      const int ea = GM == 0 ? ew : ew >> 8;
+      const int ea = __float_as_int(ent[LD::NF * R * 32 + lane]);
       float2 fm[H], fd[H], xs[H], E[H];
       get(0, fm);
       get(LD::NF - 2, fd);
@@ -1807,83 +1537,36 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
       int ft;
       float fB, vd0, mx;
       float2 vm[H], vi[H], sr[H], br[H], P[H];
-      bcells<NS, R, DM, GM>(bs, rb, rn, GM == 1 ? i == L1 : act, term, gO, gE, gX, nlive, hd, ft, fB, vm, vi, sr, br, vd0, mx);
+      bcells<NS, R, DM>(bs, rb, rn, act, gO, gE, gX, nlive, hd, ft, fB, vm, vi, sr, br, vd0, mx);
       // raw alpha (frame ea) times raw beta (frame ft), over Z
-      // (with headroom the product's exponent may leave the range of one
-      // factor: half goes to each side)
-      const int ax = ea + ft - ze;
-      const float asc = p2any(GM ? ax >> 1 : ax) * invZ, bsc = GM ? p2any(ax - (ax >> 1)) : 1.f;
-      if constexpr (GM != 0) {   // a beta near the end of the range where alpha makes it count
-        const int bx = 127 - sexp(min2<DM>(vm, nlive, hd));
-        lost = lost || (act && (DM == 0 || nlive > 0) && bx > SPREAD && ea - 126 + (ew & 255) + ft - 81 > zlog + SWB_LQUIET);
-      }
+      const float asc = p2any(ea + ft - ze) * invZ;
       float2 so = dup2(0.f);
 #pragma unroll
       for (int j = 0; j < H; ++j) {
-        const float2 q = mul2(NS == 3 ? fm[j] : fd[j], dup2(asc));
-        const float2 p = mul2(q, GM ? mul2(vm[j], dup2(bsc)) : vm[j]);
+        const float2 p = mul2(mul2(NS == 3 ? fm[j] : fd[j], dup2(asc)), vm[j]);
         P[j] = make_float2(fminf(p.x, 1.f), fminf(p.y, 1.f));   // a posterior: rounding may pass 1
-        if constexpr (GM == 0) so = fma2(fm[j], sr[j], so);
-        else if constexpr (NS == 3) so = fma2(q, sr[j], so);   // scaled first: raw values fill the range here
-        // (an excluded cell, score -inf, has posterior 0)
-        cS = fma2(P[j], GM == 0 ? xs[j] : make_float2(fmaxf(xs[j].x, NEG), fmaxf(xs[j].y, NEG)), cS);
-        if constexpr (GM == 1) cP = add2(cP, P[j]);
+        so = fma2(fm[j], sr[j], so);
+        cS = fma2(P[j], xs[j], cS);
       }
-      if constexpr (GM != 0 && NS == 3) {
-        // opens: M to I and D, I to D, and in global alignments D to I (for
-        // lane 0 of the first band from column 0 too)
-        float2 fi[H];
-        get(1, fi);
-        float2 sdi = dup2(0.f);
-#pragma unroll
-        for (int j = 0; j < H; ++j) {
-          so = fma2(mul2(fi[j], dup2(asc)), br[j], so);
-          if constexpr (GM == 1) sdi = fma2(mul2(fd[j], dup2(asc)), bs.b[j], sdi);
-        }
-        float o = fmaf(sdi.x + sdi.y, fB, so.x + so.y) * bsc * gO;
-        if constexpr (GM == 1) {
-          if (band == 0 && lane == 0 && act) {
-            const float4 e4 = s_eb[C_STEPS - 1 - cu];
-            const int x = __float_as_int(e4.z) + ft - ze;
-            o = fmaf(e4.x * (p2any(x >> 1) * invZ), vd0 * p2any(x - (x >> 1)), o);
-          }
-        }
-        if (GM == 2 || act) cA += o;
-      } else if constexpr (GM != 1) {
-        cA = fmaf((so.x + so.y) * asc, gO, cA);
-      }
-      if constexpr (NS == 3 && GM != 1) {
+      cA = fmaf((so.x + so.y) * asc, gO, cA);
+      if constexpr (NS == 3) {
         float2 fi[H];
         get(1, fi);
         float2 sxi = dup2(0.f), sxd = dup2(0.f);
 #pragma unroll
         for (int j = 0; j < H; ++j) {
-          sxi = fma2(GM ? mul2(fi[j], dup2(asc)) : fi[j], bs.b[j], sxi);
-          sxd = fma2(GM ? mul2(fd[j], dup2(asc)) : fd[j], br[j], sxd);
+          sxi = fma2(fi[j], bs.b[j], sxi);
+          sxd = fma2(fd[j], br[j], sxd);
         }
-        const float x = fmaf(sxi.x + sxi.y, fB, sxd.x + sxd.y);
-        cB = fmaf(x * (GM ? bsc : asc), gE, cB);
+        cB = fmaf(fmaf(sxi.x + sxi.y, fB, sxd.x + sxd.y) * asc, gE, cB);
       }
-      bfinish<R, GM>(bs, ft, mx, vm, vi, vd0, E, rt, rn);
-      if constexpr (GM == 1 && NS == 3) {
-        if (i == 1) {   // the D's of row 0 open into I of row 1
-          LState<NS, R> z;
-          float2 d0[H], o = dup2(0.f);
-#pragma unroll
-          for (int j = 0; j < H; ++j) d0[j] = dup2(0.f);
-          lstate_row0<NS, R, DM>(z, d0, lp, jl, nlive, hd);
-          const int x = z.e + bs.fb - ze;
-#pragma unroll
-          for (int j = 0; j < H; ++j) o = fma2(mul2(d0[j], dup2(p2any(x >> 1) * invZ)), mul2(bs.b[j], dup2(p2any(x - (x >> 1)))), o);
-          cA = fmaf(o.x + o.y, gO, cA);
-        }
-      }
+      bfinish<R>(bs, ft, mx, vm, vi, vd0, E, rt, rn);
       if (act) {
         store_pairs<R>(mrow, jl, pr, P);
         if (lane == 0 && pout) {
           pout[0 * (Lm + 1) + i] = bs.ob;
           pout[1 * (Lm + 1) + i] = bs.t[0].x;
-          pout[2 * (Lm + 1) + i] = __int_as_float(bs.nb + frame_bias<GM>());
+          pout[2 * (Lm + 1) + i] = __int_as_float(bs.nb);
         }
       }
       --i;
@@ -1894,14 +1577,11 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
     if (!SEG && kc % kSeg == 0) flush();
     __syncwarp();
   }
-  if constexpr (GM != 0) {
-    if (__any_sync(FULL, lost)) flag_redo(a, w.p, lane, PAIR_LOST);
-  }
   if constexpr (SEG) {
     flush();
-    lfinish_seg<NS, GM>(a, w, lane, seg, Sh, Sl, gsum.a.s, gsum.b.s, gsum.m.s, pp);
+    lfinish_seg<NS>(a, w, lane, seg, Sh, Sl, gsum.a.s, gsum.b.s, gsum.m.s, pp);
   } else {
-    lfinish_band<NS, GM>(a, w, lane, Sh, Sl, gsum, pp);
+    finish_pair_p<NS>(a, w, lane, Sh, Sl, gsum.a.s, gsum.b.s, gsum.m.s, pp);
   }
 }
 
@@ -1917,11 +1597,11 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
 // independently of the others (lseg_kernel).  The decisions, the states and
 // the sums are the adjoint's, so the results are its results bit for bit.
 
-template <int NS, int R, int DM, int GM>
+template <int NS, int R, int DM>
 __device__ void lbeta_band(const Args& a, const LParams& lp, const Place& w, int lane, uint64_t deadline,
                            float4* spush) {
   using LD = LDims<NS, R>;
-  constexpr int H = R / 2, AH = fwd_ahead<true>(), SUB = AH / C_STEPS, NPF = 3;
+  constexpr int H = R / 2, AH = fwd_ahead<R>(), SUB = AH / C_STEPS, NPF = 3;
   const Pair& pr = w.pr;
   const int L1 = pr.L1, L2 = pr.L2;
   const int band = w.band;
@@ -1929,8 +1609,7 @@ __device__ void lbeta_band(const Args& a, const LParams& lp, const Place& w, int
   if (!(L1 > 0 && col0 < L2)) return;
   int ze;
   float zm;
-  if (GM != 0 && redo_set(a, w.p)) return;   // run again in the log domain
-  lpair_z<R, GM>(a, w, lane, ze, zm);
+  lpair_z(a, w, lane, ze, zm);
   const int zlog = ze + fexp(zm) - 1 - SWB_LQUIET;
   const int jl = col0 + lane * R;
   const int nlive = min(max(L2 - jl, 0), R);
@@ -1945,25 +1624,21 @@ __device__ void lbeta_band(const Args& a, const LParams& lp, const Place& w, int
   float* rec = a.bck + (w.slot0 + band) * (size_t)a.nseg * BDims<R>::BREC;
 
   BState<R> bs;
-  bstate_zero<R, GM>(bs);
-  const int term = GM == 1 && L2 - 1 - jl >= 0 && L2 - 1 - jl < R ? L2 - 1 - jl : -1;
-  const int tl = (L2 - 1 - col0) / R;
-  const int ownc = GM == 1 && tl < 32 ? (L1 - 1 + tl) / C_STEPS : -1;
+  bstate_zero(bs);
   auto get_push = [&](int kc) {   // lane u < C: the right band's record lane 31 needs at backward step u
     const int i = kc * C_STEPS + C_STEPS - 1 - lane - 30;
     FieldVec<NPF> x;
     const bool ok = pin && lane < C_STEPS && i >= 1 && i <= L1;
 #pragma unroll
     for (int f = 0; f < NPF; ++f) x.v[f] = ld_poll_if(pin + f * (Lm + 1) + i, ok);
-    if (GM == 1 && !ok) x.v[2] = __int_as_float(zero_frame<GM>() + frame_bias<GM>());
     return x;
   };
   // the state at the top of a segment whose chunks above were quiet
   auto store_zero = [&](int kq, float pt, int pn) {
     BState<R> z;
-    bstate_zero<R, GM>(z);
+    bstate_zero(z);
     z.ht = lane == 31 ? pt : 0.f;
-    z.hn = lane == 31 ? pn : zero_frame<GM>();
+    z.hn = lane == 31 ? pn : 0;
     bstate_store<R>(rec + (size_t)(kq / kSeg) * BDims<R>::BREC, lane, z);
   };
   Rows<R> rows;
@@ -2001,28 +1676,27 @@ __device__ void lbeta_band(const Args& a, const LParams& lp, const Place& w, int
       __syncwarp();
     }
     if (kc == nch - 1 || (kc + 1) % kSeg == 0) bstate_store<R>(rec + (size_t)(kc / kSeg) * BDims<R>::BREC, lane, bs);
-    ea.v[2] = __int_as_float(__float_as_int(ea.v[2]) - frame_bias<GM>());
-    if (lquiet<R, GM>(bs, ckm, ea.v, lane, zlog, kc == ownc)) {
-      zero_push<GM>(pout, Lm, L1, kc, lane);
+    if (lquiet<R>(bs, ckm, ea.v, lane, zlog)) {
+      zero_push(pout, Lm, L1, kc, lane);
       float pt = __shfl_sync(FULL, ea.v[1], C_STEPS - 1);
       int pn = __shfl_sync(FULL, __float_as_int(ea.v[2]), C_STEPS - 1);
       int kn = kc - 1;
       while (kn >= 0) {
         float r1;
         int rn;
-        const int n = lquiet_run<GM>(pin, Lm, L1, ckmax, kn, 0, lane, pt, pn, zlog, ownc, r1, rn);
+        const int n = lquiet_run(pin, Lm, L1, ckmax, kn, 0, lane, pt, pn, zlog, r1, rn);
         for (int m = 0; m < n; ++m) {
           if ((kn - m + 1) % kSeg == 0) store_zero(kn - m, pt, pn);
-          zero_push<GM>(pout, Lm, L1, kn - m, lane);
+          zero_push(pout, Lm, L1, kn - m, lane);
           pt = __shfl_sync(FULL, r1, m * C_STEPS + C_STEPS - 1);
           pn = __shfl_sync(FULL, rn, m * C_STEPS + C_STEPS - 1);
         }
         kn -= n;
         if (n < 32 / C_STEPS) break;
       }
-      bstate_zero<R, GM>(bs);
+      bstate_zero(bs);
       bs.ht = lane == 31 ? pt : 0.f;
-      bs.hn = lane == 31 ? pn : zero_frame<GM>();
+      bs.hn = lane == 31 ? pn : 0;
       kc = kn;
       return true;
     }
@@ -2045,20 +1719,19 @@ __device__ void lbeta_band(const Args& a, const LParams& lp, const Place& w, int
         rt = lane == 31 ? p4.y : rt;
         rn = lane == 31 ? __float_as_int(p4.z) : rn;
         float2 xs[H], E[H];
-        lemit<R, DD, GM>(sb[S0 + cu], k, nlive, hd, xs, E);
-        if constexpr (!IN) lblank<R>(act, xs, E);
+        lemit<R, DD>(sb[S0 + cu], k, nlive, hd, xs, E);
         if constexpr (IN) rows.template fetch<VEC>(src, sb[S0 + cu]);
         else rows.load(src, i - cu - AH, sb[S0 + cu]);
         src -= rows.ld;
         int ft;
         float fB, vd0, mx;
         float2 vm[H], vi[H], sr[H], br[H];
-        bcells<NS, R, DD, GM>(bs, rb, rn, GM == 1 ? i - cu == L1 : act, term, gO, gE, gX, nlive, hd, ft, fB, vm, vi, sr, br, vd0, mx);
-        bfinish<R, GM>(bs, ft, mx, vm, vi, vd0, E, rt, rn);
+        bcells<NS, R, DD>(bs, rb, rn, act, gO, gE, gX, nlive, hd, ft, fB, vm, vi, sr, br, vd0, mx);
+        bfinish<R>(bs, ft, mx, vm, vi, vd0, E, rt, rn);
         if (act && lane == 0 && pout) {
           pout[0 * (Lm + 1) + i - cu] = bs.ob;
           pout[1 * (Lm + 1) + i - cu] = bs.t[0].x;
-          pout[2 * (Lm + 1) + i - cu] = __int_as_float(bs.nb + frame_bias<GM>());
+          pout[2 * (Lm + 1) + i - cu] = __int_as_float(bs.nb);
         }
       }
     };
@@ -2084,7 +1757,7 @@ __device__ void lbeta_band(const Args& a, const LParams& lp, const Place& w, int
   }
 }
 
-template <int NS, int R, int GM = 0>
+template <int NS, int R>
 __global__ void __launch_bounds__(128) lbeta_kernel(Args a) {
   __shared__ float4 s_push[4][C_STEPS];
   const int lane = threadIdx.x & 31;
@@ -2096,17 +1769,17 @@ __global__ void __launch_bounds__(128) lbeta_kernel(Args a) {
     if (lane == 0) task = (int)atomicAdd(a.counters + 1, 1u);
     task = __shfl_sync(FULL, task, 0);
     if (task >= ntasks) break;
-    const Place w = place_of<NS, R, GM>(a, task, true);
+    const Place w = place_of<NS, R>(a, task, true);
     if ((w.band + 1) * 32 * R > w.pr.L2 || !w.pr.vec)
-      lbeta_band<NS, R, 1, GM>(a, lp, w, lane, deadline, s_push[threadIdx.x >> 5]);
+      lbeta_band<NS, R, 1>(a, lp, w, lane, deadline, s_push[threadIdx.x >> 5]);
     else
-      lbeta_band<NS, R, 0, GM>(a, lp, w, lane, deadline, s_push[threadIdx.x >> 5]);
+      lbeta_band<NS, R, 0>(a, lp, w, lane, deadline, s_push[threadIdx.x >> 5]);
     __syncwarp();
   }
 }
 
 // The segments of every band (a.nseg per band): one warp each.
-template <int NS, int R, bool SPARSE, int GM = 0>
+template <int NS, int R, bool SPARSE>
 __global__ void __launch_bounds__(32) lseg_kernel(Args a) {
   extern __shared__ float smem[];
   const int lane = threadIdx.x;
@@ -2114,40 +1787,12 @@ __global__ void __launch_bounds__(32) lseg_kernel(Args a) {
   const int ntasks = a.B * a.nb * a.nseg;
   for (int task = blockIdx.x; task < ntasks; task += gridDim.x) {
     const int slot = task / a.nseg, seg = task - slot * a.nseg;
-    const Place w = place_of<NS, R, GM>(a, slot, false);
-    lbwd_band<NS, R, SPARSE, true, GM>(a, lp, w, lane, smem, 0, seg);
+    const Place w = place_of<NS, R>(a, slot, false);
+    if constexpr (!split_code<R>()) lbwd_band<NS, R, SPARSE, 2, true>(a, lp, w, lane, smem, 0, seg);
+    else if ((w.band + 1) * 32 * R > w.pr.L2) lbwd_band<NS, R, SPARSE, 1, true>(a, lp, w, lane, smem, 0, seg);
+    else lbwd_band<NS, R, SPARSE, 0, true>(a, lp, w, lane, smem, 0, seg);
     lcp_wait_all();
     __syncwarp();
-  }
-}
-
-// Pairs flagged for the log domain (GM 1 and 2): their completion counts to 0,
-// their cross-band buffers to the sentinel; the task counters to 0.
-template <int NS, int R, int GM>
-__global__ void __launch_bounds__(128) redo_kernel(Args a) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) { a.counters[0] = 0u; a.counters[1] = 0u; }
-  if (a.status[1] == 0u) return;
-  const float none = __uint_as_float(SENTINEL_BITS);
-  for (int p = blockIdx.x; p < a.B; p += gridDim.x) {
-    const unsigned f = a.pair_done[p];
-    __syncthreads();
-    if (!(f & (PAIR_REDO | PAIR_LOST))) continue;
-    if (threadIdx.x == 0) a.pair_done[p] = (f & PAIR_TIMEOUT) | PAIR_REDO;
-    size_t ed0, bp0, ne, np;
-    if (a.layout == 0) {
-      ne = (size_t)a.nb * 2 * NS * a.Lmax1;
-      np = (size_t)a.nb * push_fields<NS, GM>() * (a.Lmax1 + 1);
-      ed0 = p * ne;
-      bp0 = p * np;
-    } else {
-      const long long* q = a.plan_pairs + (size_t)p * PLAN_PAIR_WORDS;
-      ne = (size_t)q[PW_NB] * 2 * NS * q[PW_L1];
-      np = (size_t)q[PW_NB] * push_fields<NS, GM>() * (q[PW_L1] + 1);
-      ed0 = (size_t)q[PW_EDGE0];
-      bp0 = (size_t)q[PW_BP0];
-    }
-    for (size_t x = threadIdx.x; x < ne; x += blockDim.x) a.edge[ed0 + x] = none;
-    for (size_t x = threadIdx.x; x < np; x += blockDim.x) a.bpush[bp0 + x] = none;
   }
 }
 
@@ -2162,7 +1807,7 @@ __global__ void adjoint_reset_kernel(unsigned* counters, unsigned* pair_done, in
 
 // SPARSE: checkpoints every a.ck_every chunks (the chunks between are
 // recomputed); otherwise every chunk (a.ck_every must be 1).
-template <int NS, int R, int WARPS, bool SPARSE = false, int GM = 0>
+template <int NS, int R, int WARPS, bool SPARSE = false>
 __global__ void __launch_bounds__(32 * WARPS) lbwd_kernel(Args a) {
   extern __shared__ float smem[];
   const int lane = threadIdx.x & 31;
@@ -2176,8 +1821,10 @@ __global__ void __launch_bounds__(32 * WARPS) lbwd_kernel(Args a) {
     if (lane == 0) task = (int)atomicAdd(a.counters + 1, 1u);
     task = __shfl_sync(FULL, task, 0);
     if (task >= ntasks) break;
-    const Place w = place_of<NS, R, GM>(a, task, true);
-    lbwd_band<NS, R, SPARSE, false, GM>(a, lp, w, lane, sm, deadline, 0);
+    const Place w = place_of<NS, R>(a, task, true);
+    if constexpr (!split_code<R>()) lbwd_band<NS, R, SPARSE, 2>(a, lp, w, lane, sm, deadline);
+    else if ((w.band + 1) * 32 * R > w.pr.L2) lbwd_band<NS, R, SPARSE, 1>(a, lp, w, lane, sm, deadline);
+    else lbwd_band<NS, R, SPARSE, 0>(a, lp, w, lane, sm, deadline);
   }
 }
 
