@@ -45,7 +45,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if not force and up_to_date():
         return SO
     cmd = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-shared",
-           "--split-compile=0",   # optimise the kernels on all cores
            "-I", os.path.join(ROOT, "include"), "-o", SO + ".tmp", *SOURCES]
     if verbose:
         cmd.insert(1, "-Xptxas=-v")

@@ -1201,13 +1201,25 @@ int swb_sw_affine_forward_static(const float* scores, const int* lengths, int B,
                                  int L2max, float gap_open, float gap_ext, float temp,
                                  float* value, float* map, float* grad_open, float* grad_ext,
                                  float* grad_temp, void* stream, const swb_options* opt) {
-  // size check first: an oversize batch is rejected before any CUDA call
-  const int r = pick_r(opt, B, L2max, lin_eligible<3, 0>(gap_open, gap_ext, temp, opt));
+  // size check first: an oversize batch is rejected before any CUDA call.  A
+  // batch that fits the scratch at 8 columns per lane only (about a tenth less
+  // per cell than at 4) runs at 8 unless the caller chose.
+  const bool lin = lin_eligible<3, 0>(gap_open, gap_ext, temp, opt);
+  int r = pick_r(opt, B, L2max, lin);
+  swb_options wide{};
   if (B > 0 && L1max >= 0 && L2max >= 0 && valid_r_local(r)) {
-    const size_t need = r == 2 ? layout_for<3, 2>(B, L1max, L2max).total
-                               : (r == 4 ? layout_for<3, 4>(B, L1max, L2max).total
-                                         : layout_for<3, 8>(B, L1max, L2max).total);
-    if (need > (size_t)SWB_STATIC_SCRATCH_BYTES) return SWB_ERR_WORKSPACE;
+    auto need = [&](int cols) {
+      return cols == 2 ? layout_for<3, 2>(B, L1max, L2max).total
+                       : (cols == 4 ? layout_for<3, 4>(B, L1max, L2max).total
+                                    : layout_for<3, 8>(B, L1max, L2max).total);
+    };
+    const size_t most = (size_t)SWB_STATIC_SCRATCH_BYTES;
+    if (need(r) > most && !(opt && opt->cols_per_lane) && lin && L2max >= 256 && need(8) <= most) {
+      if (opt) wide = *opt;
+      wide.cols_per_lane = r = 8;
+      opt = &wide;
+    }
+    if (need(r) > most) return SWB_ERR_WORKSPACE;
   }
   void* ws = nullptr;
   if (B > 0) {
