@@ -449,8 +449,9 @@ __device__ __forceinline__ void col0_edge(int i, float g0, float g1, float (&e)[
 // affine (11 floats): A = (wMM, wMI, wMD, wIM), B = (wII, wDM, wDD, s), then
 // the beta-init terms C = (bM0, bI0) and D = bD0; linear (6 floats):
 // A = (map factor, wA, wU, wL), then s, then the beta-init term b0.  s is the
-// cell's scaled score.  The init terms are written only for steps where some
-// lane's init can be nonzero (fwd_cells returns that flag).
+// cell's scaled score (global linear: the entropy of its predecessor choice).
+// The init terms are written only for steps where some lane's init can be
+// nonzero (fwd_cells returns that flag).
 template <int NS, int R>
 __device__ __forceinline__ void put_weights(float* ent, int lane, int c, float4 A, float4 B,
                                             float sc) {
@@ -628,14 +629,17 @@ __device__ __forceinline__ bool fwd_cells(float (&ph)[NS][R], float (&pl)[NS][R]
       const float vu = ((uh - r) + g0) + ul;
       const float vl = ((lh[0] - r) + g0) + ll[0];
       const float ta = ex2(va), tu = ex2(vu), tl = ex2(vl);
-      const float sm = (ta + tu) + tl;
+      const float sm = (ta + tu) + tl, ls = lg2(sm);
       float Ah, Al;
-      fast2(r, lg2(sm), Ah, Al);
+      fast2(r, ls, Ah, Al);
       if (hold) { Ah = uh; Al = ul; }
       if constexpr (WT) {
         const float v = hold ? 0.f : recip(sm);
-        put_weights<NS, R>(went, lane, c, make_float4(ta * v, ta * v, tu * v, tl * v),
-                           make_float4(0.f, 0.f, 0.f, 0.f), s[c]);
+        const float wa = ta * v, wu = tu * v, wl = tl * v;
+        // the entropy of the cell's predecessor choice, in bits (bwd_band: dS/dT)
+        const float h = hold ? 0.f : ls - fmaf(wa, va, fmaf(wu, vu, wl * vl));
+        put_weights<NS, R>(went, lane, c, make_float4(wa, wa, wu, wl),
+                           make_float4(0.f, 0.f, 0.f, 0.f), h);
       }
       dgh[0] = uh; dgl[0] = ul;
       lh[0] = Ah; ll[0] = Al;
@@ -1075,9 +1079,22 @@ __global__ void __launch_bounds__(128) value_kernel(Args a) {
 // Parameters a pair's finish needs (natural units, and k = log2(e) / T).
 struct PParams { float go, ge, T, k; };
 
+// dS/dT = (S - <score>) / T in 64 bits (S and the score are large, their
+// difference is not): (Sh, Sl) = log2 Z, the match part m and the gaps g0, g1
+// in the same scaled units, o and e the expected gap counts.
+__device__ __forceinline__ float dS_dT(float Sh, float Sl, double m, double o, double g0, double e, double g1) {
+  constexpr double kLn2 = 0.693147180559945309;
+  return (float)(kLn2 * ((double)Sh + (double)Sl - (m + o * g0 + e * g1)));
+}
+
+template <bool EXACT>
+__device__ __forceinline__ double scaled(float g, float k) { return EXACT ? (double)g * k : (double)(g * k); }
+
 // Last band task of a pair to finish folds the per-band gradient partials (in
 // band order, so the result is deterministic) into the outputs.
-template <int NS, int GM = 0>
+// LIN: the linear domain, whose gap factors are 2^(gap k) of the exact product;
+// the log domain adds the rounded one.
+template <int NS, int GM = 0, bool LIN = false>
 __device__ void finish_pair_p(const Args& a, const Place& w, int lane, float Sh, float Sl,
                               float g0sum, float g1sum, float pssum, PParams pp);
 
@@ -1087,7 +1104,7 @@ __device__ void finish_pair(const Args& a, const Place& w, int lane, float Sh, f
   finish_pair_p<NS, GM>(a, w, lane, Sh, Sl, g0sum, g1sum, pssum, PParams{a.go, a.ge, a.T, a.k});
 }
 
-template <int NS, int GM>
+template <int NS, int GM, bool LIN>
 __device__ void finish_pair_p(const Args& a, const Place& w, int lane, float Sh, float Sl,
                               float g0sum, float g1sum, float pssum, PParams pp) {
   constexpr bool G = GM == 1;
@@ -1105,16 +1122,13 @@ __device__ void finish_pair_p(const Args& a, const Place& w, int lane, float Sh,
         if (a.g_ext) a.g_ext[p] = nan;
         return;
       }
-      float o = 0.f, e = 0.f, ps = 0.f;
+      double o = 0., e = 0., ps = 0.;
       for (int b = 0; b < w.nb; ++b) {
         const float* q = a.gpart + 4 * (w.slot0 + b);
         o += ld_poll(q + 0);
         e += ld_poll(q + 1);
         ps += ld_poll(q + 2);
       }
-      const float inv_k = 1.f / pp.k;         // = T * ln 2
-      const float S = (Sh + Sl) * inv_k;
-      const float match = ps * inv_k;
       if (G && (w.pr.L1 == 0 || w.pr.L2 == 0)) {
         // the terminal is a boundary cell: its value, its gap derivatives, dS/dT = 0
         float dgo, dge;
@@ -1124,16 +1138,11 @@ __device__ void finish_pair_p(const Args& a, const Place& w, int lane, float Sh,
         a.g_T[p] = 0.f;
         return;
       }
-      a.value[p] = S;
-      if (NS == 3) {
-        a.g_open[p] = o;
-        a.g_ext[p] = e;
-        a.g_T[p] = (S - (match + (o * pp.go + e * pp.ge))) / pp.T;
-      } else {
-        a.g_open[p] = o;
-        if (a.g_ext) a.g_ext[p] = 0.f;
-        a.g_T[p] = (S - (match + o * pp.go)) / pp.T;
-      }
+      a.value[p] = (Sh + Sl) * (1.f / pp.k);   // 1 / k = T ln 2
+      a.g_open[p] = (float)o;
+      if (a.g_ext) a.g_ext[p] = NS == 3 ? (float)e : 0.f;
+      if (G && NS == 1) a.g_T[p] = (float)(ps * 0.693147180559945309);   // an entropy in bits (bwd_band)
+      else a.g_T[p] = dS_dT(Sh, Sl, ps, o, scaled<LIN>(pp.go, pp.k), NS == 3 ? e : 0., scaled<LIN>(pp.ge, pp.k));
     }
   }
 }
@@ -1153,6 +1162,12 @@ __device__ void finish_pair_p(const Args& a, const Place& w, int lane, float Sh,
 // G (global alignment): the only beta-init is beta = 1 at the terminal cell
 // A[L1, L2]; pushes that leave the grid into the row-0 and column-0 boundary
 // cells (values j * gap and i * gap) add index * push to dS/dgap there.
+// Global linear: dS/dT is the entropy of the path distribution, summed cell by
+// cell as flow times the entropy of the cell's predecessor choice (all terms
+// >= 0, those of the boundary 0).  As (S - <score>) / T it is the small
+// difference of two large sums, in which the flow's own rounding, about 1e-7 a
+// step, shows: 33 x 700 at T = 0.25, S = -545, dS/dT = 19.55: 6.3e-3 off that
+// way, 8.6e-5 this way.
 template <int NS, int R, int GM = 0>
 __device__ void bwd_band(const Args& a, const Place& w, int lane, float* sm, uint64_t deadline) {
   constexpr bool G = GM == 1;
@@ -1564,7 +1579,7 @@ __device__ void bwd_band(const Args& a, const Place& w, int lane, float* sm, uin
           float4 f0, f1;
           float sc;
           get_weights<NS, R>(E, lane, c, f0, f1, sc);
-          // f0 = (map factor, wA, wU, wL)
+          // f0 = (map factor, wA, wU, wL); sc: the scaled score (G: the entropy)
           float i0 = 0.f, i1 = 0.f, i2 = 0.f;
           if (hasinit) get_inits<NS, R>(E, lane, c, i0, i1, i2);
           const float b = i0 + ac[0][c];
@@ -1572,7 +1587,7 @@ __device__ void bwd_band(const Args& a, const Place& w, int lane, float* sm, uin
           pm[c] = pv_;
           const float pU = b * f0.z, pL = b * f0.w, pD = b * f0.y;
           cA += pU + pL;
-          cS += pv_ * sc;
+          cS += (G ? b : pv_) * sc;
           if constexpr (G) {
             // pushes into the boundary: row 0 (up to column j, diag to j - 1)
             // and column 0 (left to row i, diag to row i - 1)

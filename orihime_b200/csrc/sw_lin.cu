@@ -1009,7 +1009,7 @@ __device__ __forceinline__ void lfinish_seg(const Args& a, const Place& w, int l
   done = __shfl_sync(FULL, done, 0);
   if ((done & ~PAIR_TIMEOUT) != (unsigned)(w.nb * a.nseg) - 1) return;
   __threadfence();
-  float o = 0.f, e = 0.f, m = 0.f;
+  double o = 0., e = 0., m = 0.;
   for (int b0 = 0; b0 < w.nb; b0 += 32) {
     BandSum s;
     if (b0 + lane < w.nb) {
@@ -1029,12 +1029,10 @@ __device__ __forceinline__ void lfinish_seg(const Args& a, const Place& w, int l
     if (a.g_ext) a.g_ext[p] = nan;
     return;
   }
-  const float inv_k = 1.f / pp.k;         // = T * ln 2
-  const float S = (Sh + Sl) * inv_k, match = m * inv_k;
-  a.value[p] = S;
-  a.g_open[p] = o;
-  if (a.g_ext) a.g_ext[p] = NS == 3 ? e : 0.f;
-  a.g_T[p] = NS == 3 ? (S - (match + (o * pp.go + e * pp.ge))) / pp.T : (S - (match + o * pp.go)) / pp.T;
+  a.value[p] = (Sh + Sl) * (1.f / pp.k);   // 1 / k = T ln 2
+  a.g_open[p] = (float)o;
+  if (a.g_ext) a.g_ext[p] = NS == 3 ? (float)e : 0.f;
+  a.g_T[p] = dS_dT(Sh, Sl, m, o, scaled<true>(pp.go, pp.k), NS == 3 ? e : 0., scaled<true>(pp.ge, pp.k));
 }
 
 // One row of the outside recursion for one lane: (rb, rt, rn) are the right
@@ -1239,7 +1237,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
   const int k_lo = SEG ? seg * kSeg : 0, k_hi = SEG ? min(k_lo + kSeg, nch) : nch;
   if (!(L1 > 0 && col0 < L2) || k_lo >= k_hi) {
     if constexpr (SEG) lfinish_seg<NS>(a, w, lane, seg, Sh, Sl, 0.f, 0.f, 0.f, pp);
-    else finish_pair_p<NS>(a, w, lane, Sh, Sl, 0.f, 0.f, 0.f, pp);
+    else finish_pair_p<NS, 0, true>(a, w, lane, Sh, Sl, 0.f, 0.f, 0.f, pp);
     return;
   }
   const float invZ = 1.f / zm;
@@ -1589,7 +1587,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
     flush();
     lfinish_seg<NS>(a, w, lane, seg, Sh, Sl, gsum.a.s, gsum.b.s, gsum.m.s, pp);
   } else {
-    finish_pair_p<NS>(a, w, lane, Sh, Sl, gsum.a.s, gsum.b.s, gsum.m.s, pp);
+    finish_pair_p<NS, 0, true>(a, w, lane, Sh, Sl, gsum.a.s, gsum.b.s, gsum.m.s, pp);
   }
 }
 
