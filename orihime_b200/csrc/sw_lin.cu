@@ -40,14 +40,27 @@
 // inputs' normalised frames (the lane's previous row, the left lane's row and
 // the left lane's previous row), which makes every converted input <= 1;
 // then the row's sum gives the normalised frame n = et + exponent(sum) in
-// which the row is <= 1.  Rows are never rescaled: the raw values keep the
-// compute frame et and every use scales them by 2^(frame - target) (a
-// power-of-two factor built from the exponent bits, folded into the gap
-// factors).  Frames are floored at 0: the empty alignment's weight 1 is
-// always representable and Z >= 1, so values below 2^-149 of it are dropped,
-// as the reference drops exponentials below e^-88 of their LSE's maximum.
-// Scores are within |s|/T <= 80 (the host's domain check), so E <= 2^115.4
-// and a step's raw values stay below 2^122.
+// which the row is <= 1.  Within a lane rows are never rescaled: the raw
+// values keep the compute frame et and every use scales them by
+// 2^(frame - target) (a power-of-two factor built from the exponent bits,
+// folded into the gap factors).  What a lane passes on is normalised.  Frames
+// are floored at 0: the empty alignment's weight 1 is always representable
+// and Z >= 1.  Scores are within |s|/T <= 80 (the host's domain check), so
+// E <= 2^115.4 and a step's raw values stay below 2^122.
+//
+// What is lost.  A lane's columns share one frame, so a column more than 126
+// bits below the lane's row is dropped (fewer by what a row of the lane gained
+// in one step: its own values are converted in one factor).  It matters where
+// the dropped column's path would later have caught up, which takes matches
+// worth those bits inside the lane: never at scores of a few T, often at 8
+// columns per lane and low temperature.  Pairs of 512 with a wrong map (more
+// than 1e-3 off the log domain), scores 3 N(0, 1), gap -1 (linear, the worse
+// model), 600 x 172 / 500 x 384, at 2, 4 and 8 columns per lane:
+//   T = 0.5    0 / 0     0 / 0      1 / 0
+//   T = 0.35   0 / 0     0 / 0    335 / 45
+//   T = 0.25   0 / 0    75 / 6    511 / 460
+// 172 x 600, wide instead of tall: none.  A call that needs every pair at low
+// temperature takes 2 columns per lane or the log domain (swb_options).
 //
 // The kernels run when every transition factor is at most 1 (gaps <= 0);
 // otherwise the host uses the log-domain kernels of sw_kernels.cu.
@@ -199,8 +212,9 @@ template <int NS, int R> struct LState {
   static constexpr int H = R / 2;
   float2 v[NS == 3 ? 2 : 1][H];    // raw M and I (linear: A) of the lane's latest row (frame e)
   float2 c[NS == 3 ? H : 1];       // affine: the row's column sums (M + I) + D (frame e)
-  float ds;                        // the left lane's column sum (linear: A) of that row, last column (frame e)
-  float od, oc;                    // out to the right lane: D of the column after the last, the last column's sum
+  float ds;                        // the left lane's column sum (linear: A) of that row, last column (frame nd)
+  float od, oc;                    // out to the right lane, in the normalised frame n: D of the column after
+                                   // the last, the last column's sum
   int e, n, nd;                    // raw frame, normalised frame, the left lane's normalised frame of that row
 };
 
@@ -250,6 +264,24 @@ __device__ __forceinline__ void ldchain(const float2 (&m)[R / 2], float d0, floa
     for (int c = 0; c < R; ++c)
       if (c >= nlive) col(d, c) = 0.f;
   }
+}
+
+// The normalised frame of a row from its raw frame e and sum rs (which bounds
+// every value of the row: all are >= 0), and the outputs in it.  The outputs
+// are normalised here, not by the receiver: its factor reaches down to 2^-126
+// only, and a raw value can stand up to 2^115 above its frame, so a value
+// 2^-12 below the receiver's row could become 0 there (affine pairs of 32 to
+// 1000 at T = 0.25, 4 columns per lane: 4 of 400 lost paths that way, 1 this
+// way; 600 x 172, linear: 39 and 23 of 512).  The two products,
+// with the split scale of the adjoint's posteriors, cost up to 3 % of a call
+// (64 x 1024^2 883 -> 909 us, 1 x 1023 x 2047 752 -> 754); by the receiver,
+// which then needs e as well, they cost as much or more.
+template <int NS, typename S>
+__device__ __forceinline__ void lnormal(S& s, int e, float rs) {
+  s.n = max(e - 126 + sexp(rs), 0);
+  const float f = p2b(e - s.n + 127);
+  if constexpr (NS == 3) s.od *= f;
+  s.oc *= f;
 }
 
 template <int NS, int R>
@@ -307,17 +339,17 @@ __device__ __forceinline__ void lck_restore(const float* rec, int lane, LState<N
     s.oc = s.v[0][H - 1].y;
     rs = sum2(s.v[0]);
   }
-  s.n = max(s.e - 126 + sexp(rs), 0);
+  lnormal<NS>(s, s.e, rs);
 }
 
 // One step of the forward wavefront for one lane: (xd, xc) are the left
-// lane's outputs of this row in its raw frame xe (normalised frame xn), E the
-// emissions 2^(s k) (0 past the pair).  Updates the state to this row in the
+// lane's outputs of this row in its normalised frame xn, E the emissions
+// 2^(s k) (0 past the pair).  Updates the state to this row in the
 // frame et (its raw frame from then on) and returns the row's sum over its
 // columns and states in `rs`.
 // Affine: M, I and `d` = D; linear: A and `d` = the emission part.
 template <int NS, int R, int DM>
-__device__ __forceinline__ void lcells(LState<NS, R>& s, float xd, float xc, int xe, int xn,
+__device__ __forceinline__ void lcells(LState<NS, R>& s, float xd, float xc, int xn,
                                        const float2 (&E)[R / 2], float gO, float gE, int nlive, bool hd,
                                        float2 (&d)[R / 2], float& rs) {
   constexpr int H = R / 2;
@@ -325,16 +357,16 @@ __device__ __forceinline__ void lcells(LState<NS, R>& s, float xd, float xc, int
   // converted input is <= 1 (a raw value's frame exceeds its normalised frame
   // by at most 126)
   const int et = max(max(s.n, xn), s.nd);
-  s.nd = xn;
   const int q = 127 - et;
-  const float fU = p2b(s.e + q), fL = p2b(xe + q);
+  const float fU = p2b(s.e + q), fL = p2b(xn + q), fD = p2b(s.nd + q);
+  s.nd = xn;
   const float2 fU2 = dup2(fU), st2 = dup2(p2b(q));   // st: the fresh-start term 1 in frame et
   if constexpr (NS == 3) {
     float2 m[H];
 #pragma unroll
     for (int k = 0; k < H; ++k) {
       const float2 p = k == 0 ? make_float2(s.ds, s.c[H - 1].x) : s.c[k > 0 ? k - 1 : 0];
-      m[k] = mul2(E[k], fma2(fU2, p, st2));
+      m[k] = mul2(E[k], fma2(k == 0 ? make_float2(fD, fU) : fU2, p, st2));
     }
     const float2 gOu = dup2(gO * fU), gEu = dup2(gE * fU);
 #pragma unroll
@@ -345,7 +377,7 @@ __device__ __forceinline__ void lcells(LState<NS, R>& s, float xd, float xc, int
       s.v[0][k] = m[k];
       s.c[k] = add2(add2(m[k], s.v[1][k]), d[k]);
     }
-    s.ds = xc * fL;
+    s.ds = xc;
     s.oc = s.c[H - 1].y;
     rs = sum2(s.c);
   } else {
@@ -354,12 +386,12 @@ __device__ __forceinline__ void lcells(LState<NS, R>& s, float xd, float xc, int
 #pragma unroll
     for (int k = 0; k < H; ++k) {
       const float2 p = k == 0 ? make_float2(s.ds, s.v[0][H - 1].x) : s.v[0][k > 0 ? k - 1 : 0];
-      d[k] = mul2(E[k], fma2(fU2, p, st2));
+      d[k] = mul2(E[k], fma2(k == 0 ? make_float2(fD, fU) : fU2, p, st2));
     }
 #pragma unroll
     for (int k = 0; k < H; ++k) x[k] = fma2(gU, s.v[0][k], d[k]);
-    s.ds = xc * fL;
-    col(s.v[0], 0) = fmaf(gO, s.ds, col(x, 0));
+    s.ds = xc;
+    col(s.v[0], 0) = fmaf(gO, xc * fL, col(x, 0));
 #pragma unroll
     for (int c = 1; c < R; ++c) col(s.v[0], c) = fmaf(gO, col(s.v[0], c - 1), col(x, c));
     if (masks<DM>(hd)) {
@@ -370,10 +402,9 @@ __device__ __forceinline__ void lcells(LState<NS, R>& s, float xd, float xc, int
     s.oc = s.v[0][H - 1].y;
     rs = sum2(s.v[0]);
   }
-  // the row sum over columns and states bounds every value of the row (all
-  // are >= 0) and is the row's partition term
+  // the row sum over columns and states is the row's partition term
   s.e = et;
-  s.n = max(1 - q + sexp(rs), 0);
+  lnormal<NS>(s, et, rs);
 }
 
 // Scaled scores and emissions of one step as pairs: clamped at XMAX, NEG
@@ -506,20 +537,17 @@ __device__ __forceinline__ float ld_poll_if(const float* p, bool ok) {
 }
 
 // Edge records, one per row of a band: the last lane's outputs of the row.
-// Affine: one float4 (od, oc, raw frame, normalised frame); linear: one
-// float2 (oc, the two frames packed).  A band's records start at the next
+// Affine: one float4 (od, oc, normalised frame, 0); linear: one float2 (oc,
+// normalised frame).  A band's records start at the next
 // 16-byte boundary of its edge slice (2 NS floats per row hold them with the
 // padding; slices start at even offsets).
 template <int NS> struct LEdge {
   __device__ static __forceinline__ float* base(float* edge, size_t off) {
     return edge + (NS == 3 ? (off + 3) / 4 * 4 : off);
   }
-  __device__ static __forceinline__ void put(float* b, int i, float od, float oc, int e, int n, int rs_exp) {
-    if constexpr (NS == 3) {
-      reinterpret_cast<float4*>(b)[i - 1] = make_float4(od, oc, __int_as_float(e), __int_as_float(n));
-    } else {
-      reinterpret_cast<float2*>(b)[i - 1] = make_float2(oc, __uint_as_float(((unsigned)e << 8) | (unsigned)rs_exp));
-    }
+  __device__ static __forceinline__ void put(float* b, int i, float od, float oc, int n) {
+    if constexpr (NS == 3) reinterpret_cast<float4*>(b)[i - 1] = make_float4(od, oc, __int_as_float(n), 0.f);
+    else reinterpret_cast<float2*>(b)[i - 1] = make_float2(oc, __int_as_float(n));
   }
   // record i (0 where !ok), a strong load; no branch
   __device__ static __forceinline__ float4 get(const float* b, int i, bool ok) {
@@ -538,16 +566,14 @@ template <int NS> struct LEdge {
   }
   __device__ static __forceinline__ bool missing(const float4& v) {
     if constexpr (NS == 3)
-      return is_sentinel(v.x) || is_sentinel(v.y) || is_sentinel(v.z) || is_sentinel(v.w);
+      return is_sentinel(v.x) || is_sentinel(v.y) || is_sentinel(v.z);
     else
       return is_sentinel(v.x) || is_sentinel(v.y);
   }
-  // (od, oc, e, n) of a resolved record
+  // (od, oc, n) of a resolved record
   __device__ static __forceinline__ float4 open(const float4& v) {
     if constexpr (NS == 3) return v;
-    const unsigned w = __float_as_uint(v.y);
-    const int e = (int)(w >> 8);
-    return make_float4(0.f, v.x, __int_as_float(e), __int_as_float(max(e - 126 + (int)(w & 0xffu), 0)));
+    return make_float4(0.f, v.x, v.y, 0.f);
   }
   // Bounded wait for record i; on expiry the status word and the pair's flag
   // are set and the record reads as 0.
@@ -746,11 +772,9 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
           xd = lane == 0 ? e4.x : xd;
         }
         float xc = __shfl_up_sync(FULL, s.oc, 1);
-        int xe = __shfl_up_sync(FULL, s.e, 1);
         int xn = __shfl_up_sync(FULL, s.n, 1);
         xc = lane == 0 ? e4.y : xc;
-        xe = lane == 0 ? __float_as_int(e4.z) : xe;
-        xn = lane == 0 ? __float_as_int(e4.w) : xn;
+        xn = lane == 0 ? __float_as_int(e4.z) : xn;
         float2 xs[H], E[H];
         lemit<R, DD>(sb[(h * C_STEPS + cu) % AH], k, nlive, hd, xs, E);
         if constexpr (IN) rows.template fetch<VEC>(src, sb[(h * C_STEPS + cu) % AH]);
@@ -759,10 +783,10 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
         rsv[cu] = 0.f;
         ev[cu] = 0;
         if (act) {
-          lcells<NS, R, DD>(s, xd, xc, xe, xn, E, gO, gE, nlive, hd, d, rsv[cu]);
+          lcells<NS, R, DD>(s, xd, xc, xn, E, gO, gE, nlive, hd, d, rsv[cu]);
           ev[cu] = s.e;
           cmx = max(cmx, s.n);
-          if (lane == 31) LE::put(eout, i + cu, s.od, s.oc, s.e, s.n, sexp(rsv[cu]));
+          if (lane == 31) LE::put(eout, i + cu, s.od, s.oc, s.n);
         }
       }
     };
@@ -1440,17 +1464,16 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
             float xd = 0.f;
             if constexpr (NS == 3) xd = __shfl_up_sync(FULL, st.od, 1);
             float xc = __shfl_up_sync(FULL, st.oc, 1);
-            int xe = __shfl_up_sync(FULL, st.e, 1);
             int xn = __shfl_up_sync(FULL, st.n, 1);
             const float e0 = __shfl_sync(FULL, er.x, cu), e1 = __shfl_sync(FULL, er.y, cu);
-            const float e2 = __shfl_sync(FULL, er.z, cu), e3 = __shfl_sync(FULL, er.w, cu);
-            if (lane == 0) { xd = e0; xc = e1; xe = __float_as_int(e2); xn = __float_as_int(e3); }
+            const float e2 = __shfl_sync(FULL, er.z, cu);
+            if (lane == 0) { xd = e0; xc = e1; xn = __float_as_int(e2); }
             float2 xs[H], E[H];
             lemit<R, DM>(ab[u], k, nlive, hd, xs, E);
             rows.load(src, i + PF, ab[u]);
             src += rows.ld;
             float rs;
-            if (act) lcells<NS, R, DM>(st, xd, xc, xe, xn, E, gO, gE, nlive, hd, d, rs);
+            if (act) lcells<NS, R, DM>(st, xd, xc, xn, E, gO, gE, nlive, hd, d, rs);
             ++i;
           }
         }
@@ -1465,16 +1488,15 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
       float xd = 0.f;
       if constexpr (NS == 3) xd = __shfl_up_sync(FULL, st.od, 1);
       float xc = __shfl_up_sync(FULL, st.oc, 1);
-      int xe = __shfl_up_sync(FULL, st.e, 1);
       int xn = __shfl_up_sync(FULL, st.n, 1);
       if (lane == 0) {
         const float4 e4 = s_eb[cu];
-        xd = e4.x; xc = e4.y; xe = __float_as_int(e4.z); xn = __float_as_int(e4.w);
+        xd = e4.x; xc = e4.y; xn = __float_as_int(e4.z);
       }
       float2 xs[H], E[H];
       lemit<R, DM>(nsb[cu], k, nlive, hd, xs, E);
       float rs;
-      if (act) lcells<NS, R, DM>(st, xd, xc, xe, xn, E, gO, gE, nlive, hd, d, rs);
+      if (act) lcells<NS, R, DM>(st, xd, xc, xn, E, gO, gE, nlive, hd, d, rs);
       float* ent = sm + (size_t)cu * FW * 32;
       // field g's R columns as pairs: [g][quad][lane][4] (2 columns: [g][lane][2])
       auto put = [&](int g, const float2 (&x)[H]) {
@@ -1544,17 +1566,22 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
       float fB, vd0, mx;
       float2 vm[H], vi[H], sr[H], br[H], P[H];
       bcells<NS, R, DM>(bs, rb, rn, act, gO, gE, gX, nlive, hd, ft, fB, vm, vi, sr, br, vd0, mx);
-      // raw alpha (frame ea) times raw beta (frame ft), over Z
-      const float asc = p2any(ea + ft - ze) * invZ;
+      // raw alpha (frame ea) times raw beta (frame ft), over Z: half of the
+      // scale on each.  Both may stand up to 2^115 above their frames, where
+      // the whole scale would be 0 and their product infinite.
+      const int sh = ea + ft - ze, sha = sh >> 1;
+      const float fA = p2any(sha), fZ = p2any(sh - sha) * invZ;
       float2 so = dup2(0.f);
 #pragma unroll
       for (int j = 0; j < H; ++j) {
-        const float2 p = mul2(mul2(NS == 3 ? fm[j] : fd[j], dup2(asc)), vm[j]);
+        fm[j] = mul2(fm[j], dup2(fA));
+        fd[j] = mul2(fd[j], dup2(fA));
+        const float2 p = mul2(NS == 3 ? fm[j] : fd[j], mul2(vm[j], dup2(fZ)));
         P[j] = make_float2(fminf(p.x, 1.f), fminf(p.y, 1.f));   // a posterior: rounding may pass 1
         so = fma2(fm[j], sr[j], so);
         cS = fma2(P[j], xs[j], cS);
       }
-      cA = fmaf((so.x + so.y) * asc, gO, cA);
+      cA = fmaf((so.x + so.y) * fZ, gO, cA);
       if constexpr (NS == 3) {
         float2 fi[H];
         get(1, fi);
@@ -1564,7 +1591,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
           sxi = fma2(fi[j], bs.b[j], sxi);
           sxd = fma2(fd[j], br[j], sxd);
         }
-        cB = fmaf(fmaf(sxi.x + sxi.y, fB, sxd.x + sxd.y) * asc, gE, cB);
+        cB = fmaf(fmaf((sxi.x + sxi.y) * fA, fB, sxd.x + sxd.y) * fZ, gE, cB);
       }
       bfinish<R>(bs, ft, mx, vm, vi, vd0, E, rt, rn);
       if (act) {
