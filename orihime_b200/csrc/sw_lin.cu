@@ -1128,17 +1128,21 @@ __device__ __forceinline__ void bcells(const BState<R>& s, float rb, int rn, boo
   mx = x[0];
 }
 
-// The state after the row: t = E beta_M in the row's normalised frame.
+// The state after the row: t = E beta_M in the row's normalised frame, 0 in a
+// row outside the pair (!live), whose E is of whatever score a load left there:
+// t takes part in the quiet-chunk test of its warp, and the kernels' leftovers
+// differ (and, after a quiet run that a record not written yet ended, depend on
+// timing).
 template <int R>
-__device__ __forceinline__ void bfinish(BState<R>& s, int ft, float mx, const float2 (&vm)[R / 2],
+__device__ __forceinline__ void bfinish(BState<R>& s, int ft, float mx, bool live, const float2 (&vm)[R / 2],
                                         const float2 (&vi)[R / 2], float vd0, const float2 (&E)[R / 2],
                                         float rt, int rn) {
   constexpr int H = R / 2;
   const int nn = max(ft - 126 + sexp(mx), 0);
-  const float bs = p2b(ft - nn + 127);
+  const float bs = p2b(ft - nn + 127), ts = live ? bs : 0.f;
 #pragma unroll
   for (int k = 0; k < H; ++k) {
-    s.t[k] = mul2(mul2(vm[k], dup2(bs)), E[k]);
+    s.t[k] = mul2(mul2(vm[k], dup2(ts)), E[k]);
     s.b[k] = vi[k];
   }
   s.fb = ft;
@@ -1593,7 +1597,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
         }
         cB = fmaf(fmaf((sxi.x + sxi.y) * fA, fB, sxd.x + sxd.y) * fZ, gE, cB);
       }
-      bfinish<R>(bs, ft, mx, vm, vi, vd0, E, rt, rn);
+      bfinish<R>(bs, ft, mx, act, vm, vi, vd0, E, rt, rn);
       if (act) {
         store_pairs<R>(mrow, jl, pr, P);
         if (lane == 0 && pout) {
@@ -1760,7 +1764,7 @@ __device__ void lbeta_band(const Args& a, const LParams& lp, const Place& w, int
         float fB, vd0, mx;
         float2 vm[H], vi[H], sr[H], br[H];
         bcells<NS, R, DD>(bs, rb, rn, act, gO, gE, gX, nlive, hd, ft, fB, vm, vi, sr, br, vd0, mx);
-        bfinish<R>(bs, ft, mx, vm, vi, vd0, E, rt, rn);
+        bfinish<R>(bs, ft, mx, act, vm, vi, vd0, E, rt, rn);
         if (act && lane == 0 && pout) {
           pout[0 * (Lm + 1) + i - cu] = bs.ob;
           pout[1 * (Lm + 1) + i - cu] = bs.t[0].x;

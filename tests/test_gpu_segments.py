@@ -50,3 +50,28 @@ def test_segments_equal_whole_bands(family, shape):
         rest = m[b].clone()
         rest[:a, :c] = 0
         assert not np.any(rest.cpu().numpy())
+
+
+@pytest.mark.parametrize("family", ["affine", "linear"])
+@pytest.mark.parametrize("L1,L2", [(1023, 2047), (260, 1500), (64, 700), (33, 1000)])
+def test_quiet_stretch_up_to_the_first_rows(family, L1, L2):
+    """Whole strips without mass whose chunks reach above row 1: what the
+    kernels do there, outside the pair, decides no quiet chunk differently.
+    (260 x 1500, linear, seed 1: 192 cells differed, by 3e-35.)  And a
+    second run gives the same bits."""
+    from orihime_b200 import _ops, ragged
+
+    for seed in (0, 4, 1, 3):
+        g = torch.Generator().manual_seed(seed)
+        torch.randn(1, L1, L2, generator=g)   # the noted pair follows this draw
+        s = (torch.randn(L1, 64, generator=g) @ torch.randn(L2, 64, generator=g).T * 0.75).contiguous()
+        kw = dict(gap_open=-2.0, gap_ext=-0.5) if family == "affine" else dict(gap=-1.0)
+        run = _ops.run_affine if family == "affine" else _ops.run_linear
+        v, m, *grads = run(s[None].cuda(), None, *kw.values(), 1.0)
+        flat, off, ln = ragged.pack([s])
+        plan = ragged.Plan(ln, off, family=family, device="cuda", cols_per_lane=4)
+        for _ in range(2):
+            out = plan.run(flat.cuda(), temp=1.0, **kw)
+            assert plan.status() == 0
+            assert torch.equal(v, out.value) and torch.equal(grads[-1], out.grad_temp)
+            assert torch.equal(m[0], ragged.unpack(out.map, off, ln)[0])
