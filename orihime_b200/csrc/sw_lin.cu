@@ -643,11 +643,11 @@ template <int R> __host__ __device__ constexpr int fwd_ahead() { return R == 8 ?
 // at a time (about 220 cycles a time in a lone warp).
 template <int R> __host__ __device__ constexpr int fwd_block() { return split_code<R>() ? 2 * C_STEPS : C_STEPS; }
 
-// Forward wavefront of one band: per-lane partition sums (plain within a
-// chunk, Kahan over chunks, in the lane's largest normalised frame), the
-// left-to-right edge records and, every C steps, a checkpoint of the lane
-// state plus the chunk's largest normalised frame.  The band's partition
-// partial is (frame, mantissa sum): Z_band = sum * 2^frame.
+// Forward wavefront of one band: per-lane partition sums (Kahan over the rows,
+// in the lane's largest normalised frame), the left-to-right edge records and,
+// every C steps, a checkpoint of the lane state plus the chunk's largest
+// normalised frame.  The band's partition partial is (frame, mantissa sum):
+// Z_band = sum * 2^frame.
 //
 // The left band's records of a block (WB steps) pass through shared memory,
 // where lane 0 reads the one of each step.  They are requested two blocks
@@ -695,8 +695,15 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
   float2 d[H];
 #pragma unroll
   for (int j = 0; j < H; ++j) d[j] = dup2(0.f);
+  // partition: the row sums in the frame ze (the largest normalised frame so
+  // far), Kahan-compensated
   float zm = (band == 0 && lane == 0) ? 1.f : 0.f, zc = 0.f;   // M[0,0]: the empty alignment
   int ze = 0;
+  auto zadd = [&](float v) {
+    const float y = v - zc, t = zm + y;
+    zc = (t - zm) - y;
+    zm = t;
+  };
 
   // lane u < WB holds the left band's edge record lane 0 needs at step u of a
   // block: `ea` of the next block, `eb` of the one after
@@ -800,19 +807,13 @@ __device__ void lfwd_band(const Args& a, const LParams& lp, const Place& w, int 
     }
     if (!done) steps(std::false_type{}, std::false_type{});
     i += C_STEPS;
-    // partition: the chunk's row sums in the frame ze (the largest normalised
-    // frame so far), Kahan-compensated from chunk to chunk
     {
       const int zn = max(ze, cmx);
       const float f = p2b(ze - zn + 127);
-      float y = 0.f;
-#pragma unroll
-      for (int cu = 0; cu < C_STEPS; ++cu) y = fmaf(rsv[cu], p2b(ev[cu] - zn + 127), y);
       zm *= f;
-      y -= zc * f;
-      const float tt = zm + y;
-      zc = (tt - zm) - y;
-      zm = tt;
+      zc *= f;
+#pragma unroll
+      for (int cu = 0; cu < C_STEPS; ++cu) zadd(rsv[cu] * p2b(ev[cu] - zn + 127));
       ze = zn;
     }
     if (keep_ck) {
@@ -1006,10 +1007,10 @@ __device__ __forceinline__ void bstate_load(const float* rec, int lane, BState<R
   s.hn = __float_as_int(x[2 * R + 4]);
 }
 
-// The gradient sums of a band are formed per segment of kSeg chunks (plain
-// sums per lane, then a shuffle tree) and folded over the segments, last one
-// first, with compensation: the adjoint of a whole band and the segment
-// kernel give the same bits.
+// The gradient sums of a band are formed per segment of kSeg chunks (per lane
+// plain within a chunk and compensated over the chunks, then a shuffle tree)
+// and folded over the segments, last one first, with compensation: the adjoint
+// of a whole band and the segment kernel give the same bits.
 constexpr int kSeg = 4;
 struct BandSum {
   KSum a, b, m;
@@ -1348,10 +1349,9 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
   if constexpr (SEG) bstate_load<R>(a.bck + ((w.slot0 + band) * a.nseg + seg) * BDims<R>::BREC, lane, bs);
   else bstate_zero(bs);
   BandSum gsum;
-  float cA = 0.f, cB = 0.f;   // the segment's plain sums
-  float2 cS = dup2(0.f);
+  KSum gA, gB, gS;            // the lane's sums over the segment's chunks
   auto flush = [&]() {        // at the end of a segment
-    float v0 = cA, v1 = cB, v2 = cS.x + cS.y;
+    float v0 = gA.s, v1 = gB.s, v2 = gS.s;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       v0 += __shfl_xor_sync(FULL, v0, o);
@@ -1359,7 +1359,7 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
       v2 += __shfl_xor_sync(FULL, v2, o);
     }
     gsum.add(v0, v1, v2);
-    cA = 0.f; cB = 0.f; cS = dup2(0.f);
+    gA = KSum(); gB = KSum(); gS = KSum();
   };
 
   // log2 of Z is at least zlog; a chunk is quiet (below) when every cell's
@@ -1531,6 +1531,8 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
     }
     if (lane < C_STEPS) s_pb[lane] = make_float4(pbc[0], pbc[1], pbc[2], 0.f);
     __syncwarp();
+    float cA = 0.f, cB = 0.f;   // this chunk's plain sums
+    float2 cS = dup2(0.f);
     int i = t0 + C_STEPS - lane;
     float* mrow = pr.m + (long long)(i - 1) * pr.ld + jl;
     // ---- outside recursion over the chunk, last step first ----
@@ -1611,6 +1613,9 @@ __device__ void lbwd_band(const Args& a, const LParams& lp, const Place& w, int 
     }
 #pragma unroll
     for (int f = 0; f < NPF; ++f) pbc[f] = pbn[f];
+    gA.add(cA);
+    if constexpr (NS == 3) gB.add(cB);
+    gS.add(cS.x + cS.y);
     if (!SEG && kc % kSeg == 0) flush();
     __syncwarp();
   }
