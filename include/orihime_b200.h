@@ -80,12 +80,12 @@ typedef struct swb_options {
 #define SWB_DOMAIN_LINEAR 2
 
 /* Columns per lane the padded entry points use when swb_options does not
- * set one, in a batch of one pair: for the local families (family 1 linear
- * gap, 3 affine gaps) in the linear domain, 2 on batches with L2max <= 64,
- * else 4 (8 where L2max >= 256 and the batch has at least 768 bands of 256
- * columns); in the log domain and for families 2, 4, 5 (the global and
- * Saigo-Vert models) always 4.  Results depend on it bit for
- * bit (the band decomposition orders each pair's sums), so a packed plan
+ * set one: for the local families (family 1 linear gap, 3 affine gaps) in the
+ * linear domain, 2 on batches with L2max <= 64 and at temperatures below 0.3
+ * (where more columns in a lane's exponent frame can lose paths), else 4; in
+ * the log domain and for families 2, 4, 5 (the global and Saigo-Vert models)
+ * always 4.  It does not depend on the batch size.  Results depend on it bit
+ * for bit (the band decomposition orders each pair's sums), so a packed plan
  * built with the same value reproduces a padded call exactly.  No reference
  * counterpart. */
 int swb_cols_per_lane(int family, int L2max, float gap_open, float gap_ext, float temp);
@@ -439,11 +439,12 @@ int swb_scan_scores(const float* x, int B, long long per_item, float limit, floa
  * lengths and parameters, runs the checkpointed adjoint: the marginal map
  * and dS/dparameters (and the value again).  It can run more than once.
  * ck_every in [1, 16]: 1 keeps a checkpoint per chunk (the fastest
- * adjoint); 4 keeps about 0.93 bytes per cell of a large padded batch, and the
+ * adjoint); 4 keeps about 1.05 bytes per cell of a large padded batch, and the
  * adjoint recomputes the chunks in between from the nearest checkpoint.
  * The local families in the linear domain only: gaps must be <= 0, else
- * SWB_ERR_ARG.  Columns per lane as the padded entry points take for
- * the batch (see swb_cols_per_lane).  Workspace from
+ * SWB_ERR_ARG.  2 columns per lane where L2max <= 64, else 4, which is what
+ * the padded entry points take from T = 0.3 on; below it some pairs lose paths
+ * (swb_cols_per_lane).  Workspace from
  * swb_*_checkpoint_workspace_bytes(B, L1max, L2max, ck_every).
  */
 size_t swb_sw_affine_checkpoint_workspace_bytes(int B, int L1max, int L2max, int ck_every);

@@ -319,12 +319,17 @@ def run_value(fam, scores, lengths, params):
 def run_checkpoint(fam, scores, lengths, params, ck_every):
     """Forward wavefront only (local families, gaps <= 0): value [B] and the
     workspace holding the checkpoints the adjoint needs later, or None when
-    the parameters need the log-domain kernels (a positive gap)."""
+    the parameters need other kernels: the log domain's (a positive gap), or
+    fewer columns per lane than the checkpoints have (a low temperature)."""
     B, L1, L2 = scores.shape
     dev = scores.device
     value = torch.empty(B, dtype=torch.float32, device=dev)
     affine = fam == "sw_affine"
     if any(float(p) > 0 for p in params[:-1]) or B == 0:
+        return None
+    go, ge, T = (float(p) for p in (params if affine else (params[0], 0.0, params[1])))
+    cols = lambda t: _LIB.swb_cols_per_lane(3 if affine else 1, L2, go, ge, t)  # noqa: E731
+    if cols(T) != cols(1.0):
         return None
     nbytes = int((_LIB.swb_sw_affine_checkpoint_workspace_bytes if affine
                   else _LIB.swb_sw_checkpoint_workspace_bytes)(B, L1, L2, ck_every))

@@ -57,21 +57,25 @@ bool lin_eligible(float go, float ge, float T, const swb_options* opt) {
   return xo <= 0.0 && xe <= 0.0;
 }
 // Default columns per lane of the padded entry points, for the linear-domain
-// kernels: 2 on batches at most 64 columns wide (one band with every lane
-// live), 8 on wide batches with enough bands of 256 columns to fill the GPU
-// (half the bands, each step's fixed work spread over twice the cells), else
-// 4, whose steps are shorter: what counts then is the chain of steps.  The
-// log domain always takes 4.  Forward + adjoint, affine, 4 against 8 columns,
-// us: 4 x 1024^2 (16 bands of 256) 778 / 861; 64 x 1024^2 (256) 875 / 992;
-// 256 x 512^2 (512) 534 / 548; 512 x 512^2 (1024) 834 / 715.
-constexpr long long kWideBands = 768;
-int default_r(long long B, long long L2m, bool lin) {
-  if (!lin) return kDefaultR;
-  if (L2m <= 64) return 2;
-  return L2m >= 256 && B * ((L2m + 255) / 256) >= kWideBands ? 8 : kDefaultR;
-}
-int pick_r(const swb_options* opt, long long B, long long L2m, bool lin) {
-  return (opt && opt->cols_per_lane) ? opt->cols_per_lane : default_r(B, L2m, lin);
+// kernels.  By the padded width and the temperature alone, so that a pair's
+// result depends neither on the batch it is in nor on how a batch is sharded:
+//   2 where L2max <= 64 (one band with every lane live);
+//   2 below T = 0.3: a lane's columns share one exponent frame, and at 4 a
+//     part of the pairs there loses paths (scores 3 N(0, 1), T = 0.25: of 512
+//     pairs of 600 x 172, linear gap, 75 maps wrong at 4, none at 2; at
+//     T = 0.35 none at either; sw_lin.cu).  64 x 1024^2 takes 1078 us at 2 and
+//     922 at 4, 1024 x 512^2 2366 and 1456;
+//   else 4.  8 is faster where many wide pairs fill the GPU (1024 x 512^2,
+//     affine, 1319 us against 1506 at 4; 4096 x 512^2 forward alone 1226
+//     against 1310), and slower on every smaller batch (64 x 1024^2 1161 / 920,
+//     1 x 1023 x 2047 1327 / 765): a caller's choice (swb_options), from
+//     T = 0.5 on.
+// The log domain always takes 4.
+constexpr float kTwoColsT = 0.3f;
+int ck_r(long long L2m) { return L2m <= 64 ? 2 : kDefaultR; }   // checkpointed entry points: no T
+int default_r(long long L2m, bool lin, float T) { return lin && T < kTwoColsT ? 2 : (lin ? ck_r(L2m) : kDefaultR); }
+int pick_r(const swb_options* opt, long long L2m, bool lin, float T) {
+  return (opt && opt->cols_per_lane) ? opt->cols_per_lane : default_r(L2m, lin, T);
 }
 
 struct Layout {
@@ -203,12 +207,15 @@ cudaError_t setup_lin(DevInfo& d) {
                                                          32, lbwd_smem<NS, R>())) != cudaSuccess)
     return e;
   }
-  e = cudaFuncSetAttribute(swb::lbwd_kernel<NS, R, kWarpsBwd, true>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lbwd_smem<NS, R>());
-  if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &d.locc_sparse[NS == 3][ridx(R)], swb::lbwd_kernel<NS, R, kWarpsBwd, true>, 32 * kWarpsBwd,
-      lbwd_smem<NS, R>());
+  if constexpr (R < 8) {   // the checkpointed entry points run 2 or 4 columns per lane
+    e = cudaFuncSetAttribute(swb::lbwd_kernel<NS, R, kWarpsBwd, true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lbwd_smem<NS, R>());
+    if (e != cudaSuccess) return e;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &d.locc_sparse[NS == 3][ridx(R)], swb::lbwd_kernel<NS, R, kWarpsBwd, true>, 32 * kWarpsBwd,
+        lbwd_smem<NS, R>());
+  }
+  return e;
 }
 
 template <int NS, int R, int G = 0>
@@ -427,7 +434,7 @@ template <int NS, int G = 0>
 int launch_padded(const float* scores, const int* lengths, int B, int L1m, int L2m, float go,
                   float ge, float T, float* value, float* map, float* g_open, float* g_ext,
                   float* g_T, void* ws, size_t ws_bytes, void* stream, const swb_options* opt) {
-  const int r = pick_r(opt, B, L2m, lin_eligible<NS, G>(go, ge, T, opt));
+  const int r = pick_r(opt, L2m, lin_eligible<NS, G>(go, ge, T, opt), T);
   if (r == 2)
     return launch_padded_r<NS, 2, G>(scores, lengths, B, L1m, L2m, go, ge, T, value, map, g_open,
                                      g_ext, g_T, ws, ws_bytes, stream, opt);
@@ -476,8 +483,7 @@ int launch_value(const float* scores, const int* lengths, int B, int L1m, int L2
     return launch<NS, R, G>(a, l, (long long)B * l.nb, 0, false, ws, ws_bytes, stream, nullptr, true);
   };
   if constexpr (G == 0) {
-    const int r = default_r(B, L2m, lin_eligible<NS, G>(go, ge, T, nullptr));
-    if (r == 8) return run(std::integral_constant<int, 8>{});
+    const int r = default_r(L2m, lin_eligible<NS, G>(go, ge, T, nullptr), T);
     if (r == 2) return run(std::integral_constant<int, 2>{});
   }
   return run(std::integral_constant<int, kDefaultR>{});
@@ -487,7 +493,7 @@ template <int NS, int G = 0>
 size_t value_workspace(long long B, long long L1m, long long L2m) {
   size_t n = value_layout<NS, G, kDefaultR>(B, L1m, L2m).total;
   if constexpr (G == 0)
-    n = std::max({n, value_layout<NS, G, 8>(B, L1m, L2m).total, value_layout<NS, G, 2>(B, L1m, L2m).total});
+    n = std::max(n, value_layout<NS, G, 2>(B, L1m, L2m).total);
   return n;
 }
 
@@ -879,10 +885,8 @@ int ck_adjoint_r(const float* scores, const int* lengths, int B, int L1m, int L2
   const int ob = kc > 1 ? d->locc_sparse[NS == 3][ridx(R)] : d->locc[1][NS == 3][ridx(R)];
   const long long cap = (long long)d->sms * (ob > 0 ? ob : 1);
   const int grid = (int)std::max(1LL, std::min((ntasks + kWarpsBwd - 1) / kWarpsBwd, cap));
-  if constexpr (swb::split_code<R>()) {
-    const SegPlan seg = seg_plan<R>(l, ntasks);
-    if (seg.total && ws_bytes >= seg.total) return launch_segments<NS, R>(a, *d, seg, w, kc > 1, 0, st);
-  }
+  const SegPlan seg = seg_plan<R>(l, ntasks);
+  if (seg.total && ws_bytes >= seg.total) return launch_segments<NS, R>(a, *d, seg, w, kc > 1, 0, st);
   if (kc > 1)
     swb::lbwd_kernel<NS, R, kWarpsBwd, true><<<grid, 32 * kWarpsBwd, lbwd_smem<NS, R>(), st>>>(a);
   else
@@ -895,10 +899,7 @@ int ck_adjoint_r(const float* scores, const int* lengths, int B, int L1m, int L2
 template <int NS>
 int ck_forward(const float* scores, const int* lengths, int B, int L1m, int L2m, float go, float ge,
                float T, int kc, float* value, void* ws, size_t ws_bytes, void* stream_v) {
-  const int r = default_r(B, L2m, true);
-  if (r == 8)
-    return ck_forward_r<NS, 8>(scores, lengths, B, L1m, L2m, go, ge, T, kc, value, ws, ws_bytes, stream_v);
-  if (r == 2)
+  if (ck_r(L2m) == 2)
     return ck_forward_r<NS, 2>(scores, lengths, B, L1m, L2m, go, ge, T, kc, value, ws, ws_bytes, stream_v);
   return ck_forward_r<NS, 4>(scores, lengths, B, L1m, L2m, go, ge, T, kc, value, ws, ws_bytes, stream_v);
 }
@@ -907,11 +908,7 @@ template <int NS>
 int ck_adjoint(const float* scores, const int* lengths, int B, int L1m, int L2m, float go, float ge,
                float T, int kc, float* value, float* map, float* g_open, float* g_ext, float* g_T,
                void* ws, size_t ws_bytes, void* stream_v) {
-  const int r = default_r(B, L2m, true);
-  if (r == 8)
-    return ck_adjoint_r<NS, 8>(scores, lengths, B, L1m, L2m, go, ge, T, kc, value, map, g_open, g_ext,
-                               g_T, ws, ws_bytes, stream_v);
-  if (r == 2)
+  if (ck_r(L2m) == 2)
     return ck_adjoint_r<NS, 2>(scores, lengths, B, L1m, L2m, go, ge, T, kc, value, map, g_open, g_ext,
                                g_T, ws, ws_bytes, stream_v);
   return ck_adjoint_r<NS, 4>(scores, lengths, B, L1m, L2m, go, ge, T, kc, value, map, g_open, g_ext,
@@ -925,10 +922,8 @@ template <int R> size_t with_segments(const Layout& l, long long B) {
 
 template <int NS>
 size_t ck_workspace(long long B, long long L1m, long long L2m, int kc) {
-  const int r = default_r(B, L2m, true);
-  return r == 8   ? with_segments<8>(ck_layout<NS, 8>(B, L1m, L2m, kc), B)
-         : r == 2 ? with_segments<2>(ck_layout<NS, 2>(B, L1m, L2m, kc), B)
-                  : with_segments<4>(ck_layout<NS, 4>(B, L1m, L2m, kc), B);
+  return ck_r(L2m) == 2 ? with_segments<2>(ck_layout<NS, 2>(B, L1m, L2m, kc), B)
+                        : with_segments<4>(ck_layout<NS, 4>(B, L1m, L2m, kc), B);
 }
 
 }  // namespace
@@ -937,8 +932,8 @@ extern "C" {
 
 int swb_cols_per_lane(int family, int L2max, float gap_open, float gap_ext, float temp) {
   // family: 1 linear, 3 affine (local); 2, 4, 5 global and Saigo-Vert
-  if (family == 1) return default_r(1, L2max, lin_eligible<1, 0>(gap_open, 0.f, temp, nullptr));
-  if (family == 3) return default_r(1, L2max, lin_eligible<3, 0>(gap_open, gap_ext, temp, nullptr));
+  if (family == 1) return default_r(L2max, lin_eligible<1, 0>(gap_open, 0.f, temp, nullptr), temp);
+  if (family == 3) return default_r(L2max, lin_eligible<3, 0>(gap_open, gap_ext, temp, nullptr), temp);
   return (family >= 1 && family <= 5) ? kDefaultR : SWB_ERR_ARG;
 }
 
@@ -1202,10 +1197,11 @@ int swb_sw_affine_forward_static(const float* scores, const int* lengths, int B,
                                  float* value, float* map, float* grad_open, float* grad_ext,
                                  float* grad_temp, void* stream, const swb_options* opt) {
   // size check first: an oversize batch is rejected before any CUDA call.  A
-  // batch that fits the scratch at 8 columns per lane only (about a tenth less
-  // per cell than at 4) runs at 8 unless the caller chose.
+  // batch that fits the scratch only at more columns per lane (a cell then takes
+  // less of it: at 8 a tenth less than at 4) runs at those unless the caller
+  // chose.
   const bool lin = lin_eligible<3, 0>(gap_open, gap_ext, temp, opt);
-  int r = pick_r(opt, B, L2max, lin);
+  int r = pick_r(opt, L2max, lin, temp);
   swb_options wide{};
   if (B > 0 && L1max >= 0 && L2max >= 0 && valid_r_local(r)) {
     auto need = [&](int cols) {
@@ -1214,9 +1210,10 @@ int swb_sw_affine_forward_static(const float* scores, const int* lengths, int B,
                                     : layout_for<3, 8>(B, L1max, L2max).total);
     };
     const size_t most = (size_t)SWB_STATIC_SCRATCH_BYTES;
-    if (need(r) > most && !(opt && opt->cols_per_lane) && lin && L2max >= 256 && need(8) <= most) {
+    while (need(r) > most && !(opt && opt->cols_per_lane) && lin && r < (L2max >= 256 ? 8 : ck_r(L2max))) r *= 2;
+    if (r != pick_r(opt, L2max, lin, temp)) {
       if (opt) wide = *opt;
-      wide.cols_per_lane = r = 8;
+      wide.cols_per_lane = r;
       opt = &wide;
     }
     if (need(r) > most) return SWB_ERR_WORKSPACE;

@@ -470,6 +470,16 @@ DEFAULT_COLS = {"0:0": 2, "0:256": 2, "64:0": 4, "64:256": 2, "128:0": 8, "128:2
                 "256:0": 8, "256:256": 4, "512:0": 8, "512:256": 8, "1024:0": 8, "1024:256": 8}
 
 
+def cols_limit(temp: float) -> int:
+    """The most columns per lane that keep a local alignment's paths at this
+    temperature, for scores of about 3 N(0, 1): a lane's columns share one
+    exponent frame, and the lower the temperature, the more bits a match is
+    worth.  Pairs of 512 with a wrong map at 2, 4, 8 columns (600 x 172, linear
+    gap, the worst of the measured shapes): 0, 0, 1 at T = 0.5; 0, 0, 335 at
+    0.35; 0, 75, 511 at 0.25."""
+    return 8 if temp >= 0.5 else (4 if temp >= 0.3 else 2)
+
+
 def bucket_of(L1: int, L2: int) -> str:
     l2 = max(e for e in L2_EDGES if L2 >= e)
     l1 = max(e for e in L1_EDGES if L1 >= e)
@@ -699,7 +709,8 @@ def autotune_plan(lengths, offsets, family: str = "affine", device="cuda", flat=
     timing: one Plan per columns-per-lane choice (2, 4 and, for the local
     families, 8) and the MixedPlan of the bucket table, each captured in a
     CUDA graph and replayed on `flat` (the batch's packed scores; N(0, 1) *
-    1.5 if None) with CUDA events.  The choice is cached per GPU and batch
+    1.5 if None) with CUDA events.  The local families take no more columns
+    than cols_limit(temp) allows.  The choice is cached per GPU and batch
     signature (see cols_table for the cache folder).  Returns (plan, report)
     where report = {"choice": ..., "ms": {candidate: ms}, "cached": bool}."""
     import json
@@ -710,10 +721,13 @@ def autotune_plan(lengths, offsets, family: str = "affine", device="cuda", flat=
         dev = torch.device("cuda", torch.cuda.current_device())
     ln = np.asarray(lengths, dtype=np.int32).reshape(-1, 2)
     local = family in ("affine", "linear")
+    # run's own default temperature where only gaps are given, the tuning one where nothing is
+    most = cols_limit(float(params.get("temp", 1.0 if params else 0.5))) if local else 4
     cands = {f"R{r}": (lambda r=r: Plan(ln, offsets, family=family, device=dev, cols_per_lane=r))
-             for r in ((2, 4, 8) if local else (2, 4))}
-    cands["mixed"] = lambda: MixedPlan(ln, offsets, family=family, device=dev)
-    sig = _signature(ln, family)
+             for r in (2, 4, 8) if r <= most}
+    table = {k: min(v, most) for k, v in cols_table(dev).items()}
+    cands["mixed"] = lambda: MixedPlan(ln, offsets, family=family, device=dev, table=table)
+    sig = _signature(ln, family) + ("" if most == 8 or not local else f"|c{most}")
     path = _cache_path(dev).replace("cols_", "plans_")
     cache = {}
     if use_cache and os.path.exists(path):

@@ -72,3 +72,42 @@ def test_bench_traffic_profile_per_cols():
         assert v is not None and 8.0 <= v <= 20.0, (cols, v)
         assert os.path.exists(os.path.join(ROOT, src))
     assert bench.profile_traffic(2) == (None, None)
+
+
+def test_columns_do_not_depend_on_the_batch_and_fall_with_the_temperature(monkeypatch, tmp_path):
+    from orihime_b200 import _lib, ragged
+
+    q = _lib.load().swb_cols_per_lane
+    for fam in (1, 3):
+        for L2 in (1, 64):
+            assert q(fam, L2, -2.0, -0.5, 1.0) == 2
+        for L2 in (65, 255, 256, 300, 4096):
+            for T, want in ((1.0, 4), (0.3, 4), (0.29, 2), (0.25, 2)):
+                assert q(fam, L2, -2.0, -0.5, T) == want, (fam, L2, T)
+            assert q(fam, L2, 1.0, -0.5, 0.25) == 4   # the log domain
+    for fam in (2, 4, 5):
+        assert q(fam, 300, -2.0, -0.5, 0.25) == 4
+    assert [ragged.cols_limit(T) for T in (1.0, 0.5, 0.49, 0.3, 0.25)] == [8, 8, 4, 4, 2]
+
+    # autotune_plan offers no candidate above the limit, whatever an earlier call cached
+    monkeypatch.setenv("ORIHIME_B200_CACHE", str(tmp_path))
+    monkeypatch.delenv("ORIHIME_B200_COLS", raising=False)
+    made = []
+
+    class Fake:
+        def __init__(self, ln, off, family, device, cols_per_lane=0, table=None):
+            made.append(("mixed", max(table.values())) if table else ("R", cols_per_lane))
+
+    monkeypatch.setattr(ragged, "Plan", Fake)
+    monkeypatch.setattr(ragged, "MixedPlan", Fake)
+    ln = np.array([[300, 400], [50, 60]])
+    off, ln32 = ragged.layout(ln)
+    for temp, sig in ((1.0, ""), (0.35, "|c4"), (0.25, "|c2")):
+        path = tmp_path / "plans_cpu.json"
+        monkeypatch.setattr(ragged, "_cache_path", lambda dev: str(tmp_path / "cols_cpu.json"))
+        base = ragged._signature(ln32, "affine")
+        path.write_text(json.dumps({base + s: {"choice": c} for s, c in (("", "R8"), ("|c4", "mixed"), ("|c2", "R2"))}))
+        made.clear()
+        _, report = ragged.autotune_plan(ln32, off, device="cpu", gap_open=-2.0, gap_ext=-0.5, temp=temp)
+        assert report["cached"]
+        assert made == {"": [("R", 8)], "|c4": [("mixed", 4)], "|c2": [("R", 2)]}[sig]

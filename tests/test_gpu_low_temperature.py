@@ -75,3 +75,23 @@ def test_maps_of_many_pairs_equal_the_log_domain(family, cols, T, shape):
     log = _run(family, s, T, cols_per_lane=4, domain=_lib.DOMAIN_LOG)
     assert all(torch.isfinite(x).all() for x in lin)
     assert float((lin[1] - log[1]).abs().max()) < 1e-3
+
+
+@pytest.mark.parametrize("family", ["affine", "linear"])
+def test_public_route_keeps_the_paths_of_many_pairs(family):
+    """The padded entry points' own columns at T = 0.25: map, value alone and the
+    value op's gradient."""
+    import orihime_b200 as ohm
+    from orihime_b200 import _lib
+
+    g = torch.Generator().manual_seed(6)
+    s = (torch.bmm(torch.randn(256, 600, 64, generator=g), torch.randn(256, 64, 172, generator=g)) * 0.375)
+    s = s[s.abs().amax((1, 2)) / 0.25 <= 80].contiguous().cuda()
+    log = _run(family, s, 0.25, cols_per_lane=4, domain=_lib.DOMAIN_LOG)
+    kw = (dict(gap_open_score=-2.0, gap_extend_score=-0.5) if family == "affine" else dict(gap_score=-1.0))
+    fn, fv = (ohm.sw_affine, ohm.sw_affine_value) if family == "affine" else (ohm.sw, ohm.sw_value)
+    assert float((fn(s, temperature=0.25, **kw) - log[1]).abs().max()) < 1e-3
+    torch.testing.assert_close(fv(s, temperature=0.25, **kw), log[0], rtol=1e-5, atol=1e-3)
+    x = s.clone().requires_grad_(True)
+    fv(x, temperature=0.25, **kw).sum().backward()
+    assert float((x.grad - log[1]).abs().max()) < 1e-3
