@@ -439,14 +439,32 @@ int swb_scan_scores(const float* x, int B, long long per_item, float limit, floa
  * lengths and parameters, runs the checkpointed adjoint: the marginal map
  * and dS/dparameters (and the value again).  It can run more than once.
  * ck_every in [1, 16]: 1 keeps a checkpoint per chunk (the fastest
- * adjoint); 4 keeps about 1.05 bytes per cell of a large padded batch, and the
+ * adjoint); 4 keeps about 1.1 bytes per cell of a large padded batch (linear
+ * gap: 0.7), and the
  * adjoint recomputes the chunks in between from the nearest checkpoint.
  * The local families in the linear domain only: gaps must be <= 0, else
  * SWB_ERR_ARG.  2 columns per lane where L2max <= 64, else 4, which is what
  * the padded entry points take from T = 0.3 on; below it some pairs lose paths
  * (swb_cols_per_lane).  Workspace from
  * swb_*_checkpoint_workspace_bytes(B, L1max, L2max, ck_every).
+ *
+ * swb_*_adjoint_scratch is swb_*_adjoint with device memory of its own (16-byte
+ * aligned, swb_*_adjoint_scratch_bytes(B, L1max, L2max); 0 where it would not
+ * help), about 1 byte per cell, that need not be kept between the two halves:
+ * batches of few bands then take about half the time, with the same bits.
+ * With less scratch, or NULL, it is swb_*_adjoint.
  */
+size_t swb_sw_affine_adjoint_scratch_bytes(int B, int L1max, int L2max);
+int swb_sw_affine_adjoint_scratch(const float* scores, const int* lengths, int B, int L1max, int L2max,
+                                  float gap_open, float gap_ext, float temp, int ck_every, float* value,
+                                  float* map, float* grad_open, float* grad_ext, float* grad_temp,
+                                  void* workspace, size_t workspace_bytes, void* scratch,
+                                  size_t scratch_bytes, void* stream);
+size_t swb_sw_adjoint_scratch_bytes(int B, int L1max, int L2max);
+int swb_sw_adjoint_scratch(const float* scores, const int* lengths, int B, int L1max, int L2max, float gap,
+                           float temp, int ck_every, float* value, float* map, float* grad_gap,
+                           float* grad_temp, void* workspace, size_t workspace_bytes, void* scratch,
+                           size_t scratch_bytes, void* stream);
 size_t swb_sw_affine_checkpoint_workspace_bytes(int B, int L1max, int L2max, int ck_every);
 int swb_sw_affine_checkpoint(const float* scores, const int* lengths, int B, int L1max, int L2max,
                              float gap_open, float gap_ext, float temp, int ck_every, float* value,

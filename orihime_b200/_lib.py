@@ -186,6 +186,15 @@ def load() -> ctypes.CDLL:
     lib.swb_sw_affine_checkpoint.argtypes = [vp, vp, i, i, i, f, f, f, i, vp, vp, sz, vp]
     lib.swb_sw_affine_adjoint.restype = i
     lib.swb_sw_affine_adjoint.argtypes = [vp, vp, i, i, i, f, f, f, i, vp, vp, vp, vp, vp, vp, sz, vp]
+    lib.swb_sw_affine_adjoint_scratch_bytes.restype = sz
+    lib.swb_sw_affine_adjoint_scratch_bytes.argtypes = [i, i, i]
+    lib.swb_sw_affine_adjoint_scratch.restype = i
+    lib.swb_sw_affine_adjoint_scratch.argtypes = [vp, vp, i, i, i, f, f, f, i, vp, vp, vp, vp, vp, vp, sz, vp,
+                                                  sz, vp]
+    lib.swb_sw_adjoint_scratch_bytes.restype = sz
+    lib.swb_sw_adjoint_scratch_bytes.argtypes = [i, i, i]
+    lib.swb_sw_adjoint_scratch.restype = i
+    lib.swb_sw_adjoint_scratch.argtypes = [vp, vp, i, i, i, f, f, i, vp, vp, vp, vp, vp, sz, vp, sz, vp]
     lib.swb_sw_checkpoint.restype = i
     lib.swb_sw_checkpoint.argtypes = [vp, vp, i, i, i, f, f, i, vp, vp, sz, vp]
     lib.swb_sw_adjoint.restype = i

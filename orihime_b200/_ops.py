@@ -316,6 +316,12 @@ def run_value(fam, scores, lengths, params):
 
 # ---- checkpointed value: forward now, adjoint in the backward ---------------
 
+def checkpoint_bytes(fam, B, L1, L2, ck_every) -> int:
+    """Bytes of a run_checkpoint workspace: what is kept until the adjoint."""
+    return int((_LIB.swb_sw_affine_checkpoint_workspace_bytes if fam == "sw_affine"
+                else _LIB.swb_sw_checkpoint_workspace_bytes)(B, L1, L2, ck_every))
+
+
 def run_checkpoint(fam, scores, lengths, params, ck_every):
     """Forward wavefront only (local families, gaps <= 0): value [B] and the
     workspace holding the checkpoints the adjoint needs later, or None when
@@ -331,8 +337,7 @@ def run_checkpoint(fam, scores, lengths, params, ck_every):
     cols = lambda t: _LIB.swb_cols_per_lane(3 if affine else 1, L2, go, ge, t)  # noqa: E731
     if cols(T) != cols(1.0):
         return None
-    nbytes = int((_LIB.swb_sw_affine_checkpoint_workspace_bytes if affine
-                  else _LIB.swb_sw_checkpoint_workspace_bytes)(B, L1, L2, ck_every))
+    nbytes = checkpoint_bytes(fam, B, L1, L2, ck_every)
     ws = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=dev)
     with torch.cuda.device(dev):
         if affine:
@@ -353,18 +358,21 @@ def run_adjoint(fam, scores, lengths, params, ck_every, ws):
     e = lambda: torch.empty(B, dtype=torch.float32, device=dev)  # noqa: E731
     value, amap = e(), torch.empty_like(scores)
     nbytes = ws.numel()
+    nscr = int((_LIB.swb_sw_affine_adjoint_scratch_bytes if fam == "sw_affine"
+                else _LIB.swb_sw_adjoint_scratch_bytes)(B, L1, L2))
+    scr = torch.empty(max(nscr, 1), dtype=torch.uint8, device=dev)
     with torch.cuda.device(dev):
         if fam == "sw_affine":
             go, ge, gT = e(), e(), e()
-            rc = _LIB.swb_sw_affine_adjoint(_ptr(scores), _ptr(lengths), B, L1, L2, *map(float, params),
-                                            int(ck_every), _ptr(value), _ptr(amap), _ptr(go), _ptr(ge),
-                                            _ptr(gT), _ptr(ws), nbytes, _stream(dev))
+            rc = _LIB.swb_sw_affine_adjoint_scratch(
+                _ptr(scores), _ptr(lengths), B, L1, L2, *map(float, params), int(ck_every), _ptr(value),
+                _ptr(amap), _ptr(go), _ptr(ge), _ptr(gT), _ptr(ws), nbytes, _ptr(scr), nscr, _stream(dev))
             grads = (go, ge, gT)
         else:
             gg, gT = e(), e()
-            rc = _LIB.swb_sw_adjoint(_ptr(scores), _ptr(lengths), B, L1, L2, *map(float, params),
-                                     int(ck_every), _ptr(value), _ptr(amap), _ptr(gg), _ptr(gT), _ptr(ws),
-                                     nbytes, _stream(dev))
+            rc = _LIB.swb_sw_adjoint_scratch(
+                _ptr(scores), _ptr(lengths), B, L1, L2, *map(float, params), int(ck_every), _ptr(value),
+                _ptr(amap), _ptr(gg), _ptr(gT), _ptr(ws), nbytes, _ptr(scr), nscr, _stream(dev))
             grads = (gg, gT)
     _lib.check(rc, "swb_sw_adjoint")
     return (value, amap, *grads)

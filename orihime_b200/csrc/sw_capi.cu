@@ -114,16 +114,15 @@ Layout layout_sizes(long long B, size_t slots, size_t edge_floats, size_t bp_flo
 constexpr long long kSegSlots = 192;
 struct SegPlan {
   int nseg = 0;
-  size_t off_state = 0, off_part = 0, total = 0;   // total 0: not used
+  size_t off_part = 0, bytes = 0;   // states, then partials; bytes 0: not used
 };
 template <int R>
 SegPlan seg_plan(const Layout& l, long long slots) {
   SegPlan p;
   if (!swb::split_code<R>() || slots > kSegSlots) return p;
   p.nseg = (l.nchunks + swb::kSeg - 1) / swb::kSeg;
-  p.off_state = l.total;
-  p.off_part = p.off_state + align_up(sizeof(float) * (size_t)slots * p.nseg * swb::BDims<R>::BREC);
-  p.total = p.off_part + align_up(sizeof(float) * 4 * (size_t)slots * p.nseg);
+  p.off_part = align_up(sizeof(float) * (size_t)slots * p.nseg * swb::BDims<R>::BREC);
+  p.bytes = p.off_part + align_up(sizeof(float) * 4 * (size_t)slots * p.nseg);
   return p;
 }
 
@@ -294,11 +293,12 @@ int static_scratch(void** out) {
   return SWB_OK;
 }
 
-// The outside sweep and the segments of a padded batch.
+// The outside sweep and the segments of a padded batch; `mem`: p.bytes of
+// device memory, 16-byte aligned.
 template <int NS, int R>
-int launch_segments(Args a, const DevInfo& d, const SegPlan& p, char* w, bool sparse, int max_ctas, cudaStream_t st) {
-  a.bck = reinterpret_cast<float*>(w + p.off_state);
-  a.spart = reinterpret_cast<float*>(w + p.off_part);
+int launch_segments(Args a, const DevInfo& d, const SegPlan& p, char* mem, bool sparse, int max_ctas, cudaStream_t st) {
+  a.bck = reinterpret_cast<float*>(mem);
+  a.spart = reinterpret_cast<float*>(mem + p.off_part);
   a.nseg = p.nseg;
   const long long slots = (long long)a.B * a.nb, n = slots * p.nseg;
   const int os = d.sweep[NS == 3][ridx(R)], og = d.seg[sparse][NS == 3][ridx(R)];
@@ -374,7 +374,7 @@ int launch(Args a, const Layout& l, long long ntasks, size_t map_elems, bool cle
       SegPlan seg;
       if (a.layout == 0 && !value_only && !a.fault_inject) {
         seg = seg_plan<R>(l, ntasks);
-        if (ws_bytes < seg.total) seg = SegPlan{};
+        if (ws_bytes < l.total + seg.bytes) seg = SegPlan{};
       }
       swb::lfwd_kernel<NS, R><<<grid_f, 32 * kWarpsFwd, 0, st>>>(a);
       if (cudaPeekAtLastError() != cudaSuccess) return SWB_ERR_CUDA;
@@ -386,8 +386,8 @@ int launch(Args a, const Layout& l, long long ntasks, size_t map_elems, bool cle
         return cudaPeekAtLastError() == cudaSuccess ? SWB_OK : SWB_ERR_CUDA;
       }
       if constexpr (swb::split_code<R>()) {
-        if (seg.total)
-          return launch_segments<NS, R>(a, *d, seg, w, false, opt ? opt->max_ctas : 0, st);
+        if (seg.bytes)
+          return launch_segments<NS, R>(a, *d, seg, w + l.total, false, opt ? opt->max_ctas : 0, st);
       }
       swb::lbwd_kernel<NS, R, kWarpsBwd><<<grid_b, 32 * kWarpsBwd, lbwd_smem<NS, R>(), st>>>(a);
       return cudaPeekAtLastError() == cudaSuccess ? SWB_OK : SWB_ERR_CUDA;
@@ -860,7 +860,7 @@ int ck_forward_r(const float* scores, const int* lengths, int B, int L1m, int L2
 template <int NS, int R>
 int ck_adjoint_r(const float* scores, const int* lengths, int B, int L1m, int L2m, float go, float ge,
                  float T, int kc, float* value, float* map, float* g_open, float* g_ext, float* g_T,
-                 void* ws, size_t ws_bytes, void* stream_v) {
+                 void* ws, size_t ws_bytes, void* scratch, size_t scratch_bytes, void* stream_v) {
   Args a;
   Layout l;
   int rc = ck_setup<NS, R>(a, l, scores, lengths, B, L1m, L2m, go, ge, T, kc, ws, ws_bytes);
@@ -886,7 +886,8 @@ int ck_adjoint_r(const float* scores, const int* lengths, int B, int L1m, int L2
   const long long cap = (long long)d->sms * (ob > 0 ? ob : 1);
   const int grid = (int)std::max(1LL, std::min((ntasks + kWarpsBwd - 1) / kWarpsBwd, cap));
   const SegPlan seg = seg_plan<R>(l, ntasks);
-  if (seg.total && ws_bytes >= seg.total) return launch_segments<NS, R>(a, *d, seg, w, kc > 1, 0, st);
+  if (seg.bytes && scratch && scratch_bytes >= seg.bytes)
+    return launch_segments<NS, R>(a, *d, seg, static_cast<char*>(scratch), kc > 1, 0, st);
   if (kc > 1)
     swb::lbwd_kernel<NS, R, kWarpsBwd, true><<<grid, 32 * kWarpsBwd, lbwd_smem<NS, R>(), st>>>(a);
   else
@@ -907,23 +908,33 @@ int ck_forward(const float* scores, const int* lengths, int B, int L1m, int L2m,
 template <int NS>
 int ck_adjoint(const float* scores, const int* lengths, int B, int L1m, int L2m, float go, float ge,
                float T, int kc, float* value, float* map, float* g_open, float* g_ext, float* g_T,
-               void* ws, size_t ws_bytes, void* stream_v) {
+               void* ws, size_t ws_bytes, void* scratch, size_t scratch_bytes, void* stream_v) {
   if (ck_r(L2m) == 2)
     return ck_adjoint_r<NS, 2>(scores, lengths, B, L1m, L2m, go, ge, T, kc, value, map, g_open, g_ext,
-                               g_T, ws, ws_bytes, stream_v);
+                               g_T, ws, ws_bytes, scratch, scratch_bytes, stream_v);
   return ck_adjoint_r<NS, 4>(scores, lengths, B, L1m, L2m, go, ge, T, kc, value, map, g_open, g_ext,
-                             g_T, ws, ws_bytes, stream_v);
+                             g_T, ws, ws_bytes, scratch, scratch_bytes, stream_v);
 }
 
 // A layout's bytes with the segments' states and partials, where they are used.
 template <int R> size_t with_segments(const Layout& l, long long B) {
-  return std::max(l.total, seg_plan<R>(l, B * l.nb).total);
+  return l.total + seg_plan<R>(l, B * l.nb).bytes;
 }
 
 template <int NS>
 size_t ck_workspace(long long B, long long L1m, long long L2m, int kc) {
-  return ck_r(L2m) == 2 ? with_segments<2>(ck_layout<NS, 2>(B, L1m, L2m, kc), B)
-                        : with_segments<4>(ck_layout<NS, 4>(B, L1m, L2m, kc), B);
+  return ck_r(L2m) == 2 ? ck_layout<NS, 2>(B, L1m, L2m, kc).total : ck_layout<NS, 4>(B, L1m, L2m, kc).total;
+}
+
+// What the adjoint alone needs (nothing of it is kept between the two halves).
+template <int NS>
+size_t ck_scratch(long long B, long long L1m, long long L2m) {
+  if (ck_r(L2m) == 2) {
+    const Layout l = ck_layout<NS, 2>(B, L1m, L2m, 1);
+    return seg_plan<2>(l, B * l.nb).bytes;
+  }
+  const Layout l = ck_layout<NS, 4>(B, L1m, L2m, 1);
+  return seg_plan<4>(l, B * l.nb).bytes;
 }
 
 }  // namespace
@@ -947,6 +958,14 @@ size_t swb_sw_checkpoint_workspace_bytes(int B, int L1max, int L2max, int ck_eve
   return ck_workspace<1>(B, L1max, L2max, ck_every);
 }
 
+size_t swb_sw_affine_adjoint_scratch_bytes(int B, int L1max, int L2max) {
+  return B > 0 ? ck_scratch<3>(B, L1max, L2max) : 0;
+}
+
+size_t swb_sw_adjoint_scratch_bytes(int B, int L1max, int L2max) {
+  return B > 0 ? ck_scratch<1>(B, L1max, L2max) : 0;
+}
+
 int swb_sw_affine_checkpoint(const float* scores, const int* lengths, int B, int L1max, int L2max,
                              float gap_open, float gap_ext, float temp, int ck_every, float* value,
                              void* workspace, size_t workspace_bytes, void* stream) {
@@ -959,7 +978,17 @@ int swb_sw_affine_adjoint(const float* scores, const int* lengths, int B, int L1
                           float* map, float* grad_open, float* grad_ext, float* grad_temp,
                           void* workspace, size_t workspace_bytes, void* stream) {
   return ck_adjoint<3>(scores, lengths, B, L1max, L2max, gap_open, gap_ext, temp, ck_every, value,
-                       map, grad_open, grad_ext, grad_temp, workspace, workspace_bytes, stream);
+                       map, grad_open, grad_ext, grad_temp, workspace, workspace_bytes, nullptr, 0, stream);
+}
+
+int swb_sw_affine_adjoint_scratch(const float* scores, const int* lengths, int B, int L1max, int L2max,
+                                  float gap_open, float gap_ext, float temp, int ck_every, float* value,
+                                  float* map, float* grad_open, float* grad_ext, float* grad_temp,
+                                  void* workspace, size_t workspace_bytes, void* scratch,
+                                  size_t scratch_bytes, void* stream) {
+  return ck_adjoint<3>(scores, lengths, B, L1max, L2max, gap_open, gap_ext, temp, ck_every, value, map,
+                       grad_open, grad_ext, grad_temp, workspace, workspace_bytes, scratch, scratch_bytes,
+                       stream);
 }
 
 int swb_sw_checkpoint(const float* scores, const int* lengths, int B, int L1max, int L2max,
@@ -973,7 +1002,15 @@ int swb_sw_adjoint(const float* scores, const int* lengths, int B, int L1max, in
                    float temp, int ck_every, float* value, float* map, float* grad_gap,
                    float* grad_temp, void* workspace, size_t workspace_bytes, void* stream) {
   return ck_adjoint<1>(scores, lengths, B, L1max, L2max, gap, 0.f, temp, ck_every, value, map,
-                       grad_gap, nullptr, grad_temp, workspace, workspace_bytes, stream);
+                       grad_gap, nullptr, grad_temp, workspace, workspace_bytes, nullptr, 0, stream);
+}
+
+int swb_sw_adjoint_scratch(const float* scores, const int* lengths, int B, int L1max, int L2max, float gap,
+                           float temp, int ck_every, float* value, float* map, float* grad_gap,
+                           float* grad_temp, void* workspace, size_t workspace_bytes, void* scratch,
+                           size_t scratch_bytes, void* stream) {
+  return ck_adjoint<1>(scores, lengths, B, L1max, L2max, gap, 0.f, temp, ck_every, value, map, grad_gap,
+                       nullptr, grad_temp, workspace, workspace_bytes, scratch, scratch_bytes, stream);
 }
 
 size_t swb_sw_affine_aux_workspace_bytes(int B, int L1max, int L2max) {

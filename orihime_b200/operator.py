@@ -480,18 +480,25 @@ class _ValueFn(torch.autograd.Function):
 
 
 # Checkpoint stride of the checkpointed value op: the forward keeps the DP
-# state of every CHECKPOINT_EVERY-th chunk of 4 wavefront steps (about 3.7 / k
-# bytes per computed cell at k = CHECKPOINT_EVERY), and the adjoint recomputes
-# the chunks in between.  4 keeps ~0.93 B/cell, under a quarter of the map's
-# 4 B/cell.  While every chunk's state fits in DENSE_CHECKPOINT_BYTES (about
-# 3 B/cell) they are all kept: the adjoint of 64 x 1024^2 then takes 0.56 ms
-# instead of 1.34.
+# state of every k-th chunk of 4 wavefront steps, and the adjoint recomputes
+# the chunks in between.  At CHECKPOINT_EVERY about 1.1 bytes per cell are kept
+# (affine), a quarter of the map's 4.  Keeping them all, about 3.4, spares the
+# recomputation; adjoint, us: 64 x 1024^2 622 against 1388, 4 x 8192^2 4523
+# against 10613, 4 x 16384^2 9039 against 21846.  They are all kept where the
+# workspace is no larger than the map it replaces and than
+# DENSE_CHECKPOINT_BYTES (a 180th of the GPU's memory, as several such calls can
+# wait for their backward at once), or too small to matter.
 CHECKPOINT_EVERY = 4
 DENSE_CHECKPOINT_BYTES = 1 << 30
+SMALL_CHECKPOINT_BYTES = 64 << 20
 
 
-def _checkpoint_every(scores: Tensor) -> int:
-    return 1 if 3 * scores.numel() <= DENSE_CHECKPOINT_BYTES else CHECKPOINT_EVERY
+def _checkpoint_every(name: str, scores: Tensor) -> int:
+    from . import _ops as ops_mod
+
+    kept = ops_mod.checkpoint_bytes(name, *scores.shape, 1)
+    most = min(DENSE_CHECKPOINT_BYTES, 4 * scores.numel())
+    return 1 if kept <= max(most, SMALL_CHECKPOINT_BYTES) else CHECKPOINT_EVERY
 
 
 class _CheckpointedValueFn(torch.autograd.Function):
@@ -502,9 +509,9 @@ class _CheckpointedValueFn(torch.autograd.Function):
     [B, L1, L2] is kept between the two."""
 
     @staticmethod
-    def forward(ctx, fam, lengths, vals, ws_value, scores, *params):
+    def forward(ctx, fam, lengths, vals, every, ws_value, scores, *params):
         value, ws = ws_value
-        ctx.fam, ctx.lengths, ctx.ws = fam, lengths, ws
+        ctx.fam, ctx.lengths, ctx.every, ctx.ws = fam, lengths, every, ws
         ctx.vals = vals
         ctx.pmeta = _param_meta(params)
         ctx.save_for_backward(scores)
@@ -517,11 +524,11 @@ class _CheckpointedValueFn(torch.autograd.Function):
 
         (scores,) = ctx.saved_tensors
         _, smap, *grads = ops_mod.run_adjoint(ctx.fam.name, scores, ctx.lengths, ctx.vals,
-                                              _checkpoint_every(scores), ctx.ws)
-        gs = gv.view(-1, 1, 1) * smap if ctx.needs_input_grad[4] else None
-        out = [None, None, None, None, gs]
+                                              ctx.every, ctx.ws)
+        gs = gv.view(-1, 1, 1) * smap if ctx.needs_input_grad[5] else None
+        out = [None, None, None, None, None, gs]
         for k, meta in enumerate(ctx.pmeta):
-            out.append(_param_grad((gv * grads[k]).sum(), meta, ctx.needs_input_grad[5 + k]))
+            out.append(_param_grad((gv * grads[k]).sum(), meta, ctx.needs_input_grad[6 + k]))
         return tuple(out)
 
 
@@ -533,10 +540,11 @@ def _checkpointed_value(fam, lengths, scores, params, vals):
         return None
     from . import _ops as ops_mod
 
-    got = ops_mod.run_checkpoint(fam.name, scores.detach(), lengths, vals, _checkpoint_every(scores))
+    every = _checkpoint_every(fam.name, scores)
+    got = ops_mod.run_checkpoint(fam.name, scores.detach(), lengths, vals, every)
     if got is None:
         return None
-    return _CheckpointedValueFn.apply(fam, lengths, vals, got, scores, *params)
+    return _CheckpointedValueFn.apply(fam, lengths, vals, every, got, scores, *params)
 
 
 class _MapFn(torch.autograd.Function):

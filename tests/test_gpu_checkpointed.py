@@ -49,8 +49,10 @@ def test_checkpointed_adjoint_equals_one_call(fam, ck_every):
 
 
 def test_checkpoint_bytes_per_cell_at_stride_4():
-    """The memory the value op keeps between forward and backward on a large
-    batch: below 2 bytes per cell (the map it replaces is 4)."""
+    """What is kept between forward and adjoint at checkpoint stride 4 on a large
+    batch: below 2 bytes per cell (the map is 4).  The value op takes this stride
+    above its limits for dense checkpoints; what it keeps in all is measured in
+    test_memory_kept_by_the_value_op."""
     from orihime_b200 import _lib
 
     lib = _lib.load()
@@ -126,3 +128,59 @@ def test_c4_value_backward_peak_memory():
           f"{table / 2**30:.1f} GiB")
     assert torch.isfinite(v).all() and torch.isfinite(s.grad).all()
     assert peak < 21.7 * 2**30
+
+
+@pytest.mark.parametrize("fam", ["sw_affine", "sw"])
+@pytest.mark.parametrize("B,L1,L2", [(16, 1024, 1024), (64, 1024, 1024), (1, 4096, 4096)])
+def test_memory_kept_by_the_value_op(fam, B, L1, L2):
+    """Between forward and backward the value op holds less than the map it
+    replaces (4 bytes per cell) and a little for its outputs; what the adjoint
+    alone needs is not among it."""
+    import orihime_b200 as ohm
+
+    kw = (dict(gap_open_score=-2.0, gap_extend_score=-0.5) if fam == "sw_affine" else dict(gap_score=-1.0))
+    fn = ohm.sw_affine_value if fam == "sw_affine" else ohm.sw_value
+    s = torch.randn(B, L1, L2, device="cuda").requires_grad_(True)
+    fn(s, temperature=1.0, **kw).sum().backward()
+    s.grad = None
+    torch.cuda.synchronize()
+    base = torch.cuda.memory_allocated()
+    v = fn(s, temperature=1.0, **kw)
+    kept = torch.cuda.memory_allocated() - base
+    print(f"  {fam} {B} x {L1} x {L2}: {kept / s.numel():.2f} B/cell kept")
+    assert kept < 4 * s.numel()
+    v.sum().backward()
+
+
+@pytest.mark.parametrize("fam", ["sw_affine", "sw"])
+@pytest.mark.parametrize("ck_every", [2, 4, 16])
+@pytest.mark.parametrize("B,L1,L2", [(70, 129, 300), (200, 70, 60)])
+def test_sparse_adjoint_of_whole_bands_equals_one_call(fam, ck_every, B, L1, L2):
+    """Batches of more bands than the segments take (and the entry point without
+    scratch, below): the sparse records of the whole-band adjoint."""
+    from orihime_b200 import _lib, _ops
+
+    s = _emb(B, L1, L2, 7)
+    params = (-2.0, -0.5, 0.5) if fam == "sw_affine" else (-1.0, 0.5)
+    run = _ops.run_affine if fam == "sw_affine" else _ops.run_linear
+    want = run(s, None, *params)
+    value, ws = _ops.run_checkpoint(fam, s, None, params, ck_every)
+    assert torch.equal(value, want[0])
+    for g, w in zip(_ops.run_adjoint(fam, s, None, params, ck_every, ws), want):
+        assert torch.equal(g, w)
+    # two pairs: segments with scratch, whole bands without
+    s2 = s[:2].contiguous()
+    want = run(s2, None, *params)
+    _, ws = _ops.run_checkpoint(fam, s2, None, params, ck_every)
+    for scratch in (True, False):
+        if scratch:
+            got = _ops.run_adjoint(fam, s2, None, params, ck_every, ws)
+        else:
+            e = lambda: torch.empty(2, device="cuda")  # noqa: E731
+            got = [e(), torch.empty_like(s2)] + [e() for _ in params]
+            fn = _lib.load().swb_sw_affine_adjoint if fam == "sw_affine" else _lib.load().swb_sw_adjoint
+            rc = fn(s2.data_ptr(), None, 2, L1, L2, *params, ck_every, *(t.data_ptr() for t in got),
+                    ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+            assert rc == _lib.OK
+        for g, w in zip(got, want):
+            assert torch.equal(g, w)

@@ -180,8 +180,8 @@ def test_scale_invariance_bitwise():
 
 
 @pytest.mark.parametrize("width, pairs", [
-    (420, [[300, 420], [211, 300], [64, 399]]),   # 8 columns per lane, padded and cropped
-    (200, [[300, 200], [211, 137], [64, 199]]),   # 4 columns per lane
+    (420, [[300, 420], [211, 300], [64, 399]]),   # 4 columns per lane, four bands and fewer
+    (200, [[300, 200], [211, 137], [64, 199]]),   # 4 columns per lane, two bands
 ])
 def test_padding_invariance_bitwise(width, pairs):
     """A pair inside a padded batch (lengths) equals the cropped pair bit for
