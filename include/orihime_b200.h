@@ -81,8 +81,10 @@ typedef struct swb_options {
 
 /* Columns per lane the padded entry points use when swb_options does not
  * set one: for the local families (family 1 linear gap, 3 affine gaps) in the
- * linear domain, 2 on batches with L2max <= 64 and at temperatures below 0.3
- * (where more columns in a lane's exponent frame can lose paths), else 4; in
+ * linear domain, 2 on batches with L2max <= 64 and at temperatures below 0.35
+ * (where more columns in a lane's exponent frame can lose paths; scores of
+ * standard deviation 3 are assumed: 8 columns are good up to a deviation of
+ * 6 T, 4 up to 9 T, 2 up to 12 T, and beyond that the log domain), else 4; in
  * the log domain and for families 2, 4, 5 (the global and Saigo-Vert models)
  * always 4.  It does not depend on the batch size.  Results depend on it bit
  * for bit (the band decomposition orders each pair's sums), so a packed plan
@@ -444,7 +446,7 @@ int swb_scan_scores(const float* x, int B, long long per_item, float limit, floa
  * adjoint recomputes the chunks in between from the nearest checkpoint.
  * The local families in the linear domain only: gaps must be <= 0, else
  * SWB_ERR_ARG.  2 columns per lane where L2max <= 64, else 4, which is what
- * the padded entry points take from T = 0.3 on; below it some pairs lose paths
+ * the padded entry points take from T = 0.35 on; below it some pairs lose paths
  * (swb_cols_per_lane).  Workspace from
  * swb_*_checkpoint_workspace_bytes(B, L1max, L2max, ck_every).
  *

@@ -60,7 +60,7 @@ bool lin_eligible(float go, float ge, float T, const swb_options* opt) {
 // kernels.  By the padded width and the temperature alone, so that a pair's
 // result depends neither on the batch it is in nor on how a batch is sharded:
 //   2 where L2max <= 64 (one band with every lane live);
-//   2 below T = 0.3: a lane's columns share one exponent frame, and at 4 a
+//   2 below T = 0.35: a lane's columns share one exponent frame, and at 4 a
 //     part of the pairs there loses paths (scores 3 N(0, 1), T = 0.25: of 512
 //     pairs of 600 x 172, linear gap, 75 maps wrong at 4, none at 2; at
 //     T = 0.35 none at either; sw_lin.cu).  64 x 1024^2 takes 1078 us at 2 and
@@ -71,7 +71,7 @@ bool lin_eligible(float go, float ge, float T, const swb_options* opt) {
 //     1 x 1023 x 2047 1327 / 765): a caller's choice (swb_options), from
 //     T = 0.5 on.
 // The log domain always takes 4.
-constexpr float kTwoColsT = 0.3f;
+constexpr float kTwoColsT = 0.35f;
 int ck_r(long long L2m) { return L2m <= 64 ? 2 : kDefaultR; }   // checkpointed entry points: no T
 int default_r(long long L2m, bool lin, float T) { return lin && T < kTwoColsT ? 2 : (lin ? ck_r(L2m) : kDefaultR); }
 int pick_r(const swb_options* opt, long long L2m, bool lin, float T) {

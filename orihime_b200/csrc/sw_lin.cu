@@ -52,15 +52,21 @@
 // bits below the lane's row is dropped (fewer by what a row of the lane gained
 // in one step: its own values are converted in one factor).  It matters where
 // the dropped column's path would later have caught up, which takes matches
-// worth those bits inside the lane: never at scores of a few T, often at 8
-// columns per lane and low temperature.  Pairs of 512 with a wrong map (more
-// than 1e-3 off the log domain), scores 3 N(0, 1), gap -1 (linear, the worse
-// model), 600 x 172 / 500 x 384, at 2, 4 and 8 columns per lane:
+// worth those bits inside the lane.  Scores with a standard deviation of 1 to
+// 6 T never came near it at 4 columns, 6 T to 9 T did without a wrong result.
+// Pairs of 512 with a wrong map (more than 1e-3 off the log domain), scores
+// 3 N(0, 1), gap -1 (linear, the worse model), 600 x 172 / 500 x 384, at 2, 4
+// and 8 columns per lane:
 //   T = 0.5    0 / 0     0 / 0      1 / 0
 //   T = 0.35   0 / 0     0 / 0    335 / 45
 //   T = 0.25   0 / 0    75 / 6    511 / 460
-// 172 x 600, wide instead of tall: none.  A call that needs every pair at low
-// temperature takes 2 columns per lane or the log domain (swb_options).
+// 172 x 600, wide instead of tall: none.  At a deviation of 25 T (the domain
+// check lets scores up to 80 T pass) most pairs are wrong at 4 columns and many
+// at 2.  Splitting the lane's own conversions into two factors saves none of
+// them (the same counts in a restatement of the step): what is lost there is
+// the frame's range itself.  Nothing detects it; the padded entry points and
+// ragged.cols_limit choose the columns by the temperature, and a call beyond
+// that needs the log domain (swb_options).
 //
 // The kernels run when every transition factor is at most 1 (gaps <= 0);
 // otherwise the host uses the log-domain kernels of sw_kernels.cu.

@@ -470,14 +470,16 @@ DEFAULT_COLS = {"0:0": 2, "0:256": 2, "64:0": 4, "64:256": 2, "128:0": 8, "128:2
                 "256:0": 8, "256:256": 4, "512:0": 8, "512:256": 8, "1024:0": 8, "1024:256": 8}
 
 
-def cols_limit(temp: float) -> int:
+def cols_limit(temp: float, score_std: float = 3.0) -> int:
     """The most columns per lane that keep a local alignment's paths at this
-    temperature, for scores of about 3 N(0, 1): a lane's columns share one
-    exponent frame, and the lower the temperature, the more bits a match is
+    temperature, for scores of this standard deviation: a lane's columns share
+    one exponent frame, and the lower the temperature, the more bits a match is
     worth.  Pairs of 512 with a wrong map at 2, 4, 8 columns (600 x 172, linear
-    gap, the worst of the measured shapes): 0, 0, 1 at T = 0.5; 0, 0, 335 at
-    0.35; 0, 75, 511 at 0.25."""
-    return 8 if temp >= 0.5 else (4 if temp >= 0.3 else 2)
+    gap, the worst of the measured shapes, deviation 3): 0, 0, 1 at T = 0.5;
+    0, 0, 335 at 0.35; 0, 75, 511 at 0.25.  Below T = 0.25 (a deviation above
+    12 T) 2 columns lose paths as well: the log domain is for those."""
+    t = temp * (3.0 / score_std)
+    return 8 if t >= 0.5 else (4 if t >= 0.35 else 2)
 
 
 def bucket_of(L1: int, L2: int) -> str:

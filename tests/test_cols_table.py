@@ -82,12 +82,13 @@ def test_columns_do_not_depend_on_the_batch_and_fall_with_the_temperature(monkey
         for L2 in (1, 64):
             assert q(fam, L2, -2.0, -0.5, 1.0) == 2
         for L2 in (65, 255, 256, 300, 4096):
-            for T, want in ((1.0, 4), (0.3, 4), (0.29, 2), (0.25, 2)):
+            for T, want in ((1.0, 4), (0.35, 4), (0.34, 2), (0.25, 2)):
                 assert q(fam, L2, -2.0, -0.5, T) == want, (fam, L2, T)
             assert q(fam, L2, 1.0, -0.5, 0.25) == 4   # the log domain
     for fam in (2, 4, 5):
         assert q(fam, 300, -2.0, -0.5, 0.25) == 4
-    assert [ragged.cols_limit(T) for T in (1.0, 0.5, 0.49, 0.3, 0.25)] == [8, 8, 4, 4, 2]
+    assert [ragged.cols_limit(T) for T in (1.0, 0.5, 0.49, 0.35, 0.34)] == [8, 8, 4, 4, 2]
+    assert [ragged.cols_limit(1.0, s) for s in (6.0, 8.5, 10.0)] == [8, 4, 2]
 
     # autotune_plan offers no candidate above the limit, whatever an earlier call cached
     monkeypatch.setenv("ORIHIME_B200_CACHE", str(tmp_path))

@@ -28,7 +28,7 @@ def test_large_batch_equals_its_shards_and_a_plan(family, L1, L2, T):
     for every in (1, 4):
         got = _ops.run_checkpoint(fam, s, None, (*gaps, T), every)
         if got is None:
-            assert T < 0.3
+            assert T < 0.35
             continue
         for x, y in zip(_ops.run_adjoint(fam, s, None, (*gaps, T), every, got[1]), want):
             assert torch.equal(x, y)
