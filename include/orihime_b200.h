@@ -454,7 +454,7 @@ int swb_scan_scores(const float* x, int B, long long per_item, float limit, floa
  * aligned, swb_*_adjoint_scratch_bytes(B, L1max, L2max); 0 where it would not
  * help), about 1 byte per cell, that need not be kept between the two halves:
  * batches of few bands then take about half the time, with the same bits.
- * With less scratch, or NULL, it is swb_*_adjoint.
+ * With less scratch, scratch not so aligned, or NULL, it is swb_*_adjoint.
  */
 size_t swb_sw_affine_adjoint_scratch_bytes(int B, int L1max, int L2max);
 int swb_sw_affine_adjoint_scratch(const float* scores, const int* lengths, int B, int L1max, int L2max,

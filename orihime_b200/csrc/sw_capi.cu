@@ -886,7 +886,7 @@ int ck_adjoint_r(const float* scores, const int* lengths, int B, int L1m, int L2
   const long long cap = (long long)d->sms * (ob > 0 ? ob : 1);
   const int grid = (int)std::max(1LL, std::min((ntasks + kWarpsBwd - 1) / kWarpsBwd, cap));
   const SegPlan seg = seg_plan<R>(l, ntasks);
-  if (seg.bytes && scratch && scratch_bytes >= seg.bytes)
+  if (seg.bytes && scratch && scratch_bytes >= seg.bytes && reinterpret_cast<uintptr_t>(scratch) % 16 == 0)
     return launch_segments<NS, R>(a, *d, seg, static_cast<char*>(scratch), kc > 1, 0, st);
   if (kc > 1)
     swb::lbwd_kernel<NS, R, kWarpsBwd, true><<<grid, 32 * kWarpsBwd, lbwd_smem<NS, R>(), st>>>(a);

@@ -4,9 +4,9 @@
 // buffers, polling and pair finish this file reuses.
 //
 // What bounds it.  4096 ragged pairs fill every warp slot: the forward moves
-// about 7 GB (scores and checkpoints) in 1.69 ms, two thirds of the measured
+// about 7 GB (scores and checkpoints) in 1.68 ms, two thirds of the measured
 // copy rate, and the adjoint is bound by instruction issue and dependent
-// results (3.4 ms).  A small batch is bound by the latency of one step of one
+// results (3.12 ms).  A small batch is bound by the latency of one step of one
 // warp: about 120 ns at 4 columns per lane and 160 at 8 (180 and 390 before
 // the steps were packed and their bounds, address and frame arithmetic cut),
 // times the steps of the longest chain of bands.

@@ -168,19 +168,28 @@ def test_sparse_adjoint_of_whole_bands_equals_one_call(fam, ck_every, B, L1, L2)
     assert torch.equal(value, want[0])
     for g, w in zip(_ops.run_adjoint(fam, s, None, params, ck_every, ws), want):
         assert torch.equal(g, w)
-    # two pairs: segments with scratch, whole bands without
+    # two pairs: segments with scratch, whole bands without or where it is not aligned
+    lib = _lib.load()
     s2 = s[:2].contiguous()
     want = run(s2, None, *params)
     _, ws = _ops.run_checkpoint(fam, s2, None, params, ck_every)
-    for scratch in (True, False):
-        if scratch:
-            got = _ops.run_adjoint(fam, s2, None, params, ck_every, ws)
-        else:
-            e = lambda: torch.empty(2, device="cuda")  # noqa: E731
-            got = [e(), torch.empty_like(s2)] + [e() for _ in params]
-            fn = _lib.load().swb_sw_affine_adjoint if fam == "sw_affine" else _lib.load().swb_sw_adjoint
-            rc = fn(s2.data_ptr(), None, 2, L1, L2, *params, ck_every, *(t.data_ptr() for t in got),
-                    ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
-            assert rc == _lib.OK
+    fn, size = ((lib.swb_sw_affine_adjoint_scratch, lib.swb_sw_affine_adjoint_scratch_bytes) if fam == "sw_affine"
+                else (lib.swb_sw_adjoint_scratch, lib.swb_sw_adjoint_scratch_bytes))
+    need = size(2, L1, L2)
+    assert need > 0
+    buf = torch.empty(need + 16, dtype=torch.uint8, device="cuda")
+    for scratch, nbytes in ((buf.data_ptr(), need), (buf.data_ptr() + 4, need), (buf.data_ptr(), need - 1), (None, 0)):
+        e = lambda: torch.empty(2, device="cuda")  # noqa: E731
+        got = [e(), torch.empty_like(s2)] + [e() for _ in params]
+        rc = fn(s2.data_ptr(), None, 2, L1, L2, *params, ck_every, *(t.data_ptr() for t in got),
+                ws.data_ptr(), ws.numel(), scratch, nbytes, torch.cuda.current_stream().cuda_stream)
+        assert rc == _lib.OK
         for g, w in zip(got, want):
             assert torch.equal(g, w)
+    plain = lib.swb_sw_affine_adjoint if fam == "sw_affine" else lib.swb_sw_adjoint
+    got = [torch.zeros_like(t) for t in got]
+    rc = plain(s2.data_ptr(), None, 2, L1, L2, *params, ck_every, *(t.data_ptr() for t in got),
+               ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    assert rc == _lib.OK
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
