@@ -1096,22 +1096,22 @@ __device__ __forceinline__ double scaled(float g, float k) { return EXACT ? (dou
 // the log domain adds the rounded one.
 template <int NS, int GM = 0, bool LIN = false>
 __device__ void finish_pair_p(const Args& a, const Place& w, int lane, float Sh, float Sl,
-                              float g0sum, float g1sum, float pssum, PParams pp);
+                              float g0sum, float g1sum, float pssum, PParams pp, float psum = 0.f);
 
 template <int NS, int GM = 0>
 __device__ void finish_pair(const Args& a, const Place& w, int lane, float Sh, float Sl,
-                            float g0sum, float g1sum, float pssum) {
-  finish_pair_p<NS, GM>(a, w, lane, Sh, Sl, g0sum, g1sum, pssum, PParams{a.go, a.ge, a.T, a.k});
+                            float g0sum, float g1sum, float pssum, float psum = 0.f) {
+  finish_pair_p<NS, GM>(a, w, lane, Sh, Sl, g0sum, g1sum, pssum, PParams{a.go, a.ge, a.T, a.k}, psum);
 }
 
 template <int NS, int GM, bool LIN>
 __device__ void finish_pair_p(const Args& a, const Place& w, int lane, float Sh, float Sl,
-                              float g0sum, float g1sum, float pssum, PParams pp) {
+                              float g0sum, float g1sum, float pssum, PParams pp, float psum) {
   constexpr bool G = GM == 1;
   const int p = w.p;
   if (lane == 0) {
     float* gp = a.gpart + 4 * (w.slot0 + w.band);
-    gp[0] = g0sum; gp[1] = g1sum; gp[2] = pssum; gp[3] = 0.f;
+    gp[0] = g0sum; gp[1] = g1sum; gp[2] = pssum; gp[3] = psum;
     __threadfence();
     unsigned done = atomicAdd(a.pair_done + p, 1u);
     if ((done & ~PAIR_TIMEOUT) == (unsigned)w.nb - 1) {
@@ -1122,12 +1122,13 @@ __device__ void finish_pair_p(const Args& a, const Place& w, int lane, float Sh,
         if (a.g_ext) a.g_ext[p] = nan;
         return;
       }
-      double o = 0., e = 0., ps = 0.;
+      double o = 0., e = 0., ps = 0., np = 0.;
       for (int b = 0; b < w.nb; ++b) {
         const float* q = a.gpart + 4 * (w.slot0 + b);
         o += ld_poll(q + 0);
         e += ld_poll(q + 1);
         ps += ld_poll(q + 2);
+        if (G && NS == 3) np += ld_poll(q + 3);
       }
       if (G && (w.pr.L1 == 0 || w.pr.L2 == 0)) {
         // the terminal is a boundary cell: its value, its gap derivatives, dS/dT = 0
@@ -1142,6 +1143,11 @@ __device__ void finish_pair_p(const Args& a, const Place& w, int lane, float Sh,
       a.g_open[p] = (float)o;
       if (a.g_ext) a.g_ext[p] = NS == 3 ? (float)e : 0.f;
       if (G && NS == 1) a.g_T[p] = (float)(ps * 0.693147180559945309);   // an entropy in bits (bwd_band)
+      else if (G && NS == 3) {
+        // the flow's drift (bwd_band): every path has 2 matches + gaps = L1 + L2
+        const double r = (double)(w.pr.L1 + w.pr.L2) / (2. * np + o + e);
+        a.g_T[p] = dS_dT(Sh, Sl, ps * r, o * r, scaled<LIN>(pp.go, pp.k), e * r, scaled<LIN>(pp.ge, pp.k));
+      }
       else a.g_T[p] = dS_dT(Sh, Sl, ps, o, scaled<LIN>(pp.go, pp.k), NS == 3 ? e : 0., scaled<LIN>(pp.ge, pp.k));
     }
   }
@@ -1167,7 +1173,10 @@ __device__ void finish_pair_p(const Args& a, const Place& w, int lane, float Sh,
 // >= 0, those of the boundary 0).  As (S - <score>) / T it is the small
 // difference of two large sums, in which the flow's own rounding, about 1e-7 a
 // step, shows: 33 x 700 at T = 0.25, S = -545, dS/dT = 19.55: 6.3e-3 off that
-// way, 8.6e-5 this way.
+// way, 8.6e-5 this way.  Global affine, where three entropies a cell cost a tenth
+// of the call, takes the drift out on average: every path has the same number of
+// steps, twice its matches plus its gaps, so the expected one is known (gP):
+// 860 x 35 at T = 0.25 1.4e-5 of dS/dT off instead of 2.1e-4.
 template <int NS, int R, int GM = 0>
 __device__ void bwd_band(const Args& a, const Place& w, int lane, float* sm, uint64_t deadline) {
   constexpr bool G = GM == 1;
@@ -1249,6 +1258,7 @@ __device__ void bwd_band(const Args& a, const Place& w, int lane, float* sm, uin
 #pragma unroll
   for (int q = 0; q < NP; ++q) outp[q] = 0.f;
   KSum gA, gB, gS;   // chunk sums folded in with compensation
+  [[maybe_unused]] KSum gP;   // global affine: the matches
 
   for (int kc = nch - 1; kc >= 0; --kc) {
     const int t0 = kc * C_STEPS;
@@ -1361,6 +1371,7 @@ __device__ void bwd_band(const Args& a, const Place& w, int lane, float* sm, uin
       }
     }
     float cA = 0.f, cB = 0.f, cS = 0.f;   // this chunk's plain sums
+    [[maybe_unused]] float cP = 0.f;
     // ---- restore the checkpoint and recompute the chunk's adjoint fields ----
     float ph[NS][R], pl[NS][R], lh[NS], ll[NS];
     ck_unpack<NS, R>(ckr, ph, pl, lh, ll);
@@ -1506,6 +1517,7 @@ __device__ void bwd_band(const Args& a, const Place& w, int lane, float* sm, uin
           cA += (pIM + pID) + (pDM + pDI);
           cB += pII + pDD;
           cS += bM * sc;
+          cP += bM;
           // pushes into the boundary states D(0, j) (row 0) and I(i, 0)
           // (column 0): gap_open once, gap_ext (n - 1) times; pushes toward
           // the NEG boundary states are 0
@@ -1620,17 +1632,19 @@ __device__ void bwd_band(const Args& a, const Place& w, int lane, float* sm, uin
     gA.add(cA);
     gB.add(cB);
     gS.add(cS);
+    if constexpr (G && NS == 3) gP.add(cP);
     __syncwarp();
   }
   // warp-reduce the gradient partials (fixed shuffle tree: deterministic)
-  float v0 = gA.s, v1 = gB.s, v2 = gS.s;
+  float v0 = gA.s, v1 = gB.s, v2 = gS.s, v3 = gP.s;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     v0 += __shfl_xor_sync(FULL, v0, o);
     v1 += __shfl_xor_sync(FULL, v1, o);
     v2 += __shfl_xor_sync(FULL, v2, o);
+    if constexpr (G && NS == 3) v3 += __shfl_xor_sync(FULL, v3, o);
   }
-  finish_pair<NS, GM>(a, w, lane, Sh, Sl, v0, v1, v2);
+  finish_pair<NS, GM>(a, w, lane, Sh, Sl, v0, v1, v2, v3);
 }
 
 // Shared memory per adjoint warp (floats): one chunk of adjoint fields.
